@@ -102,13 +102,13 @@ MBX_API int mbx_get_device_error(int *flags_out);
 /* Number of kernel launches this library has submitted since it was loaded (host-side count, all devices and
  * streams; launches replayed from a captured CUDA graph are not re-counted). */
 MBX_API uint64_t mbx_launch_count(void);
-/* Autotuning of the projector plans (no counterpart in the reference, whose XLA compiler picks its own
- * schedule).  The first mbx_sparse_forward_project / mbx_sparse_back_project of a call shape (geometry sizes,
- * views, pixel count rounded up to a power of two) times its candidate plans on the caller's stream,
+/* Autotuning of the forward projector's plans (no counterpart in the reference, whose XLA compiler picks its own
+ * schedule; the back projector has one plan per call shape).  The first mbx_sparse_forward_project of a call shape
+ * (geometry sizes, views, pixel count rounded up to a power of two) times its candidate plans on the caller's stream,
  * synchronising it, and caches the fastest for the process; a call made while its stream is captured uses the
- * default plan.  Forward candidates: channel-block width, pass size, and the kernel variant compiled for 2 or 3
- * resident CTAs per SM; back-projection candidates: footprints staged in shared memory or computed per thread.
- * mbx_vcd_batched_prepare tunes its two projection stages the same way, cached per batch shape.  Plans differ
+ * default plan.  Candidates: channel-block width, pass size, and the kernel variant compiled for 2 or 3 resident CTAs
+ * per SM.
+ * mbx_vcd_batched_prepare tunes its forward stage the same way, cached per batch shape.  Plans differ
  * only in float summation order.  mode: 0 = default plans, 1 = tune (default), k >= 2 = use candidate k-1 (or the
  * last one) everywhere without timing (to check every plan against the default).  Returns the previous mode. */
 MBX_API int mbx_set_autotune(int mode);
@@ -128,7 +128,8 @@ MBX_API int mbx_sparse_forward_project(const mbx_geom *g, const float *voxel_val
                                int64_t num_pixels, const int32_t *view_indices, int32_t num_views_sel,
                                float *sinogram_out, void *workspace, size_t workspace_bytes, void *stream);
 
-/* Workspace the back projector needs for a call with these sizes (0 when it needs none). */
+/* Workspace the back projector needs for a call with these sizes (0 when it needs none): partial sums of view splits,
+ * and for calls with enough pixels a transposed copy of the projected views. */
 MBX_API size_t mbx_back_project_workspace_bytes(const mbx_geom *g, int64_t num_pixels, int32_t num_views_sel);
 
 /* Sparse back projection of a full sinogram (num_views, R, C) to out (num_pixels, S) (overwritten):

@@ -18,116 +18,148 @@
 // instead of once per vertical tap.  The optional weights are multiplied into every gathered value
 // (a fused W * e).  Views may be split over CTAs with a fixed-order second-stage sum when there are too
 // few pixels to fill the GPU (caller workspace).
+#include <algorithm>
+
 #include "back_project.cuh"
 #include "bp_fast.cuh"
 
 namespace mbx {
 
+// Whether a call makes a transposed copy of its views (bp_fast.cuh): the copy moves R C values per view, the projection
+// N S.
+static bool bp_transposes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
+    return num_pixels * g.num_recon_slices * BPF_TRANSPOSE_RATIO >= (long long)g.num_det_rows * g.num_det_channels &&
+           (long long)g.num_views * (g.num_det_channels + 2 * BPF_EDGE) * bpf_padded_rows(g) < (1LL << 31);
+}
+
+bool bpf_window_map(CUtensorMap &map, const float *copy, const mbx_geom &g, int num_views_sel, int boxq) {
+    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = []() -> Encode {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
+                                                               cudaEnableDefault, &found);
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<Encode>(fn) : nullptr;
+    }();
+    if (!encode || (reinterpret_cast<uintptr_t>(copy) & 15)) return false;
+    const cuuint64_t rp = (cuuint64_t)bpf_padded_rows(g);
+    const cuuint64_t dims[2] = {rp, (cuuint64_t)bpf_transposed_views(g, num_views_sel) *
+                                        (cuuint64_t)(g.num_det_channels + 2 * BPF_EDGE)};
+    const cuuint64_t strides[1] = {rp * 4};
+    const cuuint32_t box[2] = {4u * (cuuint32_t)boxq, BPF_BOX}, elem[2] = {1, 1};
+    return encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(copy), dims, strides, box, elem,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 size_t bp_workspace_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
     const BpfPlan fp = plan_bp_fast(g, num_pixels, num_views_sel);
-    if (fp.ok) return fp.workspace;
+    if (fp.ok)
+        return fp.workspace + (bp_transposes(g, num_pixels, num_views_sel) ? bpf_transposed_bytes(g, num_views_sel) : 0);
     return plan_bp(g, num_pixels, num_views_sel).workspace;
 }
 
-template <int KIND>
-static cudaError_t launch_bp_fast(const mbx_geom &g, const BpfPlan &pl, const float *sino, const float *w,
-                                  const int32_t *pix, long long n, const int32_t *views, int nv, int cp, float scale,
-                                  float *dst, long long ss, cudaStream_t st, int out_slices = 0) {
-    auto kern = bp_fast_kernel<KIND>;
-    cudaError_t ea = set_max_dynamic_smem(reinterpret_cast<const void *>(kern), 100 * 1024);
+size_t bp_noalloc_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
+    const BpfPlan fp = plan_bp_fast(g, num_pixels, num_views_sel, 1);
+    return fp.ok ? fp.workspace : plan_bp(g, num_pixels, num_views_sel).workspace;
+}
+
+__global__ void __launch_bounds__(256) bp_transpose_kernel(const float *__restrict__ src, const float *__restrict__ wts,
+                                                           const int32_t *__restrict__ views, int num_views,
+                                                           int first, float *__restrict__ dst, int num_rows,
+                                                           int num_channels, int rp) {
+    const int j = first + blockIdx.y;
+    const int vi = views ? views[j] : j;
+    if (vi < 0 || vi >= num_views) return;  // flagged and skipped by the projection
+    bpf_transpose_block(src, wts, dst, (long long)vi * num_rows * num_channels,
+                        (long long)j * (num_channels + 2 * BPF_EDGE) * rp, blockIdx.x * 32, num_rows, num_channels, rp);
+}
+
+template <int KIND, bool TR>
+static cudaError_t launch_bp_fast_kind(const BpArgs &A, const CUtensorMap &map, cudaStream_t st) {
+    auto kern = bp_fast_kernel<KIND, TR>;
+    const cudaError_t ea = set_max_dynamic_smem(reinterpret_cast<const void *>(kern), 100 * 1024);
     if (ea != cudaSuccess) return ea;
-    BpArgs A;
-    A.g = g;
-    A.sino = sino;
-    A.wts = w;
-    A.pix = pix;
-    A.num_pixels = n;
-    A.order = nullptr;
-    A.views = views;
-    A.num_views_sel = nv;
-    A.views_per_split = pl.views_per_split;
-    A.coeff_power = cp;
-    A.scale = scale;
-    A.out = dst;
-    A.split_stride = ss;
-    A.out_by_index = 0;
-    A.out_slices = out_slices;
-    A.plan = pl;
-    dim3 grid(pl.gx, pl.gy, pl.splits);
-    kern<<<grid, BPF_THREADS, pl.smem, st>>>(A, device_error_ptr());
+    const dim3 grid((unsigned)(A.plan.gx * A.plan.gy * (BPF_WARPS / BPF_LAUNCH_WARPS)), A.plan.splits);
+    kern<<<grid, 32 * BPF_LAUNCH_WARPS, bpf_smem_bytes(KIND, BPF_LAUNCH_WARPS), st>>>(A, map, device_error_ptr());
     note_launch();
     return cudaGetLastError();
 }
 
+template <bool TR>
+static cudaError_t launch_bp_fast(const BpArgs &A, const CUtensorMap &map, cudaStream_t st) {
+    switch (A.g.kind) {
+        case MBX_GEOM_PARALLEL: return launch_bp_fast_kind<MBX_GEOM_PARALLEL, TR>(A, map, st);
+        case MBX_GEOM_CONE: return launch_bp_fast_kind<MBX_GEOM_CONE, TR>(A, map, st);
+        default: return launch_bp_fast_kind<MBX_GEOM_TRANSLATION, TR>(A, map, st);
+    }
+}
+
 int back_project(const mbx_geom &g, const float *sino, const float *w, const int32_t *pix, long long num_pixels,
                  const int32_t *views, int num_views_sel, int coeff_power, float scale, float *out, void *ws,
-                 size_t ws_bytes, cudaStream_t st) {
+                 size_t ws_bytes, cudaStream_t st, bool noalloc) {
     if (num_pixels == 0) return MBX_OK;
+    BpArgs A = {};
+    A.g = g;
+    A.sino = sino;
+    A.wts = w;
+    A.pix = pix;
+    A.num_pixels = num_pixels;
+    A.views = views;
+    A.num_views_sel = num_views_sel;
+    A.coeff_power = coeff_power;
+    A.scale = scale;
+    A.out = out;
+    CUtensorMap map = {};
     if (bp_unit_broadcast(g, sino, w)) {  // unit-weight parallel Hessian: one slice, written to every slice
-        const mbx_geom g1 = one_slice_geometry(g);
-        const BpfPlan p1 = plan_bp_fast(g1, num_pixels, num_views_sel);
-        if (p1.ok && p1.splits == 1) {
-            const cudaError_t e = launch_bp_fast<MBX_GEOM_PARALLEL>(g1, p1, nullptr, nullptr, pix, num_pixels, views,
-                                                                   num_views_sel, coeff_power, scale, out, 0, st,
-                                                                   g.num_recon_slices);
+        A.g = one_slice_geometry(g);
+        A.plan = plan_bp_fast(A.g, num_pixels, num_views_sel, noalloc);
+        if (A.plan.ok && A.plan.splits == 1) {
+            A.views_per_split = A.plan.views_per_split;
+            A.out_slices = g.num_recon_slices;
+            const cudaError_t e = launch_bp_fast<false>(A, map, st);
             return e == cudaSuccess ? MBX_OK : set_cuda_error(e);
         }
+        A.g = g;
     }
-    const BpfPlan fpl = plan_bp_fast(g, num_pixels, num_views_sel);
-    if (fpl.ok) {
-        if (fpl.workspace > 0 && (ws == nullptr || ws_bytes < fpl.workspace)) return MBX_ERR_WORKSPACE;
-        float *dst = fpl.splits > 1 ? static_cast<float *>(ws) : out;
+    A.plan = plan_bp_fast(g, num_pixels, num_views_sel, noalloc);
+    if (A.plan.ok) {
+        bool tr = !noalloc && sino && bp_transposes(g, num_pixels, num_views_sel);
+        const size_t need = A.plan.workspace + (tr ? bpf_transposed_bytes(g, num_views_sel) : 0);
+        if (need > 0 && (ws == nullptr || ws_bytes < need)) return MBX_ERR_WORKSPACE;
+        float *copy = reinterpret_cast<float *>(static_cast<char *>(ws) + A.plan.workspace);
+        tr = tr && bpf_window_map(map, copy, g, num_views_sel, A.plan.boxq);
         const long long stride = num_pixels * (long long)g.num_recon_slices;
-        const long long ss = fpl.splits > 1 ? stride : 0;
-        auto run = [&](const BpfPlan &pl) -> cudaError_t {
-            cudaError_t e;
-            if (g.kind == MBX_GEOM_PARALLEL)
-                e = launch_bp_fast<MBX_GEOM_PARALLEL>(g, pl, sino, w, pix, num_pixels, views, num_views_sel,
-                                                      coeff_power, scale, dst, ss, st);
-            else if (g.kind == MBX_GEOM_CONE)
-                e = launch_bp_fast<MBX_GEOM_CONE>(g, pl, sino, w, pix, num_pixels, views, num_views_sel, coeff_power,
-                                                  scale, dst, ss, st);
-            else
-                e = launch_bp_fast<MBX_GEOM_TRANSLATION>(g, pl, sino, w, pix, num_pixels, views, num_views_sel,
-                                                         coeff_power, scale, dst, ss, st);
-            if (e != cudaSuccess) return e;
-            if (pl.splits > 1) {
-                launch_split_sum(dst, stride, pl.splits, scale, out, stride, st);
+        A.views_per_split = A.plan.views_per_split;
+        if (A.plan.splits > 1) {
+            A.out = static_cast<float *>(ws);
+            A.split_stride = stride;
+        }
+        cudaError_t e = cudaSuccess;
+        if (tr) {
+            A.tsino = copy;
+            A.rp = bpf_padded_rows(g);
+            const int nt = bpf_transposed_views(g, num_views_sel);
+            A.tsino_all = num_views_sel > g.num_views || !views ? 1 : 0;
+            const int32_t *tv = A.tsino_all ? nullptr : views;
+            // views in grid.y, at most 65535 per launch
+            for (int j0 = 0; j0 < nt && e == cudaSuccess; j0 += 65535) {
+                bp_transpose_kernel<<<dim3((unsigned)ceil_div(g.num_det_channels + 2 * BPF_EDGE, 32), (unsigned)std::min(nt - j0, 65535)),
+                                      256, 0, st>>>(sino, w, tv, g.num_views, j0, copy, g.num_det_rows,
+                                                    g.num_det_channels, A.rp);
+                note_launch();
                 e = cudaGetLastError();
             }
-            return e;
-        };
-        // staged (shared-memory) or per-thread (inline) footprints: cached per call shape, or timed now (each
-        // candidate overwrites the whole output); both have the same grid, splits and workspace
-        BpfPlan cand[2] = {fpl, plan_bp_fast(g, num_pixels, num_views_sel, 1)};
-        int choice = 0;
-        if (autotune_forced() >= 0) {
-            choice = autotune_forced() >= 1 ? 1 : 0;
-        } else if (autotune_enabled()) {
-            long long n2 = 1;
-            while (n2 < num_pixels) n2 <<= 1;
-            const long long key[11] = {3, g.kind, num_views_sel, g.num_det_rows, g.num_det_channels, g.num_recon_slices,
-                                       g.num_recon_rows, g.num_recon_cols, n2, views ? 1 : 0, w ? 1 : 0};
-            choice = autotune_lookup(key, 11);
-            if (choice < 0 || choice > 1) {
-                choice = 0;
-                if (!stream_is_capturing(st)) {
-                    float t0 = 0.0f;  // the default first: a long call is not tuned (its output is complete)
-                    cudaError_t e = time_once([&]() { return run(cand[0]); }, st, t0);
-                    if (e != cudaSuccess) return set_cuda_error(e);
-                    if (t0 > MBX_TUNE_BUDGET_MS) {
-                        autotune_store(key, 11, 0);
-                        return MBX_OK;
-                    }
-                    float t[2] = {0.0f, 0.0f};
-                    e = time_candidates(2, [&](int c) { return run(cand[c]); }, st, t);
-                    if (e != cudaSuccess) return set_cuda_error(e);
-                    choice = t[1] < t[0] ? 1 : 0;
-                    autotune_store(key, 11, choice);
-                }
-            }
+            if (e == cudaSuccess) e = launch_bp_fast<true>(A, map, st);
+        } else {
+            e = launch_bp_fast<false>(A, map, st);
         }
-        const cudaError_t e = run(cand[choice]);
+        if (e == cudaSuccess && A.plan.splits > 1) {
+            launch_split_sum(A.out, stride, A.plan.splits, scale, out, stride, st);
+            e = cudaGetLastError();
+        }
         return e == cudaSuccess ? MBX_OK : set_cuda_error(e);
     }
     const BpPlan pl = plan_bp(g, num_pixels, num_views_sel);

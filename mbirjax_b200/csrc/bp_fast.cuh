@@ -1,74 +1,146 @@
 // Back projector specialised for psf_radius == 1 (the reference's default geometry: delta_voxel equal to the
-// detector pitch at the magnification), for parallel and cone beam.  Same contract and arithmetic as the
-// general bp_kernel (back_project.cuh); organised to minimise instructions per (pixel, slice, view):
+// detector pitch at the magnification).  Same contract and arithmetic as the general bp_kernel (back_project.cuh);
+// organised so that a (pixel, slice, view) costs few instructions and its detector samples come from shared memory:
 //
-//  * CTA = 256 threads = 8 warps; lanes run along 32 pixels, warps along slice tiles (or along further pixel
-//    groups when the cylinder has fewer than 8 tiles).  The tile height ts <= 16 is chosen so that the tiles
-//    split the slices evenly over a power-of-two number of warps; accumulators stay in registers.
-//  * Per chunk of views, each (pixel, view) footprint is computed once, by one thread, into shared memory as
-//    one float4 and read by every warp of that pixel: the first of three consecutive detector channels that
-//    hold every nonzero tap and their coefficients (already raised to coeff_power; at the detector edges the
-//    taps are shifted onto in-range channels with a zero coefficient, so every gather is three loads at
-//    constant offsets from one pointer), plus for cone beam the affine map slice -> detector row
-//    m_p(k) = A0 + k*A1 and the vertical-angle factor c2 = (mag/D)^2 so that 1/cos(phi_k) = sqrt(1 + c2 z_k^2).
-//    The cone footprint is trig-free: cos/sin(theta - theta_p) and 1/cos(theta_p) come from the per-view
-//    cos/sin and rsqrt(D^2 + u^2) instead of atan2/cos/sin per pixel.
-//  * Cone: every detector row a warp's slice tile touches is gathered once per view into the thread's column
-//    of a shared-memory row cache ([row][thread], conflict-free), rows outside the detector cached as 0; the
-//    vertical fan then reads three cached rows per slice with no bounds tests.  plan_bp_fast admits a geometry
-//    only when the rows of a slice tile (ts * max |dm/dk| + 4) fit the cache.
+//  * CTA = 256 threads = 8 independent warps; a warp owns 32 pixels (one per lane) x a tile of ts <= BPF_ST slices,
+//    with the accumulators of a lane's slices in registers (as pairs, for the two-wide FMA) across all views.
+//    Nothing but the per-view constants is shared between warps, so they run without barriers of their own.
+//  * Per view each lane computes the footprint of its pixel in registers: centre channel, three coefficients
+//    (already raised to coeff_power, zero off the detector), and for the fan geometries the affine map slice ->
+//    detector row m_p(k) = A0 + k*A1 and the vertical-angle factor c2 = (mag/D)^2, 1/cos(phi_k) = sqrt(1 + c2 z_k^2).
+//    It is trig-free: cos/sin(theta - theta_p) and 1/cos(theta_p) come from the per-view cos/sin and
+//    rsqrt(D^2 + u^2) instead of atan2/cos/sin per pixel.
+//  * The channels and rows that the warp's footprints touch (their exact range, by warp min/max) are a small window
+//    of the view, about 20 to 36 channels wide for a compact pixel list.  It is copied once into the warp's own shared
+//    memory, channels outermost ([channel][row], weights multiplied in, zeros off the detector), so that a lane reads
+//    four rows of a channel with one 16-byte load at a constant offset; the channel pitch is an odd number of 16-byte
+//    units, so lanes on neighbouring channels hit different banks.  Calls with enough pixels first make a transposed
+//    copy of their sinogram (view, channel, row), whose windows the TMA unit copies (boxes of 8 channels; no load or
+//    store instruction, and no share of the load/store pipe, which bounds the kernel); the others copy by plain loads.
+//  * Fan geometries: a lane first forms the horizontal sum of each window row in its own column of a row buffer
+//    ([row][lane], conflict-free), then the vertical fan reads three of its rows per slice with no bounds tests.
+//    plan_bp_fast admits a geometry only when the rows of a slice tile (ts * max |dm/dk| + 4) fit that buffer.
+//    Measured (B200, one subset of 4 unless said): parallel 652 x 57 x 437 1724 -> 895 us a call against the kernel that
+//    gathered each tap from global memory (21 instructions per slice and view there, 12 here), cone 360 x 256 x 512
+//    (subset of 8) 11.98 -> 6.25 ms, translation 49 x 128 x 128 (all pixels) 197 -> 123 us, weighted squared cone
+//    180 x 61 x 203 2.41 -> 1.26 ms; with windows copied by 16-byte cp.async instead of the TMA the parallel call took
+//    975 us.
+//  * Pixels without locality, which would need many windows, are handled some lanes at a time, each with private
+//    columns of its own taps in the place of the window.
 #pragma once
+
+#include <cuda.h>  // CUtensorMap
+
+#include <algorithm>
+#include <type_traits>
 
 #include "back_project.cuh"
 
 namespace mbx {
 
 constexpr int BPF_THREADS = 256;
+constexpr int BPF_WARPS = BPF_THREADS / 32;
 #ifndef MBX_BPF_ST
-#define MBX_BPF_ST 16
+#define MBX_BPF_ST 32
 #endif
-constexpr int BPF_ST = MBX_BPF_ST;  // most slices per thread
-constexpr int BPF_CACHE_ROWS = 48;  // row-cache depth per thread (cone): ts * max|dm/dk| + 4 must fit
-#ifndef MBX_BPF_CHUNK_PARALLEL
-#define MBX_BPF_CHUNK_PARALLEL 1024     // footprints staged per view chunk, parallel beam
-#endif
-#ifndef MBX_BPF_CHUNK_CONE
-#define MBX_BPF_CHUNK_CONE 512          // same, cone beam (its row cache takes most of the shared memory)
-#endif
-#ifndef MBX_BPF_PREFETCH
-#define MBX_BPF_PREFETCH 2              // parallel beam, staged footprints: views ahead whose rows are prefetched
-#endif                                  // into L1 while the current view is gathered (0: none; 1, 2 and 4 measure
-                                        // the same, 8.5% faster than none on the batched bench stage)
+constexpr int BPF_ST = MBX_BPF_ST;  // most slices per thread (a multiple of 4)
+constexpr int BPF_CACHE_ROWS = 48;  // row-buffer depth (fan geometries): ts * max|dm/dk| + 4 must fit
+constexpr int BPF_BOX = 8;          // channels per TMA box
+constexpr int BPF_EDGE = 2;         // channels of zeros on either side of a view of the transposed copy
+constexpr int BPF_FAN_QUADS = 13;   // most rows of a fan window and of the row buffer, in fours: BPF_CACHE_ROWS and the
+                                    // rounding of the first row down to a multiple of 4
+// A warp whose pixels need several windows of a view copies them one by one while their channels fall in at most
+// BPF_WINDOWS stretches of BPF_SPLIT channels.
+constexpr int BPF_SPLIT = 32;
+constexpr int BPF_WINDOWS = 4;
+// A call copies its sinogram transposed when its pixels' slices are at least 1 / this of a view's elements.
+constexpr int BPF_TRANSPOSE_RATIO = 8;
+// Window floats: 32 channels of 36 rows (parallel, two buffers), 32 channels of 52 rows (fan geometries).
+constexpr int BPF_WIN_PARALLEL = 32 * 36;
+constexpr int BPF_WIN_FAN = 32 * 4 * BPF_FAN_QUADS;
 
 struct BpfPlan {
     int nsl;      // slice tiles per CTA (warps per pixel group)
     int npg;      // pixel groups of 32 per CTA
     int lg_pcta;  // log2(32 * npg)
-    int chunk;    // footprints staged per view chunk (a multiple of BPF_THREADS); 0 with inline footprints
-    int vc;       // views per chunk = chunk / (32 * npg); with inline footprints, views per table refill
-    int inline_fp;  // 1: each thread computes its own pixel's footprints in registers (no staging, no barriers
-                    // inside a view table); pays off when few warps share a pixel (short cylinders)
+    int chunk;    // footprints staged ahead of their use: 0, a lane computes its own pixel's when it needs them
+    int vc;       // views whose constants a warp holds at a time
+    int inline_fp;  // 1 (see chunk)
     int ts;       // slices per tile (<= BPF_ST)
+    int boxq;     // rows of a window in fours, an odd number
     int tiles;    // ceil(S / ts)
     int gx, gy, splits, views_per_split;
-    size_t smem, workspace;
+    size_t smem, workspace;  // of a launched CTA; the partial sums of the splits
     bool ok;
 };
 
-// Footprint of one (pixel, view): fa = {first channel (int bits; -1: no tap), c0, c1, c2} for the channels
-// first, first+1, first+2; fb (cone) = {A0, A1, c2 = (mag/D)^2, 0}.
+// Pairs of floats in one 64-bit register, for the two-wide FMA / add / multiply (each half rounded on its own).
+using bpf2 = unsigned long long;
+__device__ __forceinline__ bpf2 bpf_pair(float a, float b) {
+    bpf2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void bpf_unpair(bpf2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ bpf2 bpf_fma(bpf2 a, bpf2 b, bpf2 c) {
+    bpf2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ bpf2 bpf_mul(bpf2 a, bpf2 b) {
+    bpf2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ bpf2 bpf_add(bpf2 a, bpf2 b) {
+    bpf2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Shared memory at byte address a + OFS: one float, or four as two pairs.
+template <int OFS>
+__device__ __forceinline__ float bpf_lds(unsigned a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(a), "n"(OFS));
+    return v;
+}
+template <int OFS>
+__device__ __forceinline__ void bpf_lds4(unsigned a, bpf2 &x, bpf2 &y) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2+%3];" : "=l"(x), "=l"(y) : "r"(a), "n"(OFS));
+}
+// A loop over I = 0 .. N-1 with I a constant (for immediate offsets).
+template <int I, int N, class F>
+__device__ __forceinline__ void bpf_for(F f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        bpf_for<I + 1, N>(f);
+    }
+}
+
+// Footprint of one (pixel, view): first of the channels that can hold a nonzero tap (nc - 1, or with two taps nc - 1
+// or nc) and the coefficients of the channels from there (0 off the detector); fan geometries: row map A0 + k*A1,
+// c2 = (mag/D)^2 and the slice-height offset (translation).
+struct BpfFoot {
+    int ch;
+    float a[3];
+    float A0, A1, c2, zv;
+};
+
+// vw, one view's constants: x, y = cos, sin of the angle (translation: tx, ty); z = tz (translation) or delta_voxel /
+// cos_alpha (parallel); w = element offset of the view in the sinogram (int bits; -1: invalid view).
 template <int KIND>
-__device__ __forceinline__ void bpf_footprint(const mbx_geom &g, float cs, float sn, float x_tilde, float y_tilde,
-                                              int coeff_power, float4 &fa, float4 &fb, float tz = 0.0f) {
+__device__ __forceinline__ void bpf_footprint(const mbx_geom &g, const float4 &vw, float x_tilde, float y_tilde,
+                                              int coeff_power, bool two, BpfFoot &f) {
+    const float cs = vw.x, sn = vw.y;
     const float inv_dc = 1.0f / g.delta_det_channel;
     const int num_channels = g.num_det_channels;
     const float det_center_channel = 0.5f * (float)(num_channels - 1);
     float n_p, w, scale;  // scale = delta_voxel / cos_alpha
-    fb = make_float4(0.f, 0.f, 0.f, 0.f);
     if (KIND == MBX_GEOM_TRANSLATION) {
-        // (cs, sn) carry the view's (tx, ty); no rotation (translation_model.py:595-656).  Coefficient
-        // L / cos(theta_p), no delta_voxel factor; the vertical fan is the cone's with slice heights
-        // delta_voxel k + z0v, z0v = -tz - delta_voxel (S-1)/2, which fb.w carries.
+        // no rotation (translation_model.py:595-656).  Coefficient L / cos(theta_p), no delta_voxel factor; the
+        // vertical fan is the cone's with slice heights delta_voxel k + zv, zv = -tz - delta_voxel (S-1)/2.
         const float x_p = x_tilde - cs;
         const float y_p = y_tilde - sn;
         const float inv_d = 1.0f / g.source_detector_dist;
@@ -80,18 +152,18 @@ __device__ __forceinline__ void bpf_footprint(const mbx_geom &g, float cs, float
         w = mag * (g.delta_voxel * inv_dc);
         scale = 1.0f / cos_tp;
         const float inv_dr = 1.0f / g.delta_det_row;
-        const float z0v = -tz - g.delta_voxel * (0.5f * (float)(g.num_recon_slices - 1));
+        const float z0v = -vw.z - g.delta_voxel * (0.5f * (float)(g.num_recon_slices - 1));
         const float mr = mag * inv_d;
-        fb.x = (mag * z0v + g.det_row_offset) * inv_dr + 0.5f * (float)(g.num_det_rows - 1);
-        fb.y = mag * g.delta_voxel * inv_dr;
-        fb.z = mr * mr;
-        fb.w = z0v;
+        f.A0 = (mag * z0v + g.det_row_offset) * inv_dr + 0.5f * (float)(g.num_det_rows - 1);
+        f.A1 = mag * g.delta_voxel * inv_dr;
+        f.c2 = mr * mr;
+        f.zv = z0v;
     } else if (KIND == MBX_GEOM_PARALLEL) {
         const float x = cs * x_tilde - sn * y_tilde;
         n_p = (x + g.det_channel_offset) * inv_dc + det_center_channel;
         const float cos_alpha = fmaxf(fabsf(cs), fabsf(sn));
         w = (g.delta_voxel * inv_dc) * cos_alpha;
-        scale = g.delta_voxel / cos_alpha;
+        scale = vw.z;
     } else {
         const float x_p = cs * x_tilde - sn * y_tilde;
         const float y_p = sn * x_tilde + cs * y_tilde;
@@ -112,34 +184,35 @@ __device__ __forceinline__ void bpf_footprint(const mbx_geom &g, float cs, float
         const float center_slice = 0.5f * (float)(g.num_recon_slices - 1);
         const float z0 = g.recon_slice_offset - g.delta_voxel * center_slice;
         const float mr = mag * inv_d;
-        fb.x = (mag * z0 + g.det_row_offset) * inv_dr + 0.5f * (float)(g.num_det_rows - 1);
-        fb.y = mag * g.delta_voxel * inv_dr;
-        fb.z = mr * mr;
+        f.A0 = (mag * z0 + g.det_row_offset) * inv_dr + 0.5f * (float)(g.num_det_rows - 1);
+        f.A1 = mag * g.delta_voxel * inv_dr;
+        f.c2 = mr * mr;
+        f.zv = z0;
     }
     const int nc = (int)rintf(n_p);
     const float half_w = (w + 1.0f) * 0.5f;
     const float l_max = fminf(1.0f, w);
     const float d = n_p - (float)nc;
-    float a[3];
+    if (KIND == MBX_GEOM_PARALLEL && two) {
+        // w <= 1: the voxel reaches at most one of the two neighbours, the one on its side of the centre channel
+        const bool up = d > 0.0f;
+        f.ch = up ? nc : nc - 1;
+        const float c = scale * fminf(fmaxf(half_w - fabsf(d), 0.0f), l_max);
+        const float e = scale * fminf(fmaxf(half_w - fabsf(d - (up ? 1.0f : -1.0f)), 0.0f), l_max);
+        f.a[0] = up ? c : e;
+        f.a[1] = up ? e : c;
+        f.a[2] = 0.0f;
+    } else {
+        f.ch = nc - 1;
 #pragma unroll
-    for (int k = -1; k <= 1; ++k) {
-        const int n = nc + k;
-        float v = scale * fminf(fmaxf(half_w - fabsf(d - (float)k), 0.0f), l_max);
-        if (n < 0 || n >= num_channels) v = 0.0f;
-        a[k + 1] = (coeff_power == 2) ? v * v : v;
+        for (int k = 0; k < 3; ++k)
+            f.a[k] = scale * fminf(fmaxf(half_w - fabsf(d - (float)(k - 1)), 0.0f), l_max);
     }
-    // channels first..first+2 on the detector; tap k of the pixel sits at position k - (first - (nc - 1))
-    const int lo = nc - 1;
-    const int first = min(max(lo, 0), num_channels - 3);
-    const int sh = first - lo;
-    float c[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const int j = k + sh;
-        c[k] = (j == 0) ? a[0] : ((j == 1) ? a[1] : ((j == 2) ? a[2] : 0.0f));
+        if ((unsigned)(f.ch + k) >= (unsigned)num_channels) f.a[k] = 0.0f;
+        if (coeff_power == 2) f.a[k] *= f.a[k];
     }
-    const bool any = c[0] != 0.0f || c[1] != 0.0f || c[2] != 0.0f;
-    fa = make_float4(__int_as_float(any ? first : -1), c[0], c[1], c[2]);
 }
 
 // Pixel position relative to the recon centre (ALU): x from the column, y from the row (translation geometry
@@ -161,6 +234,10 @@ struct BpArgs {
     mbx_geom g;
     const float *sino;         // full sinogram (num_views, R, C)
     const float *wts;          // optional weights, same shape (NULL: ones)
+    const float *tsino;        // weights x sinogram of the call's views as (view, channel, rp rows), or NULL
+    int rp;                    // rows of tsino, a multiple of 4 (0 past num_det_rows)
+    const CUtensorMap *tmap;   // its tensor map (batched lists; a plain launch passes the map as a parameter)
+    int tsino_all;             // tsino holds every view of the geometry (else the selected views in their order)
     const int32_t *pix;        // (num_pixels,) flat pixel indices
     long long num_pixels;
     const int32_t *order;      // optional permutation of [0, num_pixels): processing order (locality)
@@ -189,262 +266,502 @@ inline mbx_geom one_slice_geometry(const mbx_geom &g) {
     return g1;
 }
 
-// Parallel-beam gather of one view into the first TS accumulators: three taps at constant offsets from one
-// 32-bit element offset, one detector row per slice (TS = the tile's slice count, so no slot is predicated off).
-template <int TS>
-__device__ __forceinline__ void bpf_gather_rows(float (&acc)[BPF_ST], const float *__restrict__ sino, int o,
-                                                int num_channels, const float4 &fa) {
-#pragma unroll
-    for (int s = 0; s < TS; ++s) {
-        const float *q = sino + o;
-        acc[s] = fmaf(fa.y, __ldg(q), fmaf(fa.z, __ldg(q + 1), fmaf(fa.w, __ldg(q + 2), acc[s])));
-        o += num_channels;
+// Read-only load of *p when ok, else 0 (a predicated load: no branch, so several stay in flight).
+__device__ __forceinline__ float bpf_ldg(const float *p, bool ok) {
+    float v = 0.0f;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}" : "+f"(v) : "l"(p), "r"((int)ok));
+    return v;
+}
+
+// One warp's TMA barriers (one per window buffer; byte addresses in shared memory) and their phase parities.
+struct BpfPipe {
+    unsigned bar;
+    unsigned parity;  // bit b: parity that buffer b waits for next
+};
+
+__device__ __forceinline__ BpfPipe bpf_pipe_init(float *at) {
+    BpfPipe p;
+    p.bar = (unsigned)__cvta_generic_to_shared(at);
+    p.parity = 0;
+    if ((threadIdx.x & 31) == 0) {
+        asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(p.bar) : "memory");
+        asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(p.bar + 8) : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    return p;
+}
+
+// Waits for buffer b's copy (bounded: a copy that never completes is flagged, not waited for).
+__device__ __forceinline__ void bpf_pipe_wait(BpfPipe &p, int b, int *err) {
+    const unsigned bar = p.bar + 8u * (unsigned)b, par = (p.parity >> b) & 1u;
+    unsigned done = 0;
+    for (int i = 0; i < (1 << 22) && !done; ++i)
+        asm volatile("{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                     : "=r"(done)
+                     : "r"(bar), "r"(par)
+                     : "memory");
+    if (!done) flag_error(err, MBX_ERRFLAG_CACHE);
+    p.parity ^= 1u << b;
+}
+
+// True in one lane of the (converged) warp, by elect.sync, which the compiler knows to leave a single thread: it then
+// issues the TMA instructions without a loop over the threads that might execute them.
+__device__ __forceinline__ bool bpf_elect() {
+    unsigned one;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
+// Starts the TMA copy of channels c .. c + nch - 1 (rows of the transposed copy, counted over views and edge channels)
+// and rows r0 .. (a multiple of 4) into buffer b at win; rows outside the copy arrive as zeros.  c, nch, r0 and b are the
+// warp's.
+__device__ __forceinline__ void bpf_stage_tma(float *win, const BpArgs &A, const CUtensorMap *tmap, const BpfPipe &p,
+                                              int b, int r0, int c, int nch) {
+    const unsigned box = 16u * BPF_BOX * (unsigned)A.plan.boxq;
+    const int n = (nch + BPF_BOX - 1) / BPF_BOX;
+    c = __shfl_sync(0xffffffffu, c, 0);
+    r0 = __shfl_sync(0xffffffffu, r0, 0);
+    unsigned dst = __shfl_sync(0xffffffffu, (unsigned)__cvta_generic_to_shared(win), 0);
+    const unsigned bar = __shfl_sync(0xffffffffu, p.bar + 8u * (unsigned)b, 0);
+    if (bpf_elect()) {
+        asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(bar), "r"(box * (unsigned)n) : "memory");
+        for (int i = 0; i < n; ++i, dst += box, c += BPF_BOX)
+            asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                         ::"r"(dst), "l"(tmap), "r"(r0), "r"(c), "r"(bar)
+                         : "memory");
     }
 }
 
-// The same for a tile of TS slices when TS fits the accumulators (other TS never occur: ns <= ts <= BPF_ST).
-template <int TS>
-__device__ __forceinline__ void bpf_gather_ts(float (&acc)[BPF_ST], const float *__restrict__ sino, int o,
-                                              int num_channels, const float4 &fa) {
-    if constexpr (TS <= BPF_ST) bpf_gather_rows<TS>(acc, sino, o, num_channels, fa);
+// Copies rows r0 .. r0 + 4 nq - 1 of channels c_lo .. c_lo + nch - 1 of one view (element offset voff of the sinogram)
+// into win ([channel][row], channel pitch `pitch`), by one warp: lanes along channels, four rows per lane and 16-byte
+// store, the weights multiplied in, zeros off the detector; a NULL sinogram is all ones.
+__device__ __forceinline__ float4 bpf_four_rows(const BpArgs &A, int voff, int r, int n) {
+    const int num_channels = A.g.num_det_channels, num_rows = A.g.num_det_rows;
+    const bool cok = n >= 0 && n < num_channels;
+    const int o = voff + r * num_channels + n;
+    float v[4], w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const bool ok = cok && r + j >= 0 && r + j < num_rows;
+        v[j] = A.sino ? bpf_ldg(A.sino + (o + j * num_channels), ok) : (ok ? 1.0f : 0.0f);
+    }
+    if (A.wts) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            w[j] = bpf_ldg(A.wts + (o + j * num_channels), cok && r + j >= 0 && r + j < num_rows);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] *= w[j];
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <int KIND>
-__device__ void bp_fast_tile(const BpArgs &A, int bx, int by, int bz, float *smf, int *err) {
-    const mbx_geom &g = A.g;
-    const BpfPlan &P = A.plan;
-    const float *__restrict__ sino = A.sino;
-    const float *__restrict__ wts = A.wts;
-    const int32_t *__restrict__ pix = A.pix;
-    const long long num_pixels = A.num_pixels;
-    const int32_t *__restrict__ views = A.views;
-    const int num_views_sel = A.num_views_sel, views_per_split = A.views_per_split, coeff_power = A.coeff_power;
-    const int nsl = P.nsl, vc = P.vc, lg_pcta = P.lg_pcta, chunk = P.chunk;
-    const int pcta = 1 << lg_pcta;                  // pixels per CTA
-    float4 *s_fa = reinterpret_cast<float4 *>(smf);  // [chunk] = [view in chunk][pixel]
-    float4 *s_fb = s_fa + chunk;                     // cone: [chunk]
-    float *s_cs = reinterpret_cast<float *>(s_fa + (KIND != MBX_GEOM_PARALLEL ? 2 : 1) * chunk);
-    float *s_sn = s_cs + vc;
-    int *s_voff = reinterpret_cast<int *>(s_sn + vc);      // element offset of each view (-1: invalid view)
-    float *s_tz = reinterpret_cast<float *>(s_voff + vc);   // translation: tz of each view
-    float *cache = s_tz + (KIND == MBX_GEOM_TRANSLATION ? vc : 0);  // [BPF_CACHE_ROWS][BPF_THREADS] (cone, transl.)
+__device__ __forceinline__ void bpf_stage(float *win, const BpArgs &A, int voff, int r0, int nq, int pitch, int c_lo,
+                                          int nch, int lane) {
+    const int items = nch * nq;  // at most 416; the quotients below are exact while items * nch < 2^18
+    const unsigned inv = ((1u << 18) + (unsigned)nch - 1u) / (unsigned)nch;
+#pragma unroll 2
+    for (int it = lane; it < items; it += 32) {
+        const int q = (int)(((unsigned)it * inv) >> 18);
+        const int c = it - q * nch;
+        *reinterpret_cast<float4 *>(win + c * pitch + 4 * q) = bpf_four_rows(A, voff, r0 + 4 * q, c_lo + c);
+    }
+}
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pg = warp / nsl, stl = warp - pg * nsl;
-    const int pl = pg * 32 + lane;                                   // pixel within CTA
-    const long long slot = (long long)bx * pcta + pl;
-    const long long p = (A.order && slot < num_pixels) ? A.order[slot] : slot;  // list entry of this thread
-    const int s0 = (by * nsl + stl) * P.ts;
-    const int num_rows = g.num_det_rows, num_channels = g.num_det_channels, num_slices = g.num_recon_slices;
-    const int ns = min(P.ts, num_slices - s0);
-    const int split = bz;
-    const int v_begin = split * views_per_split;
-    const int v_end = min(num_views_sel, v_begin + views_per_split);
-    const int npix_grid = g.num_recon_rows * g.num_recon_cols;
-    const int view_stride = num_rows * num_channels;  // plan_bp_fast admits sinograms of < 2^31 elements
-    const int s0c = s0 * num_channels;
-
-    // pixel geometry of the pixel this thread computes footprints for (pixel tid % pcta of every view)
-    const int fpl = tid & (pcta - 1);
-    const long long fp_slot = (long long)bx * pcta + fpl;
-    const long long fp_pixel = (A.order && fp_slot < num_pixels) ? A.order[fp_slot] : fp_slot;
-    float fxt = 0.0f, fyt = 0.0f;
-    bool fvalid = false;
-    if (fp_pixel < num_pixels) {
-        const int idx = pix[fp_pixel];
-        if (idx >= 0 && idx < npix_grid) {
-            bpf_pixel<KIND>(g, idx, fxt, fyt);
-            fvalid = true;
-        } else if (by == 0 && split == 0 && tid < pcta) {
-            flag_error(err, MBX_ERRFLAG_PIXEL);
+// A lane's own channels ch .. ch + taps - 1, rows r0 .. r0 + 4 nq - 1, into its private columns at win.
+template <bool TR>
+__device__ __forceinline__ void bpf_stage_private(float *win, const BpArgs &A, int voff, int r0, int nq, int pitch,
+                                                  int ch, int taps) {
+    for (int k = 0; k < taps; ++k) {
+        float *dst = win + k * pitch;
+        if constexpr (TR) {  // (a lane's taps lie on the view's channels or its edge channels)
+            const float *src = A.tsino + (long long)(voff + ch + k + BPF_EDGE) * A.rp;
+            for (int q = 0, r = r0; q < nq; ++q, r += 4) {
+                const bool ok = r >= 0 && r < A.rp;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;"
+                             ::"r"((unsigned)__cvta_generic_to_shared(dst + 4 * q)), "l"(ok ? src + r : A.tsino), "r"(ok ? 16 : 0)
+                             : "memory");
+            }
+        } else {
+            for (int q = 0; q < nq; ++q)
+                *reinterpret_cast<float4 *>(dst + 4 * q) = bpf_four_rows(A, voff, r0 + 4 * q, ch + k);
         }
     }
-    bool active = p < num_pixels && ns > 0;
-    float oxt = 0.0f, oyt = 0.0f;  // this thread's own pixel (inline footprints)
+}
+
+// Waits for this warp's private columns.
+template <bool TR>
+__device__ __forceinline__ void bpf_private_wait() {
+    if (TR) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the next TMA copy into the buffer
+    }
+}
+
+// The constants of view v of a call, see bpf_footprint.
+template <int KIND, bool TR>
+__device__ __forceinline__ float4 bpf_view(const BpArgs &A, int v, bool flag, int *err) {
+    const mbx_geom &g = A.g;
+    const int vi = A.views ? A.views[v] : v;
+    const bool ok = vi >= 0 && vi < g.num_views;
+    if (!ok && flag) flag_error(err, MBX_ERRFLAG_VIEW);
+    float4 vw;
+    if (KIND == MBX_GEOM_TRANSLATION) {
+        vw.x = ok ? g.translations[3 * vi] : 0.0f;
+        vw.y = ok ? g.translations[3 * vi + 1] : 0.0f;
+        vw.z = ok ? g.translations[3 * vi + 2] : 0.0f;
+    } else {
+        const float ang = ok ? g.angles[vi] : 0.0f;
+        vw.x = cosf(ang);
+        vw.y = sinf(ang);
+        vw.z = KIND == MBX_GEOM_PARALLEL ? g.delta_voxel / fmaxf(fabsf(vw.x), fabsf(vw.y)) : 0.0f;
+    }
+    // TR: first channel of the view in the transposed copy; otherwise the element offset of the view
+    vw.w = __int_as_float(!ok ? -1
+                          : TR ? (A.tsino_all ? vi : v) * (g.num_det_channels + 2 * BPF_EDGE)
+                               : vi * (g.num_det_rows * g.num_det_channels));
+    return vw;
+}
+
+// Lanes of one pass over a view: those whose taps (channels ch .. ch + taps - 1) start within `cap` channels of the
+// lowest remaining one.
+struct BpfPass {
+    int c_lo, nch;
+    bool in;
+};
+
+__device__ __forceinline__ BpfPass bpf_pass(bool todo, int ch, int taps, int cap) {
+    BpfPass q;
+    q.c_lo = __reduce_min_sync(0xffffffffu, todo ? ch : INT_MAX);
+    q.in = todo && ch + taps - q.c_lo <= cap;
+    q.nch = __reduce_max_sync(0xffffffffu, q.in ? ch + taps - q.c_lo : 0);
+    return q;
+}
+
+// What one pass over a view needs after its window has arrived.
+struct BpfItem {
+    bool in;       // this lane takes part
+    bool tma;      // the window comes by TMA
+    int off;       // window offset of the lane's first channel
+    int row0;      // fan: detector row of the row buffer's row 0
+    int nq;        // fan: row-buffer rows in fours
+    float a[3];
+    float A0, A1, c2, zv;
+};
+
+// 1 / sqrt(x) for x >= 1 (rsqrtf without its scaling of denormals).
+__device__ __forceinline__ float bpf_rsqrt(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// The vertical fan of one pass: adds to acc the slices k_first .. of a tile (nsq fours) from the row sums in cache
+// ([row][lane], row 0 = detector row it.row0).  Two slices at a time; the row of slice k, rint(A0 + k A1), comes from
+// adding and removing 1.5 x 2^23, whose low mantissa bits are then the row (|row| < 2^22).  A voxel overlaps rows m_c
+// - 1, m_c, m_c + 1 by min(max(half_w - |m_p - m|, 0), l_max); with d = m_p - m_c in [-1/2, 1/2] and A1 <= 2 the clips
+// that cannot act are left out (WIDE: A1 > 2).  POWER: coefficients raised to coeff_power (1 otherwise).
+template <bool POWER, bool WIDE>
+__device__ __forceinline__ void bpf_vertical(bpf2 (&acc)[BPF_ST / 2], const BpfItem &it, const float *cache,
+                                             float k_first, int nsq, float delta_voxel, int coeff_power) {
+    const float magic = 12582912.0f;
+    // byte address of a row: its bits x 128 plus this (modulo 2^32)
+    const unsigned base = (unsigned)__cvta_generic_to_shared(cache) -
+                          ((unsigned)__float_as_int(magic) + (unsigned)it.row0) * 128u;
+    const float half_w = (it.A1 + 1.0f) * 0.5f;
+    const float l_max = fminf(1.0f, it.A1);
+    const float hw1 = half_w - 1.0f;
+    const bpf2 A1p = bpf_pair(it.A1, it.A1), A0p = bpf_pair(it.A0, it.A0);
+    const bpf2 mgp = bpf_pair(magic, magic), mgn = bpf_pair(-magic, -magic);
+    const bpf2 neg = bpf_pair(-1.0f, -1.0f), one = bpf_pair(1.0f, 1.0f), two = bpf_pair(2.0f, 2.0f);
+    const bpf2 hw1p = bpf_pair(hw1, hw1), c2p = bpf_pair(it.c2, it.c2);
+    const bpf2 dvp = bpf_pair(delta_voxel, delta_voxel), zvp = bpf_pair(it.zv, it.zv);
+    bpf2 k = bpf_pair(k_first, k_first + 1.0f);
+#pragma unroll
+    for (int q4 = 0; q4 < BPF_ST / 4; ++q4) {
+        if (q4 >= nsq) break;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const bpf2 m_p = bpf_fma(k, A1p, A0p);
+            const bpf2 mr = bpf_add(m_p, mgp);
+            float ma, mb;
+            bpf_unpair(mr, ma, mb);
+            const unsigned ra = base + (unsigned)__float_as_int(ma) * 128u;
+            const unsigned rb = base + (unsigned)__float_as_int(mb) * 128u;
+            const bpf2 cm = bpf_pair(bpf_lds<-128>(ra), bpf_lds<-128>(rb));
+            const bpf2 c0 = bpf_pair(bpf_lds<0>(ra), bpf_lds<0>(rb));
+            const bpf2 cp = bpf_pair(bpf_lds<128>(ra), bpf_lds<128>(rb));
+            const bpf2 d = bpf_fma(bpf_add(mr, mgn), neg, m_p);
+            const bpf2 z = bpf_fma(k, dvp, zvp);
+            const bpf2 q = bpf_fma(c2p, bpf_mul(z, z), one);
+            float qa, qb, da, db, ma1, mb1, pa1, pb1;
+            bpf_unpair(q, qa, qb);
+            bpf2 sec = bpf_mul(q, bpf_pair(bpf_rsqrt(qa), bpf_rsqrt(qb)));  // 1 / cos(phi_k)
+            bpf_unpair(d, da, db);
+            bpf_unpair(bpf_fma(d, neg, hw1p), ma1, mb1);
+            bpf_unpair(bpf_add(d, hw1p), pa1, pb1);
+            ma1 = fmaxf(ma1, 0.0f);
+            mb1 = fmaxf(mb1, 0.0f);
+            pa1 = fmaxf(pa1, 0.0f);
+            pb1 = fmaxf(pb1, 0.0f);
+            if (WIDE) {
+                ma1 = fminf(ma1, l_max);
+                mb1 = fminf(mb1, l_max);
+                pa1 = fminf(pa1, l_max);
+                pb1 = fminf(pb1, l_max);
+            }
+            bpf2 l_m = bpf_pair(ma1, mb1), l_p = bpf_pair(pa1, pb1);
+            bpf2 l_0 = bpf_pair(fminf(half_w - fabsf(da), l_max), fminf(half_w - fabsf(db), l_max));
+            if (POWER && (!WIDE || coeff_power == 2)) {
+                sec = bpf_mul(sec, sec);
+                l_m = bpf_mul(l_m, l_m);
+                l_0 = bpf_mul(l_0, l_0);
+                l_p = bpf_mul(l_p, l_p);
+            }
+            const bpf2 x = bpf_fma(l_m, cm, bpf_fma(l_0, c0, bpf_mul(l_p, cp)));
+            acc[2 * q4 + h] = bpf_fma(sec, x, acc[2 * q4 + h]);
+            k = bpf_add(k, two);
+        }
+    }
+}
+
+// One warp's unit of work: pixel group pg (32 list entries), slice tile st, view split `split`; smw: bpf_warp_floats
+// of shared memory of its own.  No barrier beyond the warp.  The window of the next pass is copied while the current
+// one is used: into a second buffer (parallel), or into the one buffer once the horizontal sums have been taken from
+// it, during the vertical fan (fan geometries).
+template <int KIND, bool TR, bool TWO>
+__device__ __forceinline__ void bp_fast_unit(const BpArgs &A, const CUtensorMap *tmap, int pg, int st, int split, float *smw, BpfPipe &pipe,
+                                             int *err) {
+    constexpr bool FAN = KIND != MBX_GEOM_PARALLEL;
+    constexpr int WIN = FAN ? BPF_WIN_FAN : BPF_WIN_PARALLEL;
+    constexpr unsigned ALL = 0xffffffffu;
+    const mbx_geom &g = A.g;
+    const BpfPlan &P = A.plan;
+    const int32_t *__restrict__ pix = A.pix;
+    const long long num_pixels = A.num_pixels;
+    const int num_views_sel = A.num_views_sel, views_per_split = A.views_per_split, coeff_power = A.coeff_power;
+
+    constexpr int TAPS = TWO ? 2 : 3;
+
+    const int lane = threadIdx.x & 31;
+    float *cache = smw + WIN + lane;                           // fan: row buffer [row][lane]
+    const int pitch = 4 * P.boxq;                              // of a window's channels
+    const int cap = WIN / pitch & ~(BPF_BOX - 1);              // channels of a window
+
+    const long long slot = (long long)pg * 32 + lane;
+    const long long p = (A.order && slot < num_pixels) ? A.order[slot] : slot;  // list entry of this thread
+    const int s0 = st * P.ts;
+    const int num_slices = g.num_recon_slices;
+    const int ns = min(P.ts, num_slices - s0);   // slices of this warp's tile
+    if (ns <= 0) return;
+    const int nsq = (ns + 3) >> 2;               // the same in fours: the slices past ns are computed, not written
+    const float k_first = (float)s0, k_last = (float)(s0 + 4 * nsq - 1);
+    const int v_end = min(num_views_sel, (split + 1) * views_per_split);
+    const int npix_grid = g.num_recon_rows * g.num_recon_cols;
+
+    bool active = p < num_pixels;
+    float xt = 0.0f, yt = 0.0f;
     if (active) {
         const int idx = pix[p];
         active = idx >= 0 && idx < npix_grid;
-        if (active) bpf_pixel<KIND>(g, idx, oxt, oyt);
+        if (active)
+            bpf_pixel<KIND>(g, idx, xt, yt);
+        else if (st == 0 && split == 0)
+            flag_error(err, MBX_ERRFLAG_PIXEL);
     }
 
-    float acc[BPF_ST];
+    bpf2 acc[BPF_ST / 2];
 #pragma unroll
-    for (int s = 0; s < BPF_ST; ++s) acc[s] = 0.0f;
+    for (int s = 0; s < BPF_ST / 2; ++s) acc[s] = 0ull;
 
-    const float z0 = g.recon_slice_offset - g.delta_voxel * 0.5f * (float)(num_slices - 1);
-    float *mycache = cache + tid;
+    float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);  // constants of view (first of 32) + lane
+    int v = split * views_per_split, t = 0;         // next view, its place among those constants
+    int voff = 0;                                   // current view: offset, footprint, lanes not yet in a pass
+    BpfFoot f;
+    bool todo = false;
+    // fan, current view: the rows of the warp's window
+    int r0 = 0, nq = 0;
+    bool fits = true;
 
-    // gather of one view into the accumulators, from the footprint fa (+ fb for cone) at view offset voff
-    auto gather = [&](const float4 &fa, const float4 &fb, int voff) {
-        const int first = __float_as_int(fa.x);
-        if (KIND == MBX_GEOM_PARALLEL) {
-            // three taps at constant offsets from one 32-bit element offset, one detector row per slice
-            int o = voff + s0c + first;
-            if (!sino) {  // unit sinogram: the same additions as gathering ones (unit-weight Hessian)
+    // the next pass: its lanes, and the copy of its window into win started; false when the views are done
+    auto next = [&](BpfItem &it, float *win, int b) -> bool {
+        while (!__any_sync(ALL, todo)) {
+            if (v >= v_end) return false;
+            if (t == 0) mine = bpf_view<KIND, TR>(A, min(v + lane, v_end - 1), pg == 0 && st == 0, err);
+            float4 vw;
+            vw.x = __shfl_sync(ALL, mine.x, t);
+            vw.y = __shfl_sync(ALL, mine.y, t);
+            vw.z = __shfl_sync(ALL, mine.z, t);
+            vw.w = __shfl_sync(ALL, mine.w, t);
+            ++v;
+            t = (t + 1) & 31;
+            voff = __float_as_int(vw.w);
+            if (voff < 0) continue;
+            bpf_footprint<KIND>(g, vw, xt, yt, coeff_power, TWO, f);
+            todo = active && (f.a[0] != 0.0f || f.a[1] != 0.0f || f.a[2] != 0.0f);
+            if constexpr (FAN) {
+                // detector rows of this lane's slices (the affine map is monotone in the slice)
+                const float m_a = rintf(fmaf(k_first, f.A1, f.A0)), m_b = rintf(fmaf(k_last, f.A1, f.A0));
+                // rows near the detector (a NaN or a row far off it would not be an index): others add 0, or the NaN
+                if (todo && !(fabsf(m_a) < 4.0e6f && fabsf(m_b) < 4.0e6f)) {
+                    const float nan_or_0 = 0.0f * (m_a + m_b);
 #pragma unroll
-                for (int s = 0; s < BPF_ST; ++s)
-                    if (s < ns) acc[s] = fa.y + (fa.z + (fa.w + acc[s]));
-            } else if (wts) {
-#pragma unroll
-                for (int s = 0; s < BPF_ST; ++s) {
-                    if (s < ns) {
-                        const float *q = sino + o, *qw = wts + o;
-                        acc[s] = fmaf(fa.y, __ldg(q) * __ldg(qw),
-                                      fmaf(fa.z, __ldg(q + 1) * __ldg(qw + 1), fmaf(fa.w, __ldg(q + 2) * __ldg(qw + 2), acc[s])));
-                    }
-                    o += num_channels;
+                    for (int s = 0; s < BPF_ST / 2; ++s) acc[s] = bpf_add(acc[s], bpf_pair(nan_or_0, nan_or_0));
+                    todo = false;
                 }
-            } else {
-                switch (ns) {  // the same for every lane of the warp (a warp holds one slice tile)
-                    case 1: bpf_gather_ts<1>(acc, sino, o, num_channels, fa); break;
-                    case 2: bpf_gather_ts<2>(acc, sino, o, num_channels, fa); break;
-                    case 3: bpf_gather_ts<3>(acc, sino, o, num_channels, fa); break;
-                    case 4: bpf_gather_ts<4>(acc, sino, o, num_channels, fa); break;
-                    case 5: bpf_gather_ts<5>(acc, sino, o, num_channels, fa); break;
-                    case 6: bpf_gather_ts<6>(acc, sino, o, num_channels, fa); break;
-                    case 7: bpf_gather_ts<7>(acc, sino, o, num_channels, fa); break;
-                    case 8: bpf_gather_ts<8>(acc, sino, o, num_channels, fa); break;
-                    case 9: bpf_gather_ts<9>(acc, sino, o, num_channels, fa); break;
-                    case 10: bpf_gather_ts<10>(acc, sino, o, num_channels, fa); break;
-                    case 11: bpf_gather_ts<11>(acc, sino, o, num_channels, fa); break;
-                    case 12: bpf_gather_ts<12>(acc, sino, o, num_channels, fa); break;
-                    case 13: bpf_gather_ts<13>(acc, sino, o, num_channels, fa); break;
-                    case 14: bpf_gather_ts<14>(acc, sino, o, num_channels, fa); break;
-                    case 15: bpf_gather_ts<15>(acc, sino, o, num_channels, fa); break;
-                    default: bpf_gather_rows<BPF_ST>(acc, sino, o, num_channels, fa); break;
-                }
-            }
-        } else {
-            const float A0 = fb.x, A1 = fb.y, c2 = fb.z;
-            const float half_w = (A1 + 1.0f) * 0.5f;
-            const float l_max = fminf(1.0f, A1);
-            const int mc_first = (int)rintf(fmaf((float)s0, A1, A0));
-            const int mc_last = (int)rintf(fmaf((float)(s0 + ns - 1), A1, A0));
-            const int m_lo = min(mc_first, mc_last) - 1;
-            const int m_hi = max(mc_first, mc_last) + 1;
-            if (m_hi - m_lo + 1 > BPF_CACHE_ROWS) {  // excluded by plan_bp_fast; never read past the cache
-                flag_error(err, MBX_ERRFLAG_CACHE);
-                return;
-            }
-            for (int m = m_lo; m <= m_hi; ++m) {
-                float c = 0.0f;
-                if (m >= 0 && m < num_rows) {
-                    const int o = voff + m * num_channels + first;
-                    const float *q = sino + o;
-                    if (!sino) {  // unit sinogram
-                        c = fa.y + (fa.z + fa.w);
-                    } else if (wts) {
-                        const float *qw = wts + o;
-                        c = fmaf(fa.y, __ldg(q) * __ldg(qw), fmaf(fa.z, __ldg(q + 1) * __ldg(qw + 1), fa.w * (__ldg(q + 2) * __ldg(qw + 2))));
-                    } else {
-                        c = fmaf(fa.y, __ldg(q), fmaf(fa.z, __ldg(q + 1), fa.w * __ldg(q + 2)));
-                    }
-                }
-                mycache[(m - m_lo) * BPF_THREADS] = c;
-            }
-#pragma unroll
-            for (int s = 0; s < BPF_ST; ++s) {
-                if (s < ns) {
-                    const float k = (float)(s0 + s);
-                    const float m_p = fmaf(k, A1, A0);
-                    const int m_c = (int)rintf(m_p);
-                    const float d = m_p - (float)m_c;
-                    const float z = fmaf(k, g.delta_voxel, KIND == MBX_GEOM_TRANSLATION ? fb.w : z0);
-                    const float q = fmaf(c2, z * z, 1.0f);
-                    float sec = q * rsqrtf(q);                       // 1 / cos(phi_k)
-                    const float l_m = fminf(fmaxf(half_w - fabsf(d + 1.0f), 0.0f), l_max);
-                    const float l_0 = fminf(fmaxf(half_w - fabsf(d), 0.0f), l_max);
-                    const float l_p = fminf(fmaxf(half_w - fabsf(d - 1.0f), 0.0f), l_max);
-                    const float *cc = mycache + (m_c - m_lo) * BPF_THREADS;
-                    const float cm = cc[-BPF_THREADS], c0 = cc[0], cp = cc[BPF_THREADS];
-                    if (coeff_power == 2) {
-                        sec *= sec;
-                        acc[s] = fmaf(sec, fmaf(l_m * l_m, cm, fmaf(l_0 * l_0, c0, (l_p * l_p) * cp)), acc[s]);
-                    } else {
-                        acc[s] = fmaf(sec, fmaf(l_m, cm, fmaf(l_0, c0, l_p * cp)), acc[s]);
+                const int m_lo = (int)fminf(m_a, m_b) - 1, m_hi = (int)fmaxf(m_a, m_b) + 1;
+                r0 = __reduce_min_sync(ALL, todo ? m_lo : INT_MAX) & ~3;
+                nq = (__reduce_max_sync(ALL, todo ? m_hi : INT_MIN) - r0 + 4) >> 2;
+                fits = nq <= P.boxq;
+                if (!fits) {  // each lane's own rows (of no use when no lane is to do)
+                    r0 = m_lo & ~3;
+                    nq = (m_hi - r0 + 4) >> 2;
+                    if (todo && nq > P.boxq) {  // excluded by plan_bp_fast
+                        flag_error(err, MBX_ERRFLAG_CACHE);
+                        todo = false;
                     }
                 }
             }
         }
-    };
-
-    // per-view table of a chunk of views: angle cos/sin and element offset (-1: invalid view)
-    auto fill_views = [&](int vb, int nv) {
-        for (int t = tid; t < nv; t += BPF_THREADS) {
-            const int vi = views ? views[vb + t] : vb + t;
-            const bool ok = vi >= 0 && vi < g.num_views;
-            if (!ok && bx == 0 && by == 0) flag_error(err, MBX_ERRFLAG_VIEW);
-            s_voff[t] = ok ? vi * view_stride : -1;
-            if (KIND == MBX_GEOM_TRANSLATION) {  // (tx, ty) in the (cos, sin) slots, tz in its own table
-                s_cs[t] = ok ? g.translations[3 * vi] : 0.0f;
-                s_sn[t] = ok ? g.translations[3 * vi + 1] : 0.0f;
-                s_tz[t] = ok ? g.translations[3 * vi + 2] : 0.0f;
-            } else {
-                const float ang = ok ? g.angles[vi] : 0.0f;
-                s_cs[t] = cosf(ang);
-                s_sn[t] = sinf(ang);
-            }
+        const BpfPass w = bpf_pass(todo, f.ch, TAPS, fits ? cap : TAPS);
+        bool window = fits;
+        if (fits && __any_sync(ALL, todo && !w.in)) {  // several windows: unless they would be many
+            const int bucket = todo ? min((f.ch - w.c_lo) / BPF_SPLIT, 31) : 31;
+            window = __popc(__reduce_or_sync(ALL, todo ? 1u << bucket : 0u)) <= BPF_WINDOWS;
         }
+        it.tma = TR && window;
+        it.in = w.in;
+        it.off = (f.ch - w.c_lo) * pitch;
+        if (window) {
+            if (TR)
+                bpf_stage_tma(win, A, tmap, pipe, b, FAN ? r0 : s0, voff + w.c_lo + BPF_EDGE, w.nch);
+            else
+                bpf_stage(win, A, voff, FAN ? r0 : s0, FAN ? nq : nsq, pitch, w.c_lo, w.nch, lane);
+        } else {  // as many lanes as there is room for, each with columns of its own
+            const int rank = __popc(__ballot_sync(ALL, todo) & ((1u << lane) - 1u));
+            it.in = todo && rank < WIN / (TAPS * pitch);
+            it.off = rank * (TAPS * pitch);
+            if (it.in)
+                bpf_stage_private<TR>(win + it.off, A, voff, FAN ? r0 : s0, FAN ? nq : nsq, pitch, f.ch, TAPS);
+        }
+        it.row0 = r0;
+        it.nq = nq;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) it.a[k] = f.a[k];
+        it.A0 = f.A0;
+        it.A1 = f.A1;
+        it.c2 = f.c2;
+        it.zv = f.zv;
+        todo = todo && !it.in;
+        return true;
     };
 
-    if (P.inline_fp) {
-        for (int vb = v_begin; vb < v_end; vb += vc) {
-            const int nv = min(vc, v_end - vb);
-            __syncthreads();
-            fill_views(vb, nv);
-            __syncthreads();
-            if (!active) continue;
-            for (int t = 0; t < nv; ++t) {
-                const int voff = s_voff[t];
-                if (voff < 0) continue;
-                float4 fa, fb;
-                bpf_footprint<KIND>(g, s_cs[t], s_sn[t], oxt, oyt, coeff_power, fa, fb,
-                                    KIND == MBX_GEOM_TRANSLATION ? s_tz[t] : 0.0f);
-                if (__float_as_int(fa.x) >= 0) gather(fa, fb, voff);
+    BpfItem cur, nxt;
+    bool have = false;
+    if (!FAN && !TR && !A.sino) {
+        // unit sinogram: the same additions as gathering ones (the unit-weight Hessian, usually of one slice)
+        for (; v < v_end; ++v, t = (t + 1) & 31) {
+            if (t == 0) mine = bpf_view<KIND, TR>(A, min(v + lane, v_end - 1), pg == 0 && st == 0, err);
+            float4 vw;
+            vw.x = __shfl_sync(ALL, mine.x, t);
+            vw.y = __shfl_sync(ALL, mine.y, t);
+            vw.z = __shfl_sync(ALL, mine.z, t);
+            vw.w = __shfl_sync(ALL, mine.w, t);
+            if (__float_as_int(vw.w) < 0) continue;
+            bpf_footprint<KIND>(g, vw, xt, yt, coeff_power, TWO, f);
+            if (active)
+#pragma unroll
+                for (int s = 0; s < BPF_ST / 2; ++s)
+                    if (2 * s < ns)
+                        acc[s] = bpf_add(bpf_pair(f.a[0], f.a[0]),
+                                         bpf_add(bpf_pair(f.a[1], f.a[1]), bpf_add(bpf_pair(f.a[2], f.a[2]), acc[s])));
+        }
+    } else if constexpr (!FAN) {
+        int b = 0;
+        for (;;) {
+            const bool more = next(nxt, smw + (b ^ 1) * WIN, b ^ 1);
+            if (have) {
+                if (TR && cur.tma)
+                    bpf_pipe_wait(pipe, b, err);
+                else
+                    bpf_private_wait<TR>();
+                __syncwarp();
+                const bpf2 a0 = bpf_pair(cur.a[0], cur.a[0]), a1 = bpf_pair(cur.a[1], cur.a[1]),
+                           a2 = bpf_pair(cur.a[2], cur.a[2]);
+                if (cur.in) {
+                    const unsigned w0 = (unsigned)__cvta_generic_to_shared(smw + b * WIN + cur.off);
+                    const unsigned w1 = w0 + 4u * (unsigned)pitch, w2 = w1 + 4u * (unsigned)pitch;
+                    bpf_for<0, BPF_ST / 4>([&](auto i) {
+                        constexpr int q = decltype(i)::value;
+                        if (q < nsq) {
+                            bpf2 x, y;
+                            if constexpr (!TWO) {
+                                bpf_lds4<16 * q>(w2, x, y);
+                                acc[2 * q] = bpf_fma(a2, x, acc[2 * q]);
+                                acc[2 * q + 1] = bpf_fma(a2, y, acc[2 * q + 1]);
+                            }
+                            bpf_lds4<16 * q>(w1, x, y);
+                            acc[2 * q] = bpf_fma(a1, x, acc[2 * q]);
+                            acc[2 * q + 1] = bpf_fma(a1, y, acc[2 * q + 1]);
+                            bpf_lds4<16 * q>(w0, x, y);
+                            acc[2 * q] = bpf_fma(a0, x, acc[2 * q]);
+                            acc[2 * q + 1] = bpf_fma(a0, y, acc[2 * q + 1]);
+                        }
+                    });
+                }
+                __syncwarp();  // this buffer takes the window after the next
             }
+            if (!more) break;
+            cur = nxt;
+            have = true;
+            b ^= 1;
         }
     } else {
-        for (int vb = v_begin; vb < v_end; vb += vc) {
-            const int nv = min(vc, v_end - vb);
-            __syncthreads();
-            fill_views(vb, nv);
-            __syncthreads();
-            for (int f = tid; f < chunk; f += BPF_THREADS) {
-                const int t = f >> lg_pcta;
-                if (t < nv) {
-                    float4 fa = make_float4(__int_as_float(-1), 0.f, 0.f, 0.f), fb = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (fvalid && s_voff[t] >= 0)
-                        bpf_footprint<KIND>(g, s_cs[t], s_sn[t], fxt, fyt, coeff_power, fa, fb,
-                                            KIND == MBX_GEOM_TRANSLATION ? s_tz[t] : 0.0f);
-                    s_fa[f] = fa;
-                    if (KIND != MBX_GEOM_PARALLEL) s_fb[f] = fb;
+        for (;;) {
+            if (have) {
+                if (TR && cur.tma)
+                    bpf_pipe_wait(pipe, 0, err);
+                else
+                    bpf_private_wait<TR>();
+                __syncwarp();
+                if (cur.in) {
+                    const bpf2 a0 = bpf_pair(cur.a[0], cur.a[0]), a1 = bpf_pair(cur.a[1], cur.a[1]),
+                               a2 = bpf_pair(cur.a[2], cur.a[2]);
+                    const unsigned w0 = (unsigned)__cvta_generic_to_shared(smw + cur.off);
+                    const unsigned w1 = w0 + 4u * (unsigned)pitch, w2 = w1 + 4u * (unsigned)pitch;
+                    bpf_for<0, BPF_FAN_QUADS>([&](auto i) {
+                        constexpr int q = decltype(i)::value;
+                        if (q < cur.nq) {
+                            bpf2 x0, x1, y0, y1, z0, z1;
+                            bpf_lds4<16 * q>(w0, x0, x1);
+                            bpf_lds4<16 * q>(w1, y0, y1);
+                            bpf_lds4<16 * q>(w2, z0, z1);
+                            float r[4];
+                            bpf_unpair(bpf_fma(a0, x0, bpf_fma(a1, y0, bpf_mul(a2, z0))), r[0], r[1]);
+                            bpf_unpair(bpf_fma(a0, x1, bpf_fma(a1, y1, bpf_mul(a2, z1))), r[2], r[3]);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) cache[(4 * q + j) * 32] = r[j];
+                        }
+                    });
                 }
+                __syncwarp();  // the window may be overwritten
             }
-            __syncthreads();
-            if (!active) continue;
-            for (int t = 0; t < nv; ++t) {
-                const int f = (t << lg_pcta) + pl;
-                if (MBX_BPF_PREFETCH > 0 && KIND == MBX_GEOM_PARALLEL && sino && t + MBX_BPF_PREFETCH < nv) {
-                    // the rows of a later view of the chunk: start their L2 -> L1 fills now, so that its gathers
-                    // hit L1 (a prefetch writes no register and faults on no address; the view and channel are
-                    // checked as for the gather).  (One prefetch per lane and view, of the warp's lowest and
-                    // highest tap line per row, was 7% slower on the batched stage than this one per slice.)
-                    const int tn = t + MBX_BPF_PREFETCH;
-                    const int first_n = __float_as_int(s_fa[(tn << lg_pcta) + pl].x);
-                    const int voff_n = s_voff[tn];
-                    if (first_n >= 0 && voff_n >= 0) {
-                        const float *q = sino + (voff_n + s0c + first_n);
-                        for (int s = 0; s < ns; ++s, q += num_channels)
-                            asm volatile("prefetch.global.L1 [%0];" ::"l"(q));
-                    }
-                }
-                const float4 fa = s_fa[f];
-                if (__float_as_int(fa.x) < 0) continue;
-                gather(fa, KIND != MBX_GEOM_PARALLEL ? s_fb[f] : make_float4(0.f, 0.f, 0.f, 0.f), s_voff[t]);
+            const bool more = next(nxt, smw, 0);
+            if (have && cur.in) {
+                if (cur.A1 > 2.0f)
+                    bpf_vertical<true, true>(acc, cur, cache, k_first, nsq, g.delta_voxel, coeff_power);
+                else if (coeff_power == 2)
+                    bpf_vertical<true, false>(acc, cur, cache, k_first, nsq, g.delta_voxel, 2);
+                else
+                    bpf_vertical<false, false>(acc, cur, cache, k_first, nsq, g.delta_voxel, 1);
             }
+            if (!more) break;
+            cur = nxt;
+            have = true;
         }
     }
-    if (p >= num_pixels || ns <= 0) return;
+    __syncwarp();  // the warp's next unit may use the shared memory
+    if (p >= num_pixels) return;
     long long row_of_out = p;
     if (A.out_by_index) {  // write into a flat recon at the pixel's index (skipped for invalid indices)
         if (!active) return;
@@ -453,85 +770,186 @@ __device__ void bp_fast_tile(const BpArgs &A, int bx, int by, int bz, float *smf
     const float sc = (A.split_stride == 0) ? A.scale : 1.0f;
     if (A.out_slices > 0) {  // the one slice's value in every slice of the cylinder
         float *out = A.out + row_of_out * (long long)A.out_slices;
-        const float v = active ? sc * acc[0] : 0.0f;
+        float v, unused;
+        bpf_unpair(acc[0], v, unused);
+        v = active ? sc * v : 0.0f;
         for (int s = 0; s < A.out_slices; ++s) out[s] = v;
         return;
     }
     float *out = A.out + (long long)split * A.split_stride + row_of_out * (long long)num_slices + s0;
 #pragma unroll
-    for (int s = 0; s < BPF_ST; ++s)
-        if (s < ns) out[s] = active ? sc * acc[s] : 0.0f;
+    for (int s = 0; s < BPF_ST / 2; ++s) {
+        float x, y;
+        bpf_unpair(acc[s], x, y);
+        if (2 * s < ns) out[2 * s] = active ? sc * x : 0.0f;
+        if (2 * s + 1 < ns) out[2 * s + 1] = active ? sc * y : 0.0f;
+    }
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(BPF_THREADS, 3) bp_fast_kernel(const BpArgs A, int *err) {
-    extern __shared__ __align__(16) float smf[];
-    bp_fast_tile<KIND>(A, blockIdx.x, blockIdx.y, blockIdx.z, smf, err);
+// Shared memory of one warp, in floats: window(s), row buffer, barriers; a multiple of the 128 bytes a TMA destination
+// is aligned to.
+__host__ __device__ constexpr int bpf_warp_floats(int kind) {
+    return (kind == MBX_GEOM_PARALLEL ? 2 * BPF_WIN_PARALLEL : BPF_WIN_FAN + 4 * BPF_FAN_QUADS * 32) + 32;
 }
 
-// inline_fp: 1 for the variant that computes footprints per thread in registers (see BpfPlan::inline_fp).
-inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_views_sel, int inline_fp = 0) {
+// CTAs of two warps: a warp whose pixels span a wide window takes longer, and holds back only one other.  Resident
+// CTAs per SM the kernels are compiled for (112 and 128 registers).
+constexpr int BPF_LAUNCH_WARPS = 2;
+__host__ __device__ constexpr int bpf_min_blocks(int kind) { return kind == MBX_GEOM_PARALLEL ? 9 : 8; }
+
+// Unit u of a call: the 8 units of plan tile (bx, by) are its npg pixel groups x nsl slice tiles.
+template <int KIND, bool TR>
+__device__ __forceinline__ void bp_fast_run(const BpArgs &A, const CUtensorMap *tmap, int tile, int w, int split, float *smw, BpfPipe &pipe,
+                                            int *err) {
+    const BpfPlan &P = A.plan;
+    const int by = tile / P.gx, bx = tile - by * P.gx;
+    const int pg = w / P.nsl;
+    const int group = bx * P.npg + pg, st = by * P.nsl + (w - pg * P.nsl);
+    if constexpr (KIND == MBX_GEOM_PARALLEL) {
+        // voxels no wider than a channel: two taps per footprint
+        if (A.g.delta_voxel * (1.0f / A.g.delta_det_channel) <= 1.0f) {
+            bp_fast_unit<KIND, TR, true>(A, tmap, group, st, split, smw, pipe, err);
+            return;
+        }
+    }
+    bp_fast_unit<KIND, TR, false>(A, tmap, group, st, split, smw, pipe, err);
+}
+
+template <int KIND, bool TR>
+__global__ void __launch_bounds__(32 * BPF_LAUNCH_WARPS, bpf_min_blocks(KIND))
+bp_fast_kernel(const BpArgs args, const __grid_constant__ CUtensorMap map, int *err) {
+    extern __shared__ __align__(128) float smf[];
+    const int warp = threadIdx.x >> 5;
+    const int unit = blockIdx.x * BPF_LAUNCH_WARPS + warp;
+    float *smw = smf + warp * bpf_warp_floats(KIND);
+    BpfPipe pipe = {0, 0};
+    if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND) - 32);
+    bp_fast_run<KIND, TR>(args, TR ? &map : nullptr, unit >> 3, unit & 7, blockIdx.y, smw, pipe, err);
+}
+
+inline size_t bpf_smem_bytes(int kind, int warps) { return 4 * (size_t)warps * bpf_warp_floats(kind); }
+
+// Transposed copy of a call's views (of every view of the geometry when the call selects more, that is repeats
+// some): per view, channel outermost with BPF_EDGE channels of zeros on either side, rows padded to a multiple of 4
+// with zeros.
+inline int bpf_padded_rows(const mbx_geom &g) { return (g.num_det_rows + 3) & ~3; }
+inline int bpf_transposed_views(const mbx_geom &g, int num_views_sel) {
+    return num_views_sel < g.num_views ? num_views_sel : g.num_views;
+}
+inline size_t bpf_transposed_bytes(const mbx_geom &g, int num_views_sel) {
+    return align256((size_t)bpf_transposed_views(g, num_views_sel) * (g.num_det_channels + 2 * BPF_EDGE) *
+                    bpf_padded_rows(g) * 4);
+}
+
+// The tensor map of a transposed copy at `copy`: boxes of BPF_BOX channels x 4 boxq rows.  False when it cannot be
+// made (a copy that is not 16-byte aligned; defined in back_project.cu).
+bool bpf_window_map(CUtensorMap &map, const float *copy, const mbx_geom &g, int num_views_sel, int boxq);
+
+// Channels c0 .. c0 + 31 (counted with the edge channels) of one view of the transposed copy, by a block of 256 threads:
+// weights x values of src (view offset soff, num_rows x num_channels) to dst (view offset doff).
+__device__ __forceinline__ void bpf_transpose_block(const float *__restrict__ src, const float *__restrict__ wts,
+                                                    float *__restrict__ dst, long long soff, long long doff, int c0,
+                                                    int num_rows, int num_channels, int rp) {
+    __shared__ float tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    for (int r0 = 0; r0 < rp; r0 += 32) {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+            const int r = r0 + ty + j, n = c0 + tx - BPF_EDGE;
+            float v = 0.0f;
+            if (r < num_rows && n >= 0 && n < num_channels) {
+                const long long o = soff + (long long)r * num_channels + n;
+                v = __ldg(src + o);
+                if (wts) v *= __ldg(wts + o);
+            }
+            tile[ty + j][tx] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+            const int c = c0 + ty + j, r = r0 + tx;
+            if (c < num_channels + 2 * BPF_EDGE && r < rp) dst[doff + (long long)c * rp + r] = tile[tx][ty + j];
+        }
+    }
+}
+
+// Slices per tile: the fewest tiles of <= most slices, the slices spread evenly over them, in fours.
+inline int bpf_tile_height(int S, int most) {
+    const int tiles = ceil_div(S, most);
+    const int ts = ((ceil_div(S, tiles) + 3) / 4) * 4;
+    return ts < most ? ts : most;
+}
+
+// The partial sums of the splits take at most BPF_PARTIAL_BYTES (which fits the scratch of the entry point that
+// allocates nothing), or twice the sinogram unless `small`.
+constexpr size_t BPF_PARTIAL_BYTES = MBX_NOALLOC_SCRATCH_BYTES / 4 * 3;
+
+inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_views_sel, int small = 0) {
     BpfPlan pl;
-    pl.inline_fp = inline_fp;
+    pl.inline_fp = 1;
+    pl.chunk = 0;
+    pl.vc = 32;
     // 32-bit element offsets address the sinogram
     pl.ok = (g.kind == MBX_GEOM_PARALLEL || g.kind == MBX_GEOM_CONE ||
              (g.kind == MBX_GEOM_TRANSLATION && g.max_magnification > 0.0f)) &&
             (g.psf_radius == 1) && g.num_det_channels >= 3 &&
             (long long)g.num_views * g.num_det_rows * g.num_det_channels < (1LL << 31);
     const int S = g.num_recon_slices;
-    // tile height: the fewest tiles of <= BPF_ST slices, rounded up to a power of two (<= 8) or a multiple of 8,
-    // then the slices spread evenly over them
-    const int t0 = ceil_div(S, BPF_ST);
-    int T = 1;
-    if (t0 <= 8) {
-        while (T < t0) T <<= 1;
-    } else {
-        T = ceil_div(t0, 8) * 8;
+    int most = BPF_ST;
+    double slope = 1.0;
+    if (g.kind != MBX_GEOM_PARALLEL) {
+        // the row buffer must hold the rows of a slice tile: ts * max |dm/dk| + 4
+        double max_mag = g.max_magnification;  // translation: the host's bound
+        if (g.kind == MBX_GEOM_CONE) {
+            const double half_r = 0.5 * (g.num_recon_rows - 1), half_c = 0.5 * (g.num_recon_cols - 1);
+            const double rho = g.delta_voxel * std::sqrt(half_r * half_r + half_c * half_c);
+            const double inv = 1.0 / g.magnification - (std::isinf(g.source_detector_dist) ? 0.0 : rho / g.source_detector_dist);
+            max_mag = inv > 1e-6 ? 1.0 / inv : 1e6;
+        }
+        slope = max_mag * g.delta_voxel / g.delta_det_row;
+        while (most > 4 && most * slope + 4 > BPF_CACHE_ROWS) most -= 4;
+        if (bpf_tile_height(S, most) * slope + 4 > BPF_CACHE_ROWS) pl.ok = false;
     }
-    pl.ts = ceil_div(S, T);
+    pl.ts = bpf_tile_height(S, most);
     pl.tiles = ceil_div(S, pl.ts);
+    // rows of a window: the tile's (parallel); its rows at the steepest slope, their rounding and some spread (fan)
+    pl.boxq = g.kind == MBX_GEOM_PARALLEL ? ((pl.ts + 3) / 4) | 1
+                                          : std::min(BPF_FAN_QUADS, (int)std::ceil((pl.ts * slope + 12) / 4) | 1);
+    // a CTA's warps on neighbouring pixels of one slice tile (their windows overlap in L1), on several tiles only when
+    // the list is shorter than a CTA
     pl.nsl = 1;
-    while (pl.nsl < pl.tiles && pl.nsl < 8) pl.nsl <<= 1;
+    while (pl.nsl < 8 && pl.tiles % (2 * pl.nsl) == 0 && num_pixels <= 32 * (8 / (2 * pl.nsl))) pl.nsl *= 2;
     pl.npg = 8 / pl.nsl;
     pl.lg_pcta = 5;
     while ((1 << pl.lg_pcta) < 32 * pl.npg) ++pl.lg_pcta;
     const int pcta = 32 * pl.npg;
-    pl.chunk = (g.kind != MBX_GEOM_PARALLEL) ? MBX_BPF_CHUNK_CONE : MBX_BPF_CHUNK_PARALLEL;
-    if (pl.chunk < pcta) pl.chunk = pcta;
-    pl.vc = pl.chunk / pcta;
-    if (inline_fp) {  // no staged footprints; a view table of up to 1024 views per refill
-        pl.chunk = 0;
-        pl.vc = 1024;
-    }
     pl.gx = ceil_div(num_pixels > 0 ? num_pixels : 1, pcta);
     pl.gy = ceil_div(pl.tiles, pl.nsl);
-    if (g.kind == MBX_GEOM_CONE) {
-        // the row cache must hold the rows of a slice tile: ts * max |dm/dk| + 4
-        const double half_r = 0.5 * (g.num_recon_rows - 1), half_c = 0.5 * (g.num_recon_cols - 1);
-        const double rho = g.delta_voxel * std::sqrt(half_r * half_r + half_c * half_c);
-        const double inv = 1.0 / g.magnification - (std::isinf(g.source_detector_dist) ? 0.0 : rho / g.source_detector_dist);
-        const double max_mag = inv > 1e-6 ? 1.0 / inv : 1e6;
-        const double slope = max_mag * g.delta_voxel / g.delta_det_row;
-        if (pl.ts * slope + 4 > BPF_CACHE_ROWS) pl.ok = false;
-    } else if (g.kind == MBX_GEOM_TRANSLATION) {  // same bound from the host's magnification bound
-        const double slope = (double)g.max_magnification * g.delta_voxel / g.delta_det_row;
-        if (pl.ts * slope + 4 > BPF_CACHE_ROWS) pl.ok = false;
-    }
+    // views split over CTAs when there are few: the fewest splits (partial sums cost memory traffic) whose last wave
+    // is full enough, as the time of a call is about waves / splits
     const long long base = (long long)pl.gx * pl.gy;
-    const int sms = num_sms();
+    const long long slots = (long long)bpf_min_blocks(g.kind) * BPF_LAUNCH_WARPS * num_sms() / BPF_WARPS;
     long long splits = 1;
-    if (base < 2LL * sms && num_views_sel >= 16) {
-        splits = (2LL * sms + base - 1) / base;
+    if (base < 2 * slots && num_views_sel >= 16) {
         long long maxs = num_views_sel / 8;
-        if (splits > maxs) splits = maxs;
-        if (splits > 64) splits = 64;
-        if (splits < 1) splits = 1;
+        if (maxs > 64) maxs = 64;
+        size_t most_bytes = BPF_PARTIAL_BYTES;
+        if (!small) most_bytes = std::max(most_bytes, (size_t)g.num_views * g.num_det_rows * g.num_det_channels * 8);
+        const long long fit = (long long)most_bytes / (4 * (num_pixels > 0 ? num_pixels : 1) * S);
+        if (maxs > fit) maxs = fit;
+        double best = 1e300;
+        for (long long s = 1; s <= maxs; ++s) {
+            const double cost = (double)((base * s + slots - 1) / slots) / s * (1.0 + 0.01 * s);
+            if (cost < best * 0.98) {
+                best = cost;
+                splits = s;
+            }
+        }
     }
     pl.views_per_split = ceil_div(num_views_sel, splits);
     pl.splits = ceil_div(num_views_sel, pl.views_per_split);
-    pl.smem = (size_t)pl.chunk * 16 * (g.kind != MBX_GEOM_PARALLEL ? 2 : 1) +
-              (size_t)pl.vc * (g.kind == MBX_GEOM_TRANSLATION ? 16 : 12) +
-              (g.kind != MBX_GEOM_PARALLEL ? (size_t)BPF_CACHE_ROWS * BPF_THREADS * 4 : 0);
+    pl.smem = bpf_smem_bytes(g.kind, BPF_LAUNCH_WARPS);
     pl.workspace = pl.splits > 1 ? align256((size_t)pl.splits * num_pixels * S * 4) : 0;
     return pl;
 }

@@ -60,7 +60,7 @@ extern "C" int mbx_sparse_back_project_noalloc(const mbx_geom *g, const float *s
         sinogram = weights;
         weights = nullptr;
     }
-    const size_t need = mbx::bp_workspace_bytes(*g, num_pixels, num_views_sel);
+    const size_t need = mbx::bp_noalloc_bytes(*g, num_pixels, num_views_sel);
     if (need > MBX_NOALLOC_SCRATCH_BYTES) return MBX_ERR_WORKSPACE;  // more scratch than the static array holds
     void *scratch = nullptr;
     if (need > 0) {
@@ -68,5 +68,5 @@ extern "C" int mbx_sparse_back_project_noalloc(const mbx_geom *g, const float *s
         if (rc != MBX_OK) return rc;
     }
     return mbx::back_project(*g, sinogram, weights, pixel_indices, num_pixels, view_indices, num_views_sel,
-                             coeff_power, scale, out, scratch, need, static_cast<cudaStream_t>(stream));
+                             coeff_power, scale, out, scratch, need, static_cast<cudaStream_t>(stream), true);
 }

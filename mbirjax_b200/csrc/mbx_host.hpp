@@ -33,6 +33,9 @@ cudaError_t set_max_dynamic_smem(const void *func, int bytes);
 
 size_t fp_workspace_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel);
 size_t bp_workspace_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel);
+// What back_project needs with noalloc: no transposed copy of the sinogram, and at most BPF_PARTIAL_BYTES of partial
+// sums where the fast kernel runs.
+size_t bp_noalloc_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel);
 
 int forward_project(const mbx_geom &g, const float *vox, const int32_t *pix, long long num_pixels,
                     const int32_t *views, int num_views_sel, float *out, void *ws, size_t ws_bytes,
@@ -40,7 +43,7 @@ int forward_project(const mbx_geom &g, const float *vox, const int32_t *pix, lon
 
 int back_project(const mbx_geom &g, const float *sino, const float *w, const int32_t *pix, long long num_pixels,
                  const int32_t *views, int num_views_sel, int coeff_power, float scale, float *out, void *ws,
-                 size_t ws_bytes, cudaStream_t st);
+                 size_t ws_bytes, cudaStream_t st, bool noalloc = false);
 
 // Autotuning.  The first call of a projector for a given call shape (geometry sizes, views, pixel count rounded
 // up to a power of two) times its candidate plans on the caller's stream and remembers the fastest; later calls

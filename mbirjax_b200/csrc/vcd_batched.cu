@@ -33,15 +33,38 @@
 
 namespace mbx {
 
-template <int KIND>
-__global__ void __launch_bounds__(BPF_THREADS, MBX_BBP_MIN_BLOCKS) b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
-    extern __shared__ __align__(16) float smb[];
-    for (int t = first + fetch_tile(L.counter); t < total; t = first + fetch_tile(L.counter)) {
+// Each warp takes units (an eighth of a list tile) of its own: warps share nothing but the counter.
+template <int KIND, bool TR>
+__global__ void __launch_bounds__(32 * BPF_LAUNCH_WARPS, bpf_min_blocks(KIND))
+b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
+    extern __shared__ __align__(128) float smb[];
+    float *smw = smb + (threadIdx.x >> 5) * bpf_warp_floats(KIND);
+    BpfPipe pipe = {0, 0};
+    if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND) - 32);
+    for (;;) {
+        int u = 0;
+        if ((threadIdx.x & 31) == 0) u = atomicAdd(L.counter, 1);
+        u = __shfl_sync(0xffffffffu, u, 0);
+        const int t = first + (u >> 3);
+        if (t >= total) break;
         const int k = find_scan(L.off, num_scans, t);
         const int s = __ldg(L.order + k);
-        const int local = t - __ldg(L.off + k);
-        const int gx = __ldg(L.dim + s);
-        bp_fast_tile<KIND>(list_record(L.bp, L, num_scans, step, s), local % gx, local / gx, 0, smb, err);
+        const BpArgs &A = list_record(L.bp, L, num_scans, step, s);
+        bp_fast_run<KIND, TR>(A, A.tmap, t - __ldg(L.off + k), u & 7, 0, smw, pipe, err);
+    }
+}
+
+// Transposed copies for a back-projection stage: of W x error sinogram (mode 0), the error sinogram (1) or W (2).
+__global__ void __launch_bounds__(256) b_transpose(BatchedTables T, int num_scans, int total, int mode) {
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        const int s = find_scan(T.tr_off, num_scans, t);
+        const VcdScan &sc = T.scans[s];
+        const int blocks = ceil_div(sc.C + 2 * BPF_EDGE, 32);
+        const int local = t - __ldg(T.tr_off + s);
+        const int v = local / blocks;
+        bpf_transpose_block(mode == 2 ? sc.wts : sc.err, mode == 0 ? sc.wts : nullptr, sc.tsino,
+                            (long long)v * sc.R * sc.C, (long long)v * (sc.C + 2 * BPF_EDGE) * sc.rp,
+                            (local - v * blocks) * 32, sc.R, sc.C, sc.rp);
     }
 }
 
@@ -364,6 +387,7 @@ struct ScanSizes {
     BpfPlan hbp;  // Hessian back projection over every pixel
     int hbp_slices;  // > 0: hbp is planned on one slice and broadcast to this many (unit-weight parallel beam)
     bool setup;   // the scan carries the set-up inputs
+    int tr_tiles; // 32-channel blocks of the transposed copy over all views
 };
 
 static int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
@@ -385,6 +409,7 @@ static int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
     z.el_tiles = (int)((z.ncyl + BT_ELEM_TILE - 1) / BT_ELEM_TILE);
     z.sn_tiles = (int)((z.nsino + BT_SINO_TILE - 1) / BT_SINO_TILE);
     z.rc_tiles = (int)((z.nrecon + BT_SINO_TILE - 1) / BT_SINO_TILE);
+    z.tr_tiles = g.num_views * ceil_div(g.num_det_channels + 2 * BPF_EDGE, 32);
     z.setup = sc.sinogram != nullptr || sc.full_indices != nullptr || sc.num_full_indices != 0;
     z.flt_tiles = 0;
     if (z.setup) {
@@ -478,13 +503,13 @@ static PlannedSizes planned_sizes(const mbx_scan &sc, const ScanSizes &z) {
 
 struct Layout {
     size_t scans, fm, qp, bpargs, fpargs, ibp, ifp, hbp, filt, planned, pl_off, pl_dim, pl_order, offs, box_first,
-        counters, sched, p_prior, p_fwd, p_l1, p_iter, p_init, alpha, alpha_init, arange, cursors, total;
+        counters, sched, maps, p_prior, p_fwd, p_l1, p_iter, p_init, alpha, alpha_init, arange, cursors, total;
     bool plan_fp;
     std::vector<size_t> plan_off;  // per scan: its subsets' planned storage, [K][PlannedSizes::total]
     int pl_total[PL_COUNT];
-    int el_total, sn_total, rc_total, flt_total, box_total, ksum, max_npix;
-    bool setup;
-    std::vector<size_t> buf_off;   // per scan: bp, delta, dsino
+    int el_total, sn_total, rc_total, flt_total, box_total, tr_total, ksum, max_npix;
+    bool setup, transposed, hess_transposed;
+    std::vector<size_t> buf_off;   // per scan: bp, delta, dsino, transposed copy
     std::vector<size_t> box_off;   // per scan: chunk boxes of its subsets, [K][chunks]
     std::vector<size_t> fbox_off;  // per scan: chunk boxes of its region-of-reconstruction list
 };
@@ -494,7 +519,8 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
     L.plan_fp = (flags & MBX_BATCHED_PLAN_FORWARD) != 0;
     zs.resize(n);
     for (int w = 0; w < PL_COUNT; ++w) L.pl_total[w] = 0;
-    L.el_total = L.sn_total = L.rc_total = L.flt_total = L.box_total = L.ksum = L.max_npix = 0;
+    L.el_total = L.sn_total = L.rc_total = L.flt_total = L.box_total = L.tr_total = L.ksum = L.max_npix = 0;
+    L.transposed = L.hess_transposed = true;
     int kind = -1, nsetup = 0;
     for (int s = 0; s < n; ++s) {
         int rc = scan_sizes(scans[s], zs[s]);
@@ -512,6 +538,12 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
         L.sn_total += zs[s].sn_tiles;
         L.rc_total += zs[s].rc_tiles;
         L.flt_total += zs[s].flt_tiles;
+        L.tr_total += zs[s].tr_tiles;
+        // every scan's copy has to be addressable (32-bit offsets); the Hessian's needs weights to copy
+        const mbx_geom &g = scans[s].geom;
+        if ((long long)g.num_views * (g.num_det_channels + 2 * BPF_EDGE) * bpf_padded_rows(g) >= (1LL << 31))
+            L.transposed = false;
+        if (!scans[s].weights) L.hess_transposed = false;
         L.ksum += scans[s].num_subsets;
         L.box_total += scans[s].num_subsets * (int)((scans[s].subset_size + CB_CHUNK - 1) / CB_CHUNK);
         L.max_npix = std::max<int>(L.max_npix, (int)zs[s].npix);
@@ -519,6 +551,7 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
     }
     if (nsetup != 0 && nsetup != n) return MBX_ERR_INVALID_ARG;  // set-up inputs for every scan or for none
     L.setup = nsetup == n;
+    L.hess_transposed = L.hess_transposed && L.transposed;
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += align256(bytes); return o; };
     L.scans = take(sizeof(VcdScan) * n);
@@ -534,7 +567,8 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
     L.pl_off = take(sizeof(int) * PL_COUNT * (n + 1));
     L.pl_dim = take(sizeof(int) * PL_COUNT * n);
     L.pl_order = take(sizeof(int) * PL_COUNT * n);
-    L.offs = take(sizeof(int) * 4 * (n + 1));
+    L.offs = take(sizeof(int) * 5 * (n + 1));
+    L.maps = take(sizeof(CUtensorMap) * n);
     L.box_first = take(sizeof(int) * (L.ksum + 1));
     L.counters = take(sizeof(int) * PL_COUNT);
     L.sched = take(sizeof(int) * (size_t)num_steps * n);  // the host-built tables end here
@@ -547,11 +581,12 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
     L.alpha_init = take(sizeof(float) * n);
     L.arange = take(L.setup ? sizeof(int32_t) * (size_t)L.max_npix : 0);
     L.cursors = take(L.plan_fp ? 16 * (size_t)L.ksum : 0);  // {unsigned long long records, int passes, pad}
-    L.buf_off.resize(3 * (size_t)n);
+    L.buf_off.resize(4 * (size_t)n);
     for (int s = 0; s < n; ++s) {
-        L.buf_off[3 * s] = take(4 * (size_t)zs[s].ncyl);
-        L.buf_off[3 * s + 1] = take(4 * (size_t)zs[s].ncyl);
-        L.buf_off[3 * s + 2] = take(4 * (size_t)zs[s].nsino);
+        L.buf_off[4 * s] = take(4 * (size_t)zs[s].ncyl);
+        L.buf_off[4 * s + 1] = take(4 * (size_t)zs[s].ncyl);
+        L.buf_off[4 * s + 2] = take(4 * (size_t)zs[s].nsino);
+        L.buf_off[4 * s + 3] = take(L.transposed ? bpf_transposed_bytes(scans[s].geom, scans[s].geom.num_views) : 0);
     }
     L.box_off.resize(n);
     L.fbox_off.assign(n, 0);
@@ -578,11 +613,13 @@ static int occupancy_grid(K kern, int threads, size_t smem, int total) {
 }
 
 // The projection stage kernels of a geometry kind.
+template <bool TR>
 static const void *bp_kernel_of(int kind) {
-    return kind == MBX_GEOM_PARALLEL ? reinterpret_cast<const void *>(b_bp<MBX_GEOM_PARALLEL>)
-           : kind == MBX_GEOM_CONE   ? reinterpret_cast<const void *>(b_bp<MBX_GEOM_CONE>)
-                                     : reinterpret_cast<const void *>(b_bp<MBX_GEOM_TRANSLATION>);
+    return kind == MBX_GEOM_PARALLEL ? reinterpret_cast<const void *>(b_bp<MBX_GEOM_PARALLEL, TR>)
+           : kind == MBX_GEOM_CONE   ? reinterpret_cast<const void *>(b_bp<MBX_GEOM_CONE, TR>)
+                                     : reinterpret_cast<const void *>(b_bp<MBX_GEOM_TRANSLATION, TR>);
 }
+static const void *bp_kernel_of(int kind, bool tr) { return tr ? bp_kernel_of<true>(kind) : bp_kernel_of<false>(kind); }
 
 // The forward stage kernels of each geometry kind (compiled in b_fp_parallel.cu, b_fp_cone.cu, b_fp_translation.cu).
 const void *fp_stage_kernel_parallel(int minb, int mode);
@@ -628,28 +665,44 @@ static cudaError_t set_smem_carveout(const void *kern, int threads, size_t smem)
     return cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 
-static int bp_grid(int kind, size_t smem, int total) {
-    return occupancy_grid(bp_kernel_of(kind), BPF_THREADS, smem, total);
+static int bp_grid(int kind, bool tr, size_t smem, int total) {
+    return occupancy_grid(bp_kernel_of(kind, tr), 32 * BPF_LAUNCH_WARPS, smem, total * (BPF_WARPS / BPF_LAUNCH_WARPS));
 }
 
 static int fp_grid(int kind, int minb, size_t smem, int total, int mode = CB_WALK) {
     return occupancy_grid(fp_kernel_of(kind, minb, mode), CB_THREADS, smem, total);
 }
 
-// One launch of a back-projection work list over tiles [first, total) (resets the list's counter first).
-static cudaError_t launch_bp_list(const BatchedPlanHost &P, int which, int step, int first, int total, int grid,
-                                  size_t smem, cudaStream_t st) {
+template <bool TR>
+static void launch_bp_kernel(int kind, int grid, size_t smem, cudaStream_t st, const ProjList &L, int n, int step,
+                             int total) {
+    constexpr int T = 32 * BPF_LAUNCH_WARPS;
+    int *err = device_error_ptr();
+    if (kind == MBX_GEOM_PARALLEL)
+        b_bp<MBX_GEOM_PARALLEL, TR><<<grid, T, smem, st>>>(L, n, step, 0, total, err);
+    else if (kind == MBX_GEOM_CONE)
+        b_bp<MBX_GEOM_CONE, TR><<<grid, T, smem, st>>>(L, n, step, 0, total, err);
+    else
+        b_bp<MBX_GEOM_TRANSLATION, TR><<<grid, T, smem, st>>>(L, n, step, 0, total, err);
+}
+
+// One launch of a back-projection work list (resets the list's counter first), after the transposed copies of what it
+// projects.
+static cudaError_t launch_bp_list(const BatchedPlanHost &P, int which, int step, cudaStream_t st) {
     ProjList L = proj_list(P.t, which, P.num_scans);
     L.stride = which == PL_BP ? P.ksum / P.num_scans : 1;
     cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    int *err = device_error_ptr();
-    if (P.kind == MBX_GEOM_PARALLEL)
-        b_bp<MBX_GEOM_PARALLEL><<<grid, BPF_THREADS, smem, st>>>(L, P.num_scans, step, first, total, err);
-    else if (P.kind == MBX_GEOM_CONE)
-        b_bp<MBX_GEOM_CONE><<<grid, BPF_THREADS, smem, st>>>(L, P.num_scans, step, first, total, err);
-    else
-        b_bp<MBX_GEOM_TRANSLATION><<<grid, BPF_THREADS, smem, st>>>(L, P.num_scans, step, first, total, err);
+    const bool tr = which == PL_HESS ? P.hess_transposed : P.transposed;
+    if (tr) {
+        b_transpose<<<P.tr_grid, 256, 0, st>>>(P.t, P.num_scans, P.tr_total,
+                                               which == PL_BP ? 0 : which == PL_INIT_BP ? 1 : 2);
+        note_launch();
+        launch_bp_kernel<true>(P.kind, P.pl_grid[which], P.pl_smem[which], st, L, P.num_scans, step, P.pl_total[which]);
+    } else {
+        launch_bp_kernel<false>(P.kind, P.pl_grid[which], P.pl_smem[which], st, L, P.num_scans, step,
+                                P.pl_total[which]);
+    }
     note_launch();
     return cudaGetLastError();
 }
@@ -724,7 +777,7 @@ static int tune_batched_fp(BatchedPlanHost &P, const Layout &L, const std::vecto
     if (stream_is_capturing(st)) return MBX_OK;
     cudaError_t e = cudaSuccess;
     for (int s = 0; s < num_scans && e == cudaSuccess; ++s)
-        e = cudaMemsetAsync(base + L.buf_off[3 * s + 1], 0, 4 * (size_t)zs[s].ncyl, st);
+        e = cudaMemsetAsync(base + L.buf_off[4 * s + 1], 0, 4 * (size_t)zs[s].ncyl, st);
     if (e != cudaSuccess) return set_cuda_error(e);
     auto run = [&]() {
         return launch_fp_list(P, PL_FP, P.fp_minb, 0, 0, P.pl_total[PL_FP], P.pl_grid[PL_FP], P.pl_smem[PL_FP], st);
@@ -838,89 +891,6 @@ static int tune_batched_fp_layouts(BatchedPlanHost &P, const Layout &L, const mb
     return MBX_OK;
 }
 
-// Autotuning of the back-projection stage, per scan: staged (shared-memory) footprints, the tables as built,
-// against per-thread footprints computed in registers (same tiles).  Each scan is timed alone on step 0 (the
-// launch walks only that scan's tiles; the stage only writes the scans' back-projection scratch), so that every
-// scan keeps the plan that suits its shape, as the plain path's per-call tuner would choose.  The choices are
-// cached per batch shape.
-static int tune_batched_bp(BatchedPlanHost &P, const Layout &L, const mbx_scan *scans, const BpArgs *hb1,
-                           const int *o_bp, const int *order_bp, cudaStream_t st) {
-    const int num_scans = P.num_scans;
-    const int K = scans[0].num_subsets;  // every scan of a batch has the same number of subsets
-    const int ksum = L.ksum;
-    std::vector<BpArgs> cur(hb1, hb1 + ksum), alt(hb1, hb1 + ksum);
-    std::vector<char> can(num_scans, 1);
-    size_t smem_alt = 0;
-    for (int k = 0; k < ksum; ++k) {
-        const BpfPlan q = plan_bp_fast(alt[k].g, alt[k].num_pixels, alt[k].g.num_views, 1);
-        if (!q.ok || q.gx != alt[k].plan.gx || q.gy != alt[k].plan.gy || q.splits != 1) {
-            can[k / K] = 0;
-            continue;
-        }
-        alt[k].plan = q;
-        smem_alt = std::max(smem_alt, q.smem);
-    }
-    char *base = reinterpret_cast<char *>(P.t.scans) - L.scans;
-    std::vector<long long> key = batch_key(4, P, scans, true);
-    key[3] = -1;
-    auto upload = [&]() -> cudaError_t {
-        cudaError_t e = cudaMemcpyAsync(base + L.bpargs, cur.data(), sizeof(BpArgs) * ksum, cudaMemcpyHostToDevice, st);
-        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-    };
-    auto apply_smem = [&]() {
-        size_t sm = 0;
-        for (int k = 0; k < ksum; ++k) sm = std::max(sm, cur[k].plan.smem);
-        P.pl_smem[PL_BP] = sm;
-        P.pl_grid[PL_BP] = bp_grid(P.kind, sm, P.pl_total[PL_BP]);
-    };
-    auto use = [&](int s, int c) {
-        for (int j = 0; j < K; ++j) cur[s * K + j] = c ? alt[s * K + j] : hb1[s * K + j];
-    };
-    bool all_cached = true;
-    std::vector<int> choice(num_scans, 0);
-    for (int s = 0; s < num_scans; ++s) {
-        if (!can[s]) continue;
-        if (autotune_forced() >= 0) {
-            choice[s] = autotune_forced() >= 1 ? 1 : 0;
-        } else {
-            key[4] = s;
-            const int c = autotune_lookup(key.data(), (int)key.size());
-            if (c < 0) all_cached = false;
-            choice[s] = c == 1 ? 1 : 0;
-        }
-    }
-    if (all_cached || autotune_forced() >= 0 || stream_is_capturing(st)) {
-        for (int s = 0; s < num_scans; ++s) use(s, can[s] ? choice[s] : 0);
-        cudaError_t e = upload();
-        if (e != cudaSuccess) return set_cuda_error(e);
-        apply_smem();
-        return MBX_OK;
-    }
-    P.pl_smem[PL_BP] = std::max(P.pl_smem[PL_BP], smem_alt);  // tuning launches fit either plan
-    for (int k = 0; k < num_scans; ++k) {
-        const int s = order_bp[k];
-        if (!can[s]) continue;
-        const int first = o_bp[k], last = o_bp[k + 1];
-        const int grid = std::min(P.pl_grid[PL_BP], last - first);
-        auto run = [&]() { return launch_bp_list(P, PL_BP, 0, first, last, grid, P.pl_smem[PL_BP], st); };
-        float t[2] = {0.0f, 0.0f};
-        for (int c = 0; c < 2; ++c) {
-            use(s, c);
-            cudaError_t e = upload();
-            if (e == cudaSuccess) e = time_on_stream(run, st, t[c]);
-            if (e != cudaSuccess) return set_cuda_error(e);
-        }
-        choice[s] = t[1] < t[0] ? 1 : 0;
-        use(s, choice[s]);
-        key[4] = s;
-        autotune_store(key.data(), (int)key.size(), choice[s]);
-    }
-    cudaError_t e = upload();
-    if (e != cudaSuccess) return set_cuda_error(e);
-    apply_smem();
-    return MBX_OK;
-}
-
 // Per-call parameter tables: fm constants and qGGMRF parameters.
 static void fill_params(const mbx_scan *scans, int n, float *fm, QParams *qp) {
     for (int s = 0; s < n; ++s) {
@@ -999,9 +969,18 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     int *hpl_order = reinterpret_cast<int *>(host.data() + L.pl_order);
     int *hoff = reinterpret_cast<int *>(host.data() + L.offs);
     int *hbox_first = reinterpret_cast<int *>(host.data() + L.box_first);
-    int *o_el = hoff, *o_sn = hoff + n1, *o_rc = hoff + 2 * n1, *o_flt = hoff + 3 * n1;
+    int *o_el = hoff, *o_sn = hoff + n1, *o_rc = hoff + 2 * n1, *o_flt = hoff + 3 * n1, *o_tr = hoff + 4 * n1;
+    // one tensor map per scan serves all its back projections: the window's rows depend on the geometry alone
+    bool transposed = L.transposed;
+    for (int s = 0; s < n && transposed; ++s) {
+        CUtensorMap map = {};
+        transposed = bpf_window_map(map, reinterpret_cast<const float *>(base + L.buf_off[4 * s + 3]), scans[s].geom,
+                                    scans[s].geom.num_views, zs[s].bpp.boxq);
+        std::memcpy(host.data() + L.maps + sizeof(map) * s, &map, sizeof(map));
+    }
+    const bool hess_transposed = transposed && L.hess_transposed;
     fill_params(scans, n, reinterpret_cast<float *>(host.data() + L.fm), reinterpret_cast<QParams *>(host.data() + L.qp));
-    o_el[0] = o_sn[0] = o_rc[0] = o_flt[0] = 0;
+    o_el[0] = o_sn[0] = o_rc[0] = o_flt[0] = o_tr[0] = 0;
     hbox_first[0] = 0;
     auto bp_args = [](const mbx_geom &g, const float *sino, const float *wts, const int32_t *pix, long long npix,
                       int cp, float *out, int by_index, const BpfPlan &plan) {
@@ -1035,9 +1014,20 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         v.wts = sc.weights;
         v.hess = const_cast<float *>(sc.fm_hessian);
         v.partition = sc.partition;
-        v.bp = reinterpret_cast<float *>(base + L.buf_off[3 * s]);
-        v.delta = reinterpret_cast<float *>(base + L.buf_off[3 * s + 1]);
-        v.dsino = reinterpret_cast<float *>(base + L.buf_off[3 * s + 2]);
+        v.bp = reinterpret_cast<float *>(base + L.buf_off[4 * s]);
+        v.delta = reinterpret_cast<float *>(base + L.buf_off[4 * s + 1]);
+        v.dsino = reinterpret_cast<float *>(base + L.buf_off[4 * s + 2]);
+        v.tsino = transposed ? reinterpret_cast<float *>(base + L.buf_off[4 * s + 3]) : nullptr;
+        v.V = g.num_views;
+        v.R = g.num_det_rows;
+        v.C = g.num_det_channels;
+        v.rp = bpf_padded_rows(g);
+        auto window_source = [&](BpArgs &a) {  // the scan's transposed copy
+            a.tsino = v.tsino;
+            a.rp = v.rp;
+            a.tsino_all = 1;
+            a.tmap = reinterpret_cast<const CUtensorMap *>(base + L.maps) + s;
+        };
         v.y = sc.sinogram;
         v.nsino = z.nsino;
         v.nrecon = z.nrecon;
@@ -1049,6 +1039,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         for (int k = 0; k < sc.num_subsets; ++k, ++ki) {
             const int32_t *pix = sc.partition + (size_t)k * sc.subset_size;
             hb[ki] = bp_args(g, sc.error_sinogram, sc.weights, pix, sc.subset_size, 1, v.bp, 0, z.bpp);
+            if (transposed) window_source(hb[ki]);
             if (sc.partition_order) hb[ki].order = sc.partition_order + (size_t)k * sc.subset_size;
             FpArgs &f = hf[ki];
             std::memset(&f, 0, sizeof(f));
@@ -1101,6 +1092,8 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
                              reinterpret_cast<const int32_t *>(base + L.arange), z.npix, 2,
                              const_cast<float *>(sc.fm_hessian), 0, z.hbp);
             hhb[s].out_slices = z.hbp_slices;
+            if (transposed) window_source(hib[s]);
+            if (hess_transposed) window_source(hhb[s]);
             FiltScan &fl = hfl[s];
             fl.in = sc.sinogram;
             fl.out = sc.error_sinogram;
@@ -1118,6 +1111,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         o_sn[s + 1] = o_sn[s] + z.sn_tiles;
         o_rc[s + 1] = o_rc[s] + z.rc_tiles;
         o_flt[s + 1] = o_flt[s] + z.flt_tiles;
+        o_tr[s + 1] = o_tr[s] + z.tr_tiles;
     }
     // projection work lists: scans in decreasing order of per-tile cost, so that the dynamically scheduled tail of
     // a launch is made of the cheapest tiles
@@ -1129,8 +1123,8 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
             list_dims(w, scans[s], zs[s], tiles[s], dim[s], cost[s], L.plan_fp);
             ord[s] = s;
             const ScanSizes &z = zs[s];
-            const size_t sm = w == PL_BP ? z.bpp.smem : (w == PL_FP || w == PL_INIT_FP || w == PL_BUILD) ? z.fpp.walk.smem
-                              : w == PL_INIT_BP ? (z.setup ? z.ibp.smem : 0) : (z.setup ? z.hbp.smem : 0);
+            const bool fp = w == PL_FP || w == PL_INIT_FP || w == PL_BUILD;
+            const size_t sm = fp ? z.fpp.walk.smem : bpf_smem_bytes(scans[s].geom.kind, BPF_LAUNCH_WARPS);
             pl_smem[w] = std::max(pl_smem[w], sm);
         }
         std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return cost[a] > cost[b]; });
@@ -1176,6 +1170,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     P.t.sn_off = doff + n1;
     P.t.rc_off = doff + 2 * n1;
     P.t.flt_off = doff + 3 * n1;
+    P.t.tr_off = doff + 4 * n1;
     P.t.box_first = reinterpret_cast<int *>(base + L.box_first);
     P.t.counters = reinterpret_cast<int *>(base + L.counters);
     P.t.schedule = reinterpret_cast<int *>(base + L.sched);
@@ -1205,6 +1200,9 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     P.rc_total = L.rc_total;
     P.flt_total = L.flt_total;
     P.box_total = L.box_total;
+    P.tr_total = L.tr_total;
+    P.transposed = transposed ? 1 : 0;
+    P.hess_transposed = hess_transposed ? 1 : 0;
     P.fp_minb = 2;
     size_t flt_smem = 0;
     for (int s = 0; s < n; ++s)
@@ -1213,8 +1211,9 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
                                                             scans[s].geom.kind != MBX_GEOM_PARALLEL));
     P.flt_smem = flt_smem;
     // kernel attributes and resident-CTA grids
-    const void *kbp = bp_kernel_of(P.kind), *kfp2 = fp_kernel_of(P.kind, 2), *kfp3 = fp_kernel_of(P.kind, 3);
-    e = set_max_dynamic_smem(kbp, 100 * 1024);
+    const void *kfp2 = fp_kernel_of(P.kind, 2), *kfp3 = fp_kernel_of(P.kind, 3);
+    e = set_max_dynamic_smem(bp_kernel_of(P.kind, false), 100 * 1024);
+    if (e == cudaSuccess) e = set_max_dynamic_smem(bp_kernel_of(P.kind, true), 100 * 1024);
     if (e == cudaSuccess) e = set_max_dynamic_smem(kfp2, 200 * 1024);
     if (e == cudaSuccess) e = set_max_dynamic_smem(kfp3, 200 * 1024);
     for (int mb = 2; mb <= 3 && e == cudaSuccess && L.plan_fp; ++mb) {
@@ -1223,11 +1222,11 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     }
     if (e == cudaSuccess) e = set_max_dynamic_smem(reinterpret_cast<const void *>(b_filter), 200 * 1024);
     if (e != cudaSuccess) return set_cuda_error(e);
-    P.pl_grid[PL_BP] = bp_grid(P.kind, P.pl_smem[PL_BP], P.pl_total[PL_BP]);
+    P.pl_grid[PL_BP] = bp_grid(P.kind, transposed, P.pl_smem[PL_BP], P.pl_total[PL_BP]);
     P.pl_grid[PL_FP] = fp_grid(P.kind, 2, P.pl_smem[PL_FP], P.pl_total[PL_FP]);
-    P.pl_grid[PL_INIT_BP] = bp_grid(P.kind, P.pl_smem[PL_INIT_BP], std::max(1, P.pl_total[PL_INIT_BP]));
+    P.pl_grid[PL_INIT_BP] = bp_grid(P.kind, transposed, P.pl_smem[PL_INIT_BP], std::max(1, P.pl_total[PL_INIT_BP]));
     P.pl_grid[PL_INIT_FP] = fp_grid(P.kind, 2, P.pl_smem[PL_INIT_FP], std::max(1, P.pl_total[PL_INIT_FP]));
-    P.pl_grid[PL_HESS] = bp_grid(P.kind, P.pl_smem[PL_HESS], std::max(1, P.pl_total[PL_HESS]));
+    P.pl_grid[PL_HESS] = bp_grid(P.kind, hess_transposed, P.pl_smem[PL_HESS], std::max(1, P.pl_total[PL_HESS]));
     {   // load every stage kernel now (lazy module loading must not happen inside a stream capture)
         cudaFuncAttributes fa;
         const void *ks[] = {reinterpret_cast<const void *>(b_delta), reinterpret_cast<const void *>(b_linquad),
@@ -1240,6 +1239,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
                             reinterpret_cast<const void *>(b_init_alpha),
                             reinterpret_cast<const void *>(b_init_apply),
                             reinterpret_cast<const void *>(b_copy_sino),
+                            reinterpret_cast<const void *>(b_transpose),
                             reinterpret_cast<const void *>(b_chunk_bounds)};
         for (const void *k : ks) cudaFuncGetAttributes(&fa, k);
         device_error_ptr();
@@ -1248,6 +1248,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     P.sn_grid = occupancy_grid(b_linquad, BT_THREADS, 0, L.sn_total);
     P.rc_grid = occupancy_grid(b_iter_partials, BT_THREADS, 0, L.sn_total + L.rc_total);
     P.flt_grid = occupancy_grid(b_filter, FILT_THREADS, std::max<size_t>(flt_smem, 1), std::max(1, L.flt_total));
+    P.tr_grid = occupancy_grid(b_transpose, 256, 0, std::max(1, L.tr_total));
     P.box_grid = occupancy_grid(b_chunk_bounds, CB_CHUNK, 0, std::max(1, L.box_total));
     e = cudaGetLastError();
     if (e != cudaSuccess) return set_cuda_error(e);
@@ -1272,10 +1273,9 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return set_cuda_error(e);
     if (autotune_enabled()) {  // (also in forced mode: the tune functions then apply the forced choice)
-        const int *o_bp = hpl_off + PL_BP * n1, *o_fp = hpl_off + PL_FP * n1;
+        const int *o_fp = hpl_off + PL_FP * n1;
         int rc2 = tune_batched_fp(P, L, zs, scans, hf, st);
         if (rc2 == MBX_OK) rc2 = tune_batched_fp_layouts(P, L, scans, o_fp, hpl_order + PL_FP * n, st);
-        if (rc2 == MBX_OK) rc2 = tune_batched_bp(P, L, scans, hb, o_bp, hpl_order + PL_BP * n, st);
         if (rc2 != MBX_OK) return rc2;
     }
     if (P.planned_fp) {  // the replay and build kernels of the forward variant the tuner kept
@@ -1300,7 +1300,7 @@ static int launch_stage(const BatchedPlanHost *P, int step, int stage, cudaStrea
     cudaError_t e = cudaSuccess;
     switch (stage) {
         case 0:
-            e = launch_bp_list(*P, PL_BP, step, 0, P->pl_total[PL_BP], P->pl_grid[PL_BP], P->pl_smem[PL_BP], st);
+            e = launch_bp_list(*P, PL_BP, step, st);
             return e == cudaSuccess ? MBX_OK : set_cuda_error(e);
         case 1: b_delta<<<P->el_grid, BT_THREADS, 0, st>>>(T, n, step, P->el_total, err); break;
         case 2:
@@ -1369,8 +1369,7 @@ extern "C" int mbx_vcd_batched_setup(const mbx_batched_plan *plan, void *stream)
         note_launch();
         e = cudaGetLastError();
         if (e == cudaSuccess)
-            e = launch_bp_list(*P, PL_INIT_BP, 0, 0, P->pl_total[PL_INIT_BP], P->pl_grid[PL_INIT_BP],
-                               P->pl_smem[PL_INIT_BP], st);
+            e = launch_bp_list(*P, PL_INIT_BP, 0, st);
         if (e == cudaSuccess)
             e = launch_fp_list(*P, PL_INIT_FP, 2, 0, 0, P->pl_total[PL_INIT_FP], P->pl_grid[PL_INIT_FP],
                                P->pl_smem[PL_INIT_FP], st);
@@ -1384,7 +1383,7 @@ extern "C" int mbx_vcd_batched_setup(const mbx_batched_plan *plan, void *stream)
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
-        e = launch_bp_list(*P, PL_HESS, 0, 0, P->pl_total[PL_HESS], P->pl_grid[PL_HESS], P->pl_smem[PL_HESS], st);
+        e = launch_bp_list(*P, PL_HESS, 0, st);
     return e == cudaSuccess ? MBX_OK : set_cuda_error(e);
 }
 

@@ -28,6 +28,8 @@ struct VcdScan {
     const float *y;             // measured sinogram (set-up input) or NULL
     long long nsino, nrecon;
     int K, M, nr, nc, ns;
+    float *tsino;               // transposed copy of the sinogram a back-projection stage reads, or NULL (bp_fast.cuh)
+    int V, R, C, rp;
 };
 
 // Direct-recon filtering of one scan in the set-up: rows of y into err.
@@ -71,7 +73,7 @@ struct BatchedTables {
     int *pl_off;        // [PL_COUNT][num_scans + 1]
     int *pl_dim;        // [PL_COUNT][num_scans]
     int *pl_order;      // [PL_COUNT][num_scans]
-    int *el_off, *sn_off, *rc_off, *flt_off;  // [num_scans + 1] tile prefix offsets (scan order)
+    int *el_off, *sn_off, *rc_off, *flt_off, *tr_off;  // [num_scans + 1] tile prefix offsets (scan order)
     int *box_first;     // [num_scans * K + 1] chunk prefix over (scan, subset) records
     int *counters;      // [PL_COUNT]
     int *schedule;      // [num_steps][num_scans]
@@ -91,8 +93,10 @@ struct BatchedPlanHost {
     size_t plan_cursor_bytes;
     int pl_total[PL_COUNT], pl_grid[PL_COUNT];
     size_t pl_smem[PL_COUNT];
-    int el_total, sn_total, rc_total, flt_total, box_total;
-    int el_grid, sn_grid, rc_grid, flt_grid, box_grid;
+    int el_total, sn_total, rc_total, flt_total, box_total, tr_total;
+    int el_grid, sn_grid, rc_grid, flt_grid, box_grid, tr_grid;
+    int transposed;       // the back projections read transposed copies (PL_HESS: when hess_transposed)
+    int hess_transposed;
     size_t flt_smem;
     int fp_minb;  // b_fp variant of the subset stage: 2 or 3 resident CTAs per SM
     size_t fp_smem_replay;  // shared memory of the replay kernel (the replay layouts of the subset plans)
@@ -158,10 +162,6 @@ __device__ __forceinline__ int fetch_tile(int *counter) {
 
 #ifndef MBX_BATCHED_FP_CAP
 #define MBX_BATCHED_FP_CAP 2048  // most records per pass of the batched forward projections (and their stored passes)
-#endif
-
-#ifndef MBX_BBP_MIN_BLOCKS
-#define MBX_BBP_MIN_BLOCKS 3  // resident CTAs per SM the batched back projection is compiled for
 #endif
 
 // Record of scan s in a work list at a step.
