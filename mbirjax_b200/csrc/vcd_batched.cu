@@ -35,7 +35,7 @@ namespace mbx {
 
 // Each warp takes units (an eighth of a list tile) of its own: warps share nothing but the counter.
 template <int KIND, bool TR>
-__global__ void __launch_bounds__(32 * BPF_LAUNCH_WARPS, bpf_min_blocks(KIND))
+__global__ void __launch_bounds__(32 * BPF_LAUNCH_WARPS, 8)
 b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
     extern __shared__ __align__(128) float smb[];
     float *smw = smb + (threadIdx.x >> 5) * bpf_warp_floats(KIND);
