@@ -291,14 +291,14 @@ __global__ void __launch_bounds__(BT_THREADS) b_zero_recon(BatchedTables T, int 
     }
 }
 
-// FBP / FDK filtering of every scan's sinogram, FILT_ROWS detector rows per tile (direct_filter_rows).
-__global__ void __launch_bounds__(FILT_THREADS) b_filter(BatchedTables T, int num_scans, int total) {
-    extern __shared__ __align__(16) float smflt[];
+// FBP / FDK filtering of every scan's sinogram, filter_shape(C).rows detector rows per tile (direct_filter_rows).
+__global__ void __launch_bounds__(FILT_THREADS, 2) b_filter(BatchedTables T, int num_scans, int total) {
+    extern __shared__ __align__(16) double smflt[];
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         const int s = find_scan(T.flt_off, num_scans, t);
         const int local = t - __ldg(T.flt_off + s);
         const FiltScan &f = T.filt[s];
-        direct_filter_rows(f.in, f.out, (long long)local * FILT_ROWS, f.rows, f.R, f.C, f.filter_scale, f.out_scale,
+        direct_filter_rows(f.in, f.out, (long long)local * filter_shape(f.C).rows, f.rows, f.R, f.C, f.filter_scale, f.out_scale,
                            f.fdk, f.D, f.ddc, f.ddr, f.dco, f.dro, smflt);
     }
 }
@@ -425,11 +425,11 @@ static int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
         if (z.hbp_slices == 0) z.hbp = plan_bp_fast(g, z.npix, g.num_views);
         if (!z.hbp.ok) return MBX_ERR_UNSUPPORTED;
         if (g.kind != MBX_GEOM_TRANSLATION) {  // translation geometry starts from zeros (no direct recon)
-            if (filter_smem_bytes(g.num_det_channels, g.kind != MBX_GEOM_PARALLEL) > 200 * 1024)
+            if (!filter_admits(g.num_det_channels, g.kind != MBX_GEOM_PARALLEL))
                 return MBX_ERR_UNSUPPORTED;
             z.ibp = plan_bp_fast(g, sc.num_full_indices, g.num_views);
             if (!z.ibp.ok) return MBX_ERR_UNSUPPORTED;
-            z.flt_tiles = (int)(((long long)g.num_views * g.num_det_rows + FILT_ROWS - 1) / FILT_ROWS);
+            z.flt_tiles = ceil_div((long long)g.num_views * g.num_det_rows, filter_shape(g.num_det_channels).rows);
         } else {
             z.ibp = z.hbp;  // unused
         }
@@ -1207,8 +1207,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     size_t flt_smem = 0;
     for (int s = 0; s < n; ++s)
         if (zs[s].setup)
-            flt_smem = std::max(flt_smem, filter_smem_bytes(scans[s].geom.num_det_channels,
-                                                            scans[s].geom.kind != MBX_GEOM_PARALLEL));
+            flt_smem = std::max(flt_smem, filter_smem_bytes(scans[s].geom.num_det_channels));
     P.flt_smem = flt_smem;
     // kernel attributes and resident-CTA grids
     const void *kfp2 = fp_kernel_of(P.kind, 2), *kfp3 = fp_kernel_of(P.kind, 3);
