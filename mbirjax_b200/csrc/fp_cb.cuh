@@ -77,7 +77,10 @@ struct CbPlan {
 // secant-weighted voxels of the slices its rows of one row pass touch, for slopes of at least 2/3 row per slice;
 // a record with a wider span is read tap by tap instead).
 __host__ __device__ constexpr int cb_cone_records(int rpl) { return (CB_LOADS / rpl) > 0 ? (CB_LOADS / rpl) : 1; }
-__host__ __device__ constexpr int cb_cone_window(int ppw, int rpl) { return (3 * rpl * (32 / ppw)) / 2 + 4; }
+// Whole steps of the sub-group's lanes, which stage the window without a guard on its end.
+__host__ __device__ constexpr int cb_cone_window(int ppw, int rpl) {
+    return ((3 * rpl * (32 / ppw)) / 2 + 4 + 32 / ppw - 1) / (32 / ppw) * (32 / ppw);
+}
 
 // Walk layout for passes of cap records: tile copies, sorted records (+ the cone's second words), bins, scan
 // order, bin starts, histogram, per-warp counts and starts, cone row tables, chunk hit list, warp counts, cone
@@ -460,25 +463,11 @@ __device__ __forceinline__ float cb_value(const float *cyl, int m, int num_slice
     return val;
 }
 
-// The same value for a cone / translation record from its slice window: wp points at slice k_c of the window,
-// which holds voxel k times its secant (the product cb_value forms), so the taps, their order and their rounding
-// are cb_value's.
-__device__ __forceinline__ float cb_value_win(const float *wp, int k_c, int m, int num_slices, const float4 &cv,
-                                              const CbRow &rw, float kconst) {
-    const float w_r = cv.y;
-    const float k_m0 = fmaf(rw.vb, cv.x, kconst);
-    const float dm = fmaf(w_r, (float)k_c - k_m0, (float)(rw.b0 - m));
-    const float half_w = (w_r + 1.0f) * 0.5f, l_max = fminf(1.0f, w_r);
-    float val = 0.0f;
-#pragma unroll
-    for (int ko = -1; ko <= 1; ++ko) {
-        const int k = k_c + ko;
-        if (k >= 0 && k < num_slices) {
-            const float a = fminf(fmaxf(half_w - fabsf(fmaf(w_r, (float)ko, dm)), 0.0f), l_max);
-            val = fmaf(a, wp[ko], val);
-        }
-    }
-    return val;
+// 1 / sqrt(x) for x >= 1 (rsqrtf without its scaling of denormals).
+__device__ __forceinline__ float cb_rsqrt(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
 // What one warp needs to accumulate one pass.
@@ -493,13 +482,25 @@ struct CbPass {
     int b_lo, b_hi;            // this warp's bins
 };
 
+// Read-only load of *p into v when ok; v keeps its value otherwise (a predicated load, no select).
+__device__ __forceinline__ void ldg_if(float &v, const float *p, int ok) {
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+        : "+f"(v)
+        : "l"(p), "r"(ok));
+}
+
 // Accumulation of one pass by one warp: PPW sub-groups, RPL rows per lane; then the edge writes.
-// Cone and translation records: per loop iteration the warp stages, for each of its U records per sub-group,
-// the slices the sub-group's rows of the row pass touch (a window of voxel x secant, one coalesced load per
-// slice) in shared memory, and each row reads its three taps from there; a record whose slice span exceeds the
-// window (slopes under 2/3 row per slice) makes the warp read tap by tap for that iteration (cb_value).  Both
-// ways give a record's row value with the same operations in the same order.  Against three scattered loads and
-// three secants per row, the window made the cone subset projection 1.57x faster (256 views x 128 x 256).
+// Cone and translation records: per loop iteration the warp stages, for each of its U records per sub-group, the slices
+// the sub-group's rows of the row pass touch (a window of voxel x secant, zero off the volume, one coalesced load per
+// slice) in shared memory, and each row reads its three taps from there with no bounds tests.  The row of a lane takes
+// slices k_c - 1, k_c, k_c + 1 with k_c the nearest to the row centre's k_m (rounded by adding and removing 1.5 x 2^23,
+// whose low mantissa bits are then the slice), with overlap min(max(half_w - |dm + w_r ko|, 0), l_max), |dm| <= w_r / 2;
+// for w_r >= 1/2 the clips that cannot act are left out.  A record whose slice span exceeds the window (slopes under 2/3
+// row per slice), with w_r < 1/2 or with rows off any sensible volume makes the warp read tap by tap for that iteration
+// (cb_value).
+// The kernel is bound by instruction issue.  Against three scattered loads and three secants per row, the window made
+// the cone subset projection 1.57x faster (256 views x 128 x 256); leaving out the tests and clips, one search for each
+// record's window and two running sums less per row took it from 1.79 to 1.64 ms.
 template <int KIND, int PPW, int RPL>
 __device__ __forceinline__ void cb_accumulate(const FpArgs &A, const CbPass &P, int warp, int lane, float kconst) {
     const mbx_geom &g = A.g;
@@ -507,146 +508,171 @@ __device__ __forceinline__ void cb_accumulate(const FpArgs &A, const CbPass &P, 
     constexpr int RL = 32 / PPW;
     constexpr int U = cb_cone_records(RPL);          // records prefetched per lane
     constexpr int WIN = cb_cone_window(PPW, RPL);    // window floats per record and sub-group
+    const float magic = 12582912.0f;
     const int sub = lane / RL, lr = lane % RL;
-    const int num_rows = g.num_det_rows, num_slices = g.num_recon_slices, nb = pl.nb;
+    const int num_rows = g.num_det_rows, num_slices = g.num_recon_slices, nb = pl.nb, pitch = pl.pitch;
     // this sub-group's records: every PPW-th of the warp's range, so the sub-groups walk the same bins in step
     const int w_lo = P.bstart[P.b_lo], w_hi = P.bstart[P.b_hi];
     const int r_a = w_lo + sub, r_b = w_hi;
     // edge channels of the warp's range: E0, E1 (shared with the warp below), E2, E3 (with the warp above)
     const int E0 = P.b_lo - 2, E1 = P.b_lo - 1, E2 = P.b_hi - 2, E3 = P.b_hi - 1;
+    float *wbase = P.win + ((size_t)warp * U * PPW + sub) * WIN;  // window of record u: + u * PPW * WIN
     for (int rp = 0; rp < pl.row_passes; ++rp) {
-        int m[RPL], mcl[RPL];
-        const float *vb[RPL];
-        float *trow[RPL];
-        CbRow rw[RPL];
+        const int m0 = rp * RPL * RL + lr;  // row of slot 0; slot j is row m0 + j * RL
+        float vm[RPL], vb[RPL], b0m[RPL];   // detector heights of the row and its batch's first row, batch row - row
 #pragma unroll
         for (int j = 0; j < RPL; ++j) {
-            m[j] = (rp * RPL + j) * RL + lr;
-            const int mc = min(m[j], num_rows - 1);  // rows past R read a valid row; never written out
-            mcl[j] = mc;
-            vb[j] = A.vox + (KIND == MBX_GEOM_PARALLEL ? mc : 0);
-            trow[j] = P.tile + ((size_t)sub * pl.rpad + m[j]) * pl.pitch;
-            rw[j].vm = rw[j].vb = 0.f;
-            rw[j].b0 = 0;
-            if (KIND != MBX_GEOM_PARALLEL) {
-                rw[j].vm = P.s_vm[mc];
-                rw[j].vb = P.s_vb[mc];
-                rw[j].b0 = P.s_b0[mc];
-            }
+            const int mc = min(m0 + j * RL, num_rows - 1);  // rows past R read a valid row; never written out
+            vm[j] = P.s_vm[mc];
+            vb[j] = P.s_vb[mc];
+            b0m[j] = (float)(P.s_b0[mc] - mc);
         }
-        // before bin bc: x = sum for channel bc-2, y = sum for channel bc-1; bin bc adds s0/s1/s2 to them and bc
-        float x[RPL], y[RPL], s0[RPL], s1[RPL], s2[RPL], e0[RPL], e1[RPL], e2[RPL], e3[RPL];
+        float *trow0 = P.tile + ((size_t)sub * pl.rpad + m0) * pitch;
+        // running sums: before bin bc completes, ca, cbb, cc hold channels bc-2, bc-1, bc; as in cb_accumulate_par
+        float ca[RPL], cbb[RPL], cc[RPL], e0[RPL], e1[RPL];
 #pragma unroll
-        for (int j = 0; j < RPL; ++j) x[j] = y[j] = s0[j] = s1[j] = s2[j] = e0[j] = e1[j] = e2[j] = e3[j] = 0.0f;
+        for (int j = 0; j < RPL; ++j) ca[j] = cbb[j] = cc[j] = e0[j] = e1[j] = 0.0f;
         int bc = (r_a < r_b) ? P.sbin[r_a] : 0;
-        // bin bc is complete: channel bc-2 receives its sum
+        // bin bc is complete: channel bc-2 is done
         auto finish = [&]() {
             const int c = bc - 2;
-            const bool interior = c >= P.b_lo && c <= P.b_hi - 3;
+            const bool interior = c >= P.b_lo;  // in the walk c <= b_hi - 4 always
+            const bool is0 = c == E0, is1 = c == E1;
 #pragma unroll
             for (int j = 0; j < RPL; ++j) {
-                const float v = x[j] + s0[j];
-                x[j] = y[j] + s1[j];
-                y[j] = s2[j];
-                s0[j] = s1[j] = s2[j] = 0.0f;
-                if (interior) {
-                    trow[j][c] += v;
-                } else {
-                    e0[j] += (c == E0) ? v : 0.0f;
-                    e1[j] += (c == E1) ? v : 0.0f;
-                    e2[j] += (c == E2) ? v : 0.0f;
-                    e3[j] += (c == E3) ? v : 0.0f;
-                }
+                if (interior) trow0[j * RL * pitch + c] += ca[j];
+                e0[j] = is0 ? ca[j] : e0[j];
+                e1[j] = is1 ? ca[j] : e1[j];
+                ca[j] = cbb[j];
+                cbb[j] = cc[j];
+                cc[j] = 0.0f;
             }
             ++bc;
         };
-        float *wbase = P.win + (size_t)warp * U * PPW * WIN;
         // detector heights of the sub-group's first and last rows of this row pass: their centre slices bound
         // those of all its rows (k_c is monotone in the row)
-        const float vm_first = __shfl_sync(0xffffffffu, rw[0].vm, sub * RL);
-        const float vm_last = __shfl_sync(0xffffffffu, rw[RPL - 1].vm, sub * RL + RL - 1);
-        // first slice of a record's window and the window's length
-        auto window_of = [&](const float4 &cv, int &lo, int &len) {
-            const int kf = (int)rintf(fmaf(vm_first, cv.x, kconst));
-            const int kl = (int)rintf(fmaf(vm_last, cv.x, kconst));
-            lo = min(kf, kl) - 1;
-            len = max(kf, kl) - lo + 2;
-        };
+        const float vm_first = __shfl_sync(0xffffffffu, vm[0], sub * RL);
+        const float vm_last = __shfl_sync(0xffffffffu, vm[RPL - 1], sub * RL + RL - 1);
         // the loop runs over the warp's range (the same trip count in every sub-group, for the warp-wide window
         // exchange); a sub-group's records past its own range are read but contribute nothing
         for (int i = r_a; i - sub < w_hi; i += U * PPW) {
-            float4 rq[U], cq[U];
-            int bq[U];
+            // records past the end: reread the last record of the warp's range
+            auto second = [&](int u) { return P.rec2[min(i + u * PPW, w_hi - 1)]; };
+            int lo[U], len[U];  // first slice and length of each record's window
             float vq[U][RPL];
-            int fits = 1;
+            bool fits = true;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                // past the end: reread the last record of the warp's range, contribute nothing
-                const int ii = min(i + u * PPW, w_hi - 1);
-                rq[u] = P.rec[ii];
-                bq[u] = P.sbin[ii];
-                cq[u] = P.rec2[ii];
-                int lo, len;
-                window_of(cq[u], lo, len);
-                if (len > WIN) fits = 0;
+                const float4 cq = second(u);
+                const float kf = fmaf(vm_first, cq.x, kconst), kl = fmaf(vm_last, cq.x, kconst);
+                lo[u] = (int)rintf(fminf(kf, kl)) - 1;
+                len[u] = (int)rintf(fmaxf(kf, kl)) - lo[u] + 2;
+                fits = fits && len[u] <= WIN && fabsf(kf) < 4.0e6f && fabsf(kl) < 4.0e6f && cq.y >= 0.5f;
             }
             if (__all_sync(0xffffffffu, fits)) {
+                float y[U][WIN / RL];  // every record's slices in flight together
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    int lo, len;
-                    window_of(cq[u], lo, len);
-                    float *w = wbase + (u * PPW + sub) * WIN;
-                    const float *cyl = A.vox + __float_as_int(rq[u].x);
-                    for (int t = lr; t < len; t += RL) {
-                        const int k = lo + t;
-                        float y = 0.0f;
-                        if (k >= 0 && k < num_slices) {
-                            const float tt = fmaf((float)k, cq[u].z, cq[u].w);
+                    const int k0 = lo[u] + lr;
+                    const float *cyl = A.vox + (__float_as_int(P.rec[min(i + u * PPW, w_hi - 1)].x) + k0);
+#pragma unroll
+                    for (int t = 0; t < WIN / RL; ++t) {
+                        y[u][t] = 0.0f;
+                        ldg_if(y[u][t], cyl + t * RL, (unsigned)(k0 + t * RL) < (unsigned)num_slices && t * RL < len[u]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const float4 cq = second(u);
+                    float *w = wbase + u * PPW * WIN + lr;
+                    const float kf = (float)(lo[u] + lr);
+#pragma unroll
+                    for (int t = 0; t < WIN / RL; ++t) {
+                        if (t * RL < len[u]) {
+                            const float tt = fmaf(kf + (float)(t * RL), cq.z, cq.w);
                             const float q = fmaf(tt, tt, 1.0f);
-                            y = __ldg(cyl + k) * (q * rsqrtf(q));
+                            w[t * RL] = y[u][t] * (q * cb_rsqrt(q));
                         }
-                        w[t] = y;
                     }
                 }
                 __syncwarp();
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    int lo, len;
-                    window_of(cq[u], lo, len);
-                    const float *w = wbase + (u * PPW + sub) * WIN;
+                    const float4 cq = second(u);
+                    const float w_r = cq.y;
+                    const float half_w = (w_r + 1.0f) * 0.5f, l_max = fminf(1.0f, w_r);
+                    const float hw1 = half_w - w_r;
+                    const float *w = wbase + u * PPW * WIN;
+                    const int bits0 = __float_as_int(magic) + lo[u];
 #pragma unroll
                     for (int j = 0; j < RPL; ++j) {
-                        const int k_c = (int)rintf(fmaf(rw[j].vm, cq[u].x, kconst));
-                        vq[u][j] = cb_value_win(w + (k_c - lo), k_c, mcl[j], num_slices, cq[u], rw[j], kconst);
+                        const float r = fmaf(vm[j], cq.x, kconst) + magic;
+                        const float k_c = r - magic;
+                        const float *wp = w + (__float_as_int(r) - bits0);
+                        const float dm = fmaf(w_r, k_c - fmaf(vb[j], cq.x, kconst), b0m[j]);
+                        const float l_m = fmaxf(hw1 + dm, 0.0f), l_p = fmaxf(hw1 - dm, 0.0f);
+                        const float l_0 = fminf(half_w - fabsf(dm), l_max);
+                        vq[u][j] = fmaf(l_p, wp[1], fmaf(l_0, wp[0], l_m * wp[-1]));
                     }
                 }
                 __syncwarp();  // the next iteration's windows overwrite these
             } else {
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int off = __float_as_int(rq[u].x);  // 32-bit element offset of the cylinder
+                    const int off = __float_as_int(P.rec[min(i + u * PPW, w_hi - 1)].x);  // 32-bit element offset
+#pragma unroll 1
+                    for (int j = 0; j < RPL; ++j) {
+                        const int mc = min(m0 + j * RL, num_rows - 1);
+                        CbRow rw;
+                        rw.vm = P.s_vm[mc];
+                        rw.vb = P.s_vb[mc];
+                        rw.b0 = P.s_b0[mc];
+                        const float v = cb_value<KIND>(A.vox + off, mc, num_slices, second(u), rw, kconst);
 #pragma unroll
-                    for (int j = 0; j < RPL; ++j)
-                        vq[u][j] = cb_value<KIND>(vb[j] + off, mcl[j], num_slices, cq[u], rw[j], kconst);
+                        for (int jj = 0; jj < RPL; ++jj)
+                            if (jj == j) vq[u][jj] = v;
+                    }
                 }
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                if (i + u * PPW < r_b) {
-                    while (bc < bq[u]) finish();
+                const int ii = i + u * PPW;
+                if (ii < r_b) {
+                    const float4 rq = P.rec[ii];
+                    const int bq = P.sbin[ii];
+                    while (bc < bq) finish();
 #pragma unroll
                     for (int j = 0; j < RPL; ++j) {
-                        s0[j] = fmaf(rq[u].y, vq[u][j], s0[j]);
-                        s1[j] = fmaf(rq[u].z, vq[u][j], s1[j]);
-                        s2[j] = fmaf(rq[u].w, vq[u][j], s2[j]);
+                        ca[j] = fmaf(rq.y, vq[u][j], ca[j]);
+                        cbb[j] = fmaf(rq.z, vq[u][j], cbb[j]);
+                        cc[j] = fmaf(rq.w, vq[u][j], cc[j]);
                     }
                 }
             }
         }
-        if (r_a < r_b) {  // the last bin and the two channels above it
-            finish();
-            finish();
-            finish();
+        // final flush: channels bc-2, bc-1, bc; the ones above b_hi - 3 are shared with the warp above
+        float e2[RPL], e3[RPL];
+#pragma unroll
+        for (int j = 0; j < RPL; ++j) e2[j] = e3[j] = 0.0f;
+        if (r_a < r_b) {
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                const int c = bc - 2 + t;
+#pragma unroll
+                for (int j = 0; j < RPL; ++j) {
+                    const float v = (t == 0) ? ca[j] : (t == 1 ? cbb[j] : cc[j]);
+                    if (c == E0)
+                        e0[j] = v;
+                    else if (c == E1)
+                        e1[j] = v;
+                    else if (c == E2)
+                        e2[j] = v;
+                    else if (c == E3)
+                        e3[j] = v;
+                    else
+                        trow0[j * RL * pitch + c] += v;
+                }
+            }
         }
         // edge channels: even warps first, then odd warps
 #pragma unroll
@@ -655,21 +681,15 @@ __device__ __forceinline__ void cb_accumulate(const FpArgs &A, const CbPass &P, 
             if ((warp & 1) == ph) {
 #pragma unroll
                 for (int j = 0; j < RPL; ++j) {
-                    if (E0 >= 0) trow[j][E0] += e0[j];
-                    if (E1 >= 0) trow[j][E1] += e1[j];
-                    if (E2 < nb) trow[j][E2] += e2[j];
-                    if (E3 < nb) trow[j][E3] += e3[j];
+                    float *tr = trow0 + j * RL * pitch;
+                    if (E0 >= 0) tr[E0] += e0[j];
+                    if (E1 >= 0) tr[E1] += e1[j];
+                    if (E2 < nb) tr[E2] += e2[j];
+                    if (E3 < nb) tr[E3] += e3[j];
                 }
             }
         }
     }
-}
-
-// Read-only load of *p into v when ok; v keeps its value otherwise (a predicated load, no select).
-__device__ __forceinline__ void ldg_if(float &v, const float *p, int ok) {
-    asm("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
-        : "+f"(v)
-        : "l"(p), "r"(ok));
 }
 
 #ifndef MBX_FPCB_LOADS2
