@@ -106,8 +106,8 @@ MBX_API uint64_t mbx_launch_count(void);
  * schedule; the back projector has one plan per call shape).  The first mbx_sparse_forward_project of a call shape
  * (geometry sizes, views, pixel count rounded up to a power of two) times its candidate plans on the caller's stream,
  * synchronising it, and caches the fastest for the process; a call made while its stream is captured uses the
- * default plan.  Candidates: channel-block width, pass size, and the kernel variant compiled for 2 or 3 resident CTAs
- * per SM.
+ * default plan.  Candidates: channel-block width, pass size, lane layout, and the kernel variant compiled for 2 or
+ * for more (parallel beam 4, else 3) resident CTAs per SM.
  * mbx_vcd_batched_prepare tunes its forward stage the same way, cached per batch shape.  Plans differ
  * only in float summation order.  mode: 0 = default plans, 1 = tune (default), k >= 2 = use candidate k-1 (or the
  * last one) everywhere without timing (to check every plan against the default).  Returns the previous mode. */

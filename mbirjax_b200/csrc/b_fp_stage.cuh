@@ -6,7 +6,7 @@
 
 namespace mbx {
 
-// MINB: resident CTAs per SM the variant is compiled for (2 or 3, matching the plans' fp_cb minb).
+// MINB: resident CTAs per SM the variant is compiled for (2 or cb_many, matching the plans' fp_cb minb).
 template <int KIND, int MINB>
 __global__ void __launch_bounds__(CB_THREADS, MINB) b_fp(ProjList L, int num_scans, int step, int first, int total, int *err) {
     extern __shared__ __align__(16) float smf2[];
@@ -63,12 +63,12 @@ __global__ void __launch_bounds__(CB_THREADS, MINB) b_fp_build(ProjList L, int n
 template <int KIND>
 const void *fp_stage_kernel_kind(int minb, int mode) {
     if (mode == CB_REPLAY)
-        return minb >= 3 ? reinterpret_cast<const void *>(b_fp_replay<KIND, 3>)
+        return minb > 2 ? reinterpret_cast<const void *>(b_fp_replay<KIND, cb_many(KIND)>)
                          : reinterpret_cast<const void *>(b_fp_replay<KIND, 2>);
     if (mode == CB_BUILD)
-        return minb >= 3 ? reinterpret_cast<const void *>(b_fp_build<KIND, 3>)
+        return minb > 2 ? reinterpret_cast<const void *>(b_fp_build<KIND, cb_many(KIND)>)
                          : reinterpret_cast<const void *>(b_fp_build<KIND, 2>);
-    return minb >= 3 ? reinterpret_cast<const void *>(b_fp<KIND, 3>) : reinterpret_cast<const void *>(b_fp<KIND, 2>);
+    return minb > 2 ? reinterpret_cast<const void *>(b_fp<KIND, cb_many(KIND)>) : reinterpret_cast<const void *>(b_fp<KIND, 2>);
 }
 
 template <int KIND, int MINB>
@@ -86,8 +86,8 @@ void launch_fp_stage_minb(int mode, int grid, size_t smem, cudaStream_t st, cons
 template <int KIND>
 void launch_fp_stage_kind(int minb, int mode, int grid, size_t smem, cudaStream_t st, const ProjList &L, int n,
                           int step, int first, int total, int *err) {
-    if (minb >= 3)
-        launch_fp_stage_minb<KIND, 3>(mode, grid, smem, st, L, n, step, first, total, err);
+    if (minb > 2)
+        launch_fp_stage_minb<KIND, cb_many(KIND)>(mode, grid, smem, st, L, n, step, first, total, err);
     else
         launch_fp_stage_minb<KIND, 2>(mode, grid, smem, st, L, n, step, first, total, err);
 }

@@ -244,15 +244,17 @@ static cudaError_t launch_fp_cb_v(const FpArgs &A, cudaStream_t st) {
 }
 
 static cudaError_t launch_fp_cb(const FpArgs &A, cudaStream_t st) {
-    const bool three = A.plan.minb >= 3;
+    const bool many = A.plan.minb > 2;
     switch (A.g.kind) {
         case MBX_GEOM_PARALLEL:
-            return three ? launch_fp_cb_v<MBX_GEOM_PARALLEL, 3>(A, st) : launch_fp_cb_v<MBX_GEOM_PARALLEL, 2>(A, st);
+            return many ? launch_fp_cb_v<MBX_GEOM_PARALLEL, cb_many(MBX_GEOM_PARALLEL)>(A, st)
+                        : launch_fp_cb_v<MBX_GEOM_PARALLEL, 2>(A, st);
         case MBX_GEOM_CONE:
-            return three ? launch_fp_cb_v<MBX_GEOM_CONE, 3>(A, st) : launch_fp_cb_v<MBX_GEOM_CONE, 2>(A, st);
+            return many ? launch_fp_cb_v<MBX_GEOM_CONE, cb_many(MBX_GEOM_CONE)>(A, st)
+                        : launch_fp_cb_v<MBX_GEOM_CONE, 2>(A, st);
         default:
-            return three ? launch_fp_cb_v<MBX_GEOM_TRANSLATION, 3>(A, st)
-                         : launch_fp_cb_v<MBX_GEOM_TRANSLATION, 2>(A, st);
+            return many ? launch_fp_cb_v<MBX_GEOM_TRANSLATION, cb_many(MBX_GEOM_TRANSLATION)>(A, st)
+                        : launch_fp_cb_v<MBX_GEOM_TRANSLATION, 2>(A, st);
     }
 }
 

@@ -43,6 +43,12 @@ namespace mbx {
 
 constexpr int CB_THREADS = 256;
 constexpr int CB_WARPS = CB_THREADS / 32;
+// Resident CTAs per SM of the second kernel variant (the first is compiled for 2): 4 for parallel beam, whose walk waits
+// on row loads and gains from twice the warps (64 registers and 55 KB of shared memory are enough for it with 64 channels
+// and 1024 records: 652 x 57 x 437 subset 1.66 -> 1.58 ms, 400 x 22 x 300 0.50 -> 0.41 ms in the same lane layout); 3 for
+// the fan geometries, which need more registers.
+__host__ __device__ constexpr int cb_many(int kind) { return kind == MBX_GEOM_PARALLEL ? 4 : 3; }
+constexpr int CB_MANY_CHANNELS = 64, CB_MANY_CAP = 1024;  // channels per block and records per pass of the 4-CTA variant
 constexpr int CB_LOADS = 8;  // loads in flight per lane in the accumulation walk
 constexpr int CB_PAD = 32;   // padding records after a pass's last record: the parallel walk reads U * PPW <= 32 ahead
 constexpr int CB_MAX_PASSES = 64;  // passes of one tile a planned list can hold (more: the tile is not planned)
@@ -65,7 +71,7 @@ struct CbPlan {
     int pitch;       // tile row pitch (nb + 1)
     int nbins;       // nb + 2
     int cblocks;     // channel blocks per view
-    int minb;        // resident CTAs per SM the kernel variant is compiled for (2 or 3)
+    int minb;        // resident CTAs per SM the kernel variant is compiled for (2 or cb_many)
     CbLayout walk;   // scan, sort and walk passes of walk.cap records (also the build of stored passes)
     CbLayout replay; // replay of stored passes (of walk.cap records): the tile, records, bins and bin starts only,
                      // which leaves the rest of the SM's shared memory to the L1 cache that serves the row loads
@@ -159,8 +165,8 @@ inline void cb_plan_replay(CbPlan &pl, int kind, int R) {
 }
 
 // num_views_sel: views per call (0 = all); min_blocks: CTAs wanted per call (a narrower channel block is
-// chosen to reach it); 0 = widest block.  minb: 2 (first shared-memory tier 112 KB) or 3 (74 KB, for the kernel
-// variant compiled for three resident CTAs per SM); nb_max: widest channel block allowed.
+// chosen to reach it); 0 = widest block.  minb: 2 (first shared-memory tier 112 KB), 3 (74 KB) or 4 (55 KB), for the
+// kernel variants compiled for that many resident CTAs per SM; nb_max: widest channel block allowed.
 // avoid_ppw: when nonzero, the best lane layout with a different number of sub-groups (an autotuner candidate).
 // max_cap: most records per pass.
 inline CbPlan plan_fp_cb(const mbx_geom &g, int num_views_sel = 0, long long min_blocks = 0, int minb = 2,
@@ -192,7 +198,10 @@ inline CbPlan plan_fp_cb(const mbx_geom &g, int num_views_sel = 0, long long min
     pl.row_passes = ceil_div(R, pl.rl * pl.rpl);
     pl.rpad = pl.row_passes * pl.rl * pl.rpl;
     // widest channel block, then largest pass, that fit the shared-memory tier (2, then 1 CTA per SM)
-    const size_t tiers[2] = {minb >= 3 ? (size_t)74 * 1024 : (size_t)MBX_FPCB_SMEM_TIER0, (size_t)200 * 1024};
+    const size_t tiers[2] = {minb >= 4   ? (size_t)55 * 1024
+                             : minb >= 3 ? (size_t)74 * 1024
+                                         : (size_t)MBX_FPCB_SMEM_TIER0,
+                             (size_t)200 * 1024};
     bool found = false;
     for (int t = 0; t < 2 && !found; ++t) {
         for (int nb = nb_max; nb >= 32 && !found; nb >>= 1) {
@@ -224,17 +233,25 @@ inline CbPlan plan_fp_cb(const mbx_geom &g, int num_views_sel = 0, long long min
     return pl;
 }
 
-// The plans an autotuner times for one call shape: the default, the variant compiled for three resident CTAs
-// per SM (smaller passes), narrower channel blocks (more CTAs, shorter bins), and the best lane layout with a
-// different number of sub-groups per warp.  Returns how many are usable.
-constexpr int CB_MAX_CANDIDATES = 4;
+// The plan of the second kernel variant for channel blocks of at most nb_max channels.
+inline CbPlan plan_fp_many(const mbx_geom &g, int num_views_sel, long long min_blocks, int nb_max, int avoid_ppw = 0,
+                           int max_cap = 2048) {
+    const bool four = cb_many(g.kind) >= 4;
+    return plan_fp_cb(g, num_views_sel, min_blocks, cb_many(g.kind), four ? std::min(nb_max, CB_MANY_CHANNELS) : nb_max,
+                      avoid_ppw, four ? std::min(max_cap, CB_MANY_CAP) : max_cap);
+}
+
+// The plans an autotuner times for one call shape: the default, the variant compiled for more resident CTAs per SM
+// (narrower blocks or smaller passes), narrower channel blocks (more CTAs, shorter bins), and the best lane layout with
+// a different number of sub-groups per warp of the first two.  Returns how many are usable.
+constexpr int CB_MAX_CANDIDATES = 5;
 inline int fp_cb_candidates(const mbx_geom &g, int num_views_sel, long long min_blocks,
                             CbPlan out[CB_MAX_CANDIDATES]) {
     int n = 0;
     const CbPlan c0 = plan_fp_cb(g, num_views_sel, min_blocks, 2, 128);
     if (!c0.ok) return 0;
     out[n++] = c0;
-    const CbPlan c1 = plan_fp_cb(g, num_views_sel, min_blocks, 3, 128);
+    const CbPlan c1 = plan_fp_many(g, num_views_sel, min_blocks, 128);
     if (c1.ok) out[n++] = c1;
     if (c0.nb > 32) {
         const CbPlan c2 = plan_fp_cb(g, num_views_sel, min_blocks, 2, c0.nb / 2);
@@ -242,6 +259,10 @@ inline int fp_cb_candidates(const mbx_geom &g, int num_views_sel, long long min_
     }
     const CbPlan c3 = plan_fp_cb(g, num_views_sel, min_blocks, 2, 128, c0.ppw);
     if (c3.ok) out[n++] = c3;
+    if (c1.ok && cb_many(g.kind) >= 4) {
+        const CbPlan c4 = plan_fp_many(g, num_views_sel, min_blocks, 128, c1.ppw);
+        if (c4.ok) out[n++] = c4;
+    }
     return n;
 }
 
@@ -696,7 +717,7 @@ __device__ __forceinline__ void cb_accumulate(const FpArgs &A, const CbPass &P, 
 #define MBX_FPCB_LOADS2 12  // parallel walk: row loads in flight per lane, variant for 2 CTAs per SM
 #endif
 #ifndef MBX_FPCB_LOADS3
-#define MBX_FPCB_LOADS3 16  // the same, variant for 3 CTAs per SM (85 registers)
+#define MBX_FPCB_LOADS3 8  // the same, variant for 4 CTAs per SM (64 registers)
 #endif
 
 // Parallel-beam accumulation of one pass by one warp (same contract and record interleaving as cb_accumulate).
@@ -1276,7 +1297,7 @@ __device__ void fp_cb_tile(const FpArgs &A, int j, int cb, float *sm, int *err, 
     }
 }
 
-// MINB = plan.minb: the variant compiled for 2 resident CTAs per SM (up to 128 registers) or 3 (up to 85).
+// MINB = plan.minb: the variant compiled for 2 resident CTAs per SM (up to 128 registers) or cb_many (64 or 80).
 template <int KIND, int MINB>
 __global__ void __launch_bounds__(CB_THREADS, MINB) fp_cb_kernel(const FpArgs A, int *err) {
     extern __shared__ __align__(16) float smcb[];

@@ -398,7 +398,8 @@ static int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
     if (sc.num_subsets <= 0 || sc.subset_size <= 0) return MBX_ERR_INVALID_ARG;
     if (!(sc.qp.sigma_x > 0.0f) || !(sc.qp.T > 0.0f) || !(sc.qp.p > 0.0f)) return MBX_ERR_INVALID_ARG;
     z.bpp = plan_bp_fast(g, sc.subset_size, g.num_views);
-    z.fpp = plan_fp_cb(g, 0, 0, 2, 128, 0, MBX_BATCHED_FP_CAP);
+    // the channel blocks of either kernel variant (the tuner keeps the faster): the second's are the narrower
+    z.fpp = plan_fp_cb(g, 0, 0, 2, cb_many(g.kind) >= 4 ? CB_MANY_CHANNELS : 128, 0, MBX_BATCHED_FP_CAP);
     if (!z.bpp.ok || !z.fpp.ok) return MBX_ERR_UNSUPPORTED;  // batched path needs the radius-1 kernels
     if ((long long)sc.subset_size * g.num_recon_slices >= (1LL << 31)) return MBX_ERR_UNSUPPORTED;
     if (sc.subset_size > (1 << 24)) return MBX_ERR_UNSUPPORTED;  // list positions share a word with the bin
@@ -751,7 +752,7 @@ static int tune_batched_fp(BatchedPlanHost &P, const Layout &L, const std::vecto
     size_t smem3 = 0, smem3r = 0;
     int ki = 0;
     for (int s = 0; s < num_scans; ++s) {
-        const CbPlan c3 = plan_fp_cb(scans[s].geom, 0, 0, 3, zs[s].fpp.nb, 0, MBX_BATCHED_FP_CAP);
+        const CbPlan c3 = plan_fp_many(scans[s].geom, 0, 0, zs[s].fpp.nb, 0, MBX_BATCHED_FP_CAP);
         if (!c3.ok || c3.nb != zs[s].fpp.nb || c3.cblocks != zs[s].fpp.cblocks) return MBX_OK;  // same work list only
         smem3 = std::max(smem3, c3.walk.smem);
         smem3r = std::max(smem3r, c3.replay.smem);
@@ -764,10 +765,10 @@ static int tune_batched_fp(BatchedPlanHost &P, const Layout &L, const std::vecto
                                          st);
         if (e3 == cudaSuccess) e3 = cudaStreamSynchronize(st);
         if (e3 != cudaSuccess) return set_cuda_error(e3);
-        P.fp_minb = 3;
+        P.fp_minb = cb_many(P.kind);
         P.pl_smem[PL_FP] = smem3;
         P.fp_smem_replay = smem3r;
-        P.pl_grid[PL_FP] = fp_grid(P.kind, 3, smem3, P.pl_total[PL_FP]);
+        P.pl_grid[PL_FP] = fp_grid(P.kind, P.fp_minb, smem3, P.pl_total[PL_FP]);
         return MBX_OK;
     };
     const int cached = autotune_forced() >= 0 ? (autotune_forced() >= 1 ? 3 : 2)
@@ -819,7 +820,8 @@ static int tune_batched_fp_layouts(BatchedPlanHost &P, const Layout &L, const mb
     size_t smem_alt = 0;
     for (int sc = 0; sc < num_scans; ++sc) {
         const CbPlan &c0 = orig[sc * K].plan;
-        const CbPlan q = plan_fp_cb(scans[sc].geom, 0, 0, c0.minb, c0.nb, c0.ppw, MBX_BATCHED_FP_CAP);
+        const CbPlan q = c0.minb > 2 ? plan_fp_many(scans[sc].geom, 0, 0, c0.nb, c0.ppw, MBX_BATCHED_FP_CAP)
+                                     : plan_fp_cb(scans[sc].geom, 0, 0, c0.minb, c0.nb, c0.ppw, MBX_BATCHED_FP_CAP);
         if (!q.ok || q.nb != c0.nb || q.cblocks != c0.cblocks || q.minb != c0.minb) continue;
         can[sc] = 1;
         for (int j = 0; j < K; ++j) alt[sc * K + j].plan = q;
@@ -1210,12 +1212,13 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
             flt_smem = std::max(flt_smem, filter_smem_bytes(scans[s].geom.num_det_channels));
     P.flt_smem = flt_smem;
     // kernel attributes and resident-CTA grids
-    const void *kfp2 = fp_kernel_of(P.kind, 2), *kfp3 = fp_kernel_of(P.kind, 3);
+    const void *kfp2 = fp_kernel_of(P.kind, 2), *kfp3 = fp_kernel_of(P.kind, cb_many(P.kind));
     e = set_max_dynamic_smem(bp_kernel_of(P.kind, false), 100 * 1024);
     if (e == cudaSuccess) e = set_max_dynamic_smem(bp_kernel_of(P.kind, true), 100 * 1024);
     if (e == cudaSuccess) e = set_max_dynamic_smem(kfp2, 200 * 1024);
     if (e == cudaSuccess) e = set_max_dynamic_smem(kfp3, 200 * 1024);
-    for (int mb = 2; mb <= 3 && e == cudaSuccess && L.plan_fp; ++mb) {
+    for (int mb : {2, cb_many(P.kind)}) {
+        if (e != cudaSuccess || !L.plan_fp) break;
         e = set_max_dynamic_smem(fp_kernel_of(P.kind, mb, CB_REPLAY), 200 * 1024);
         if (e == cudaSuccess) e = set_max_dynamic_smem(fp_kernel_of(P.kind, mb, CB_BUILD), 200 * 1024);
     }

@@ -98,7 +98,7 @@ struct BatchedPlanHost {
     int transposed;       // the back projections read transposed copies (PL_HESS: when hess_transposed)
     int hess_transposed;
     size_t flt_smem;
-    int fp_minb;  // b_fp variant of the subset stage: 2 or 3 resident CTAs per SM
+    int fp_minb;  // b_fp variant of the subset stage: 2 or cb_many resident CTAs per SM
     size_t fp_smem_replay;  // shared memory of the replay kernel (the replay layouts of the subset plans)
     int magic;
 };
@@ -172,7 +172,7 @@ __device__ __forceinline__ const A &list_record(const A *recs, const ProjList &L
 }
 
 // The forward-projection stage kernels of one geometry kind: b_fp (walk), b_fp_replay (stored passes) and
-// b_fp_build (store the passes), each compiled for 2 or 3 resident CTAs per SM (minb).  fp_stage_kernel returns
+// b_fp_build (store the passes), each compiled for 2 or cb_many resident CTAs per SM (minb).  fp_stage_kernel returns
 // the kernel of (minb, mode) for occupancy queries and attributes; launch_fp_stage launches it over a work list.
 const void *fp_stage_kernel(int kind, int minb, int mode);
 void launch_fp_stage(int kind, int minb, int mode, int grid, size_t smem, cudaStream_t st, const ProjList &L, int n,
