@@ -6,10 +6,12 @@
 // Per subset, fully on the device, with the step size kept in device memory:
 //   1. dn_delta_kernel: qGGMRF gradient/Hessian (g_p, h_p) per voxel, g_f = -fm e, delta = -(g_f + g_p)/(1 + h_p),
 //      float64 block partials of <g_p, delta>, <h_p, delta^2>, <e, delta>, <delta, delta>
-//   2. dn_alpha_kernel (one warp): fixed-order sums, alpha = clip((fm <e,d> - <g_p,d>) / (fm <d,d> +
-//      <h_p,d^2>/1.1 + eps), eps, 1.5)
-//   3. dn_apply_kernel: image[idx] += alpha delta, e[idx] -= alpha delta, float64 partials of |alpha delta|
-//   4. the l1 partials are summed into stats[1]
+//   2. dn_apply_kernel: every block adds the partials up in the same fixed order and finds alpha = clip((fm <e,d> -
+//      <g_p,d>) / (fm <d,d> + <h_p,d^2>/1.1 + eps), eps, 1.5); image[idx] += alpha delta, e[idx] -= alpha delta,
+//      float64 partials of |alpha delta|, which the last block to finish sums into stats[1]
+// Two launches a subset: a subset of a 128 x 128 x 100 volume (102400 voxels, 400 blocks) is some microseconds of work,
+// so what bounds it is the launches and the latency of a pass: 3 iterations of 16 such subsets take 1.96 ms as a whole
+// call, against 2.22 ms with the step size and the l1 sum in launches of one block of their own.
 // mbx_median_filter3d replaces median_filter3d (denoising.py:414-490): median of the 27 voxels of each 3x3x3
 // neighbourhood with edge replication.
 #include "mbx_common.cuh"
@@ -25,7 +27,8 @@ constexpr int DN_THREADS = 256;
 __global__ void dn_delta_kernel(const float *__restrict__ image, const float *__restrict__ err, int nr, int nc, int ns,
                                 const int32_t *__restrict__ pix, long long num_pixels, float fm_constant,
                                 const QParams q, float *__restrict__ delta, double *__restrict__ partials,
-                                int *errw) {
+                                unsigned *__restrict__ finished, int *errw) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *finished = 0;  // counts the blocks of the apply kernel that follows
     const long long total = num_pixels * ns;
     double pl = 0.0, pq = 0.0, fl = 0.0, fq = 0.0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -53,38 +56,45 @@ __global__ void dn_delta_kernel(const float *__restrict__ image, const float *__
     block_reduce_store_n<4>(v, partials);
 }
 
-// stats: [0] alpha, [1] l1 of the update (written by the l1 sum), [2] alpha numerator, [3] alpha denominator
-__global__ void dn_alpha_kernel(const double *__restrict__ partials, int nblocks, double fm_constant,
-                                float *__restrict__ alpha_out, double *__restrict__ stats) {
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    double s[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
+// The sums of the delta kernel's block partials, one warp per value (lane l adds blocks l, l + 32, ..., then a fixed
+// shuffle tree: the same result in every block), and the step size from them.  All threads of the block; returns alpha.
+// stats (one block passes it): [0] alpha, [2] its numerator, [3] its denominator.
+__device__ __forceinline__ float dn_alpha(const double *__restrict__ partials, int nblocks, double fm_constant,
+                                          double *__restrict__ stats) {
+    __shared__ double sums[4];
+    __shared__ float alpha;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 4) {
         double a = 0.0;
-        for (int b = lane; b < nblocks; b += 32) a += partials[b * 4 + v];
-        s[v] = __shfl_sync(0xffffffffu, warp_sum(a), 0);
+#pragma unroll 4
+        for (int b = lane; b < nblocks; b += 32) a += partials[b * 4 + warp];
+        a = warp_sum(a);
+        if (lane == 0) sums[warp] = a;
     }
-    if (lane == 0) {
-        const double num = fm_constant * s[2] - s[0];
-        const double den = fm_constant * s[3] + s[1] / 1.1 + (double)DN_EPS_F32;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double num = fm_constant * sums[2] - sums[0];
+        const double den = fm_constant * sums[3] + sums[1] / 1.1 + (double)DN_EPS_F32;
         float a = (float)(num / den);
         a = fminf(fmaxf(a, DN_EPS_F32), 1.5f);  // jnp.clip(alpha, eps, 1.5)
         if (num != num || den != den) a = nanf("");
-        *alpha_out = a;
+        alpha = a;
         if (stats) {
             stats[0] = (double)a;
             stats[2] = num;
             stats[3] = den;
         }
     }
+    __syncthreads();
+    return alpha;
 }
 
 __global__ void dn_apply_kernel(float *__restrict__ image, float *__restrict__ err, int ns,
                                 const int32_t *__restrict__ pix, long long num_pixels, int npix_grid,
-                                const float *__restrict__ delta, const float *__restrict__ alpha_ptr,
-                                double *__restrict__ partials) {
-    const float alpha = *alpha_ptr;
+                                const float *__restrict__ delta, const double *__restrict__ sums, int nblocks,
+                                double fm_constant, double *__restrict__ partials, unsigned *__restrict__ finished,
+                                double *__restrict__ stats) {
+    const float alpha = dn_alpha(sums, nblocks, fm_constant, blockIdx.x == 0 ? stats : nullptr);
     const long long total = num_pixels * ns;
     double l1 = 0.0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -100,6 +110,19 @@ __global__ void dn_apply_kernel(float *__restrict__ image, float *__restrict__ e
         l1 += (double)fabsf(d);
     }
     block_reduce_store(l1, partials);
+    if (!stats) return;
+    __shared__ bool last;
+    if (threadIdx.x == 0) {  // the thread that stored the block's partial
+        __threadfence();
+        last = atomicAdd(finished, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    double a = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += 32) a += __ldcg(partials + b);
+    a = warp_sum(a);
+    if (threadIdx.x == 0) stats[1] = a;
 }
 
 // 3x3x3 median with edge replication: the 14th smallest of the 27 values (a partial selection sort).
@@ -137,7 +160,7 @@ __global__ void median3_kernel(const float *__restrict__ x, int d0, int d1, int 
 }
 
 struct DnLayout {
-    size_t delta, partials, l1, alpha, total;
+    size_t delta, partials, l1, finished, total;
     int max_blocks;
 };
 
@@ -151,7 +174,7 @@ static DnLayout dn_layout(long long num_pixels, int ns) {
     off += align256((size_t)L.max_blocks * 4 * sizeof(double));
     L.l1 = off;
     off += align256((size_t)L.max_blocks * sizeof(double));
-    L.alpha = off;
+    L.finished = off;
     off += 256;
     L.total = off;
     return L;
@@ -186,20 +209,18 @@ extern "C" int mbx_qggmrf_denoise_step(float *flat_image, float *flat_error_imag
     float *delta = reinterpret_cast<float *>(base + L.delta);
     double *partials = reinterpret_cast<double *>(base + L.partials);
     double *l1 = reinterpret_cast<double *>(base + L.l1);
-    float *alpha = reinterpret_cast<float *>(base + L.alpha);
+    unsigned *finished = reinterpret_cast<unsigned *>(base + L.finished);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long ncyl = num_pixels * num_slices;
     const unsigned nb = dn_blocks(ncyl, L.max_blocks);
     dn_delta_kernel<<<nb, DN_THREADS, 0, st>>>(flat_image, flat_error_image, num_rows, num_cols, num_slices,
                                                pixel_indices, num_pixels, fm_constant, make_qparams(*qp), delta,
-                                               partials, device_error_ptr());
-    note_launch();
-    dn_alpha_kernel<<<1, 32, 0, st>>>(partials, (int)nb, (double)fm_constant, alpha, stats_out);
+                                               partials, finished, device_error_ptr());
     note_launch();
     dn_apply_kernel<<<nb, DN_THREADS, 0, st>>>(flat_image, flat_error_image, num_slices, pixel_indices, num_pixels,
-                                               num_rows * num_cols, delta, alpha, l1);
+                                               num_rows * num_cols, delta, partials, (int)nb, (double)fm_constant, l1,
+                                               finished, stats_out);
     note_launch();
-    if (stats_out) launch_sum_partials(l1, (int)nb, 1, stats_out + 1, st);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? MBX_OK : set_cuda_error(e);
 }
