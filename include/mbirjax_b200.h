@@ -102,6 +102,11 @@ MBX_API int mbx_get_device_error(int *flags_out);
 /* Number of kernel launches this library has submitted since it was loaded (host-side count, all devices and
  * streams; launches replayed from a captured CUDA graph are not re-counted). */
 MBX_API uint64_t mbx_launch_count(void);
+/* Host only: shuffles n items of item_bytes (4 or 8; x may be NULL when n <= 1) the way a legacy numpy RandomState
+ * does: i = n-1..1, j a masked-rejection draw from [0, i], swap x[i] and x[j].  key (624 words) and pos are the
+ * generator's MT19937 state and are advanced.  Lets the per-scan draws of a batch run on several host threads at once
+ * (numpy's own shuffles hold the interpreter lock). */
+MBX_API int mbx_mt19937_shuffle(uint32_t *key, int32_t *pos, void *x, int64_t n, int32_t item_bytes);
 /* Autotuning of the forward projector's plans (no counterpart in the reference, whose XLA compiler picks its own
  * schedule; the back projector has one plan per call shape).  The first mbx_sparse_forward_project of a call shape
  * (geometry sizes, views, pixel count rounded up to a power of two) times its candidate plans on the caller's stream,

@@ -60,6 +60,7 @@ _SIGNATURES = {
     'mbx_last_cuda_error': (ctypes.c_int, []),
     'mbx_get_device_error': (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
     'mbx_launch_count': (ctypes.c_uint64, []),
+    'mbx_mt19937_shuffle': (c_int32, [c_void_p, ctypes.POINTER(c_int32), c_void_p, ctypes.c_int64, c_int32]),
     'mbx_set_autotune': (ctypes.c_int, [ctypes.c_int]),
     'mbx_forward_project_workspace_bytes': (c_size_t, [ctypes.POINTER(MbxGeom), c_int64, c_int32]),
     'mbx_sparse_forward_project': (ctypes.c_int, [ctypes.POINTER(MbxGeom), c_void_p, c_void_p, c_int64, c_void_p,

@@ -19,6 +19,7 @@ radius 1, and use a single partition with the same number of subsets (``granular
 has no direct recon for that geometry).
 """
 import collections
+import ctypes
 import warnings
 
 import numpy as np
@@ -62,6 +63,36 @@ def release_batched_sessions():
     """Free the device state (buffers, plans, graphs) kept for the batch shapes reconstructed so far."""
     while _SESSIONS:
         _SESSIONS.popitem(last=False)[1].close()
+
+
+class _SeededStream:
+    """The draws of np.random.RandomState(seed) that a scan makes, shuffled by the library without the interpreter
+    lock: permutation, shuffle and choice without replacement of 1-D arrays of 4- or 8-byte items.
+
+    A batch of six scans (about 80 000 pixels each) makes 24 shuffles; numpy's hold the lock, so that the scans'
+    threads take turns and the host part outlasts the set-up graph it runs beside (34 ms against 27)."""
+
+    def __init__(self, seed):
+        _, key, pos, self._has_gauss, self._gauss = np.random.RandomState(int(seed)).get_state()
+        self._key, self._pos = np.array(key, dtype=np.uint32), ctypes.c_int32(int(pos))
+        self._call = _capi.load_library().mbx_mt19937_shuffle
+
+    def shuffle(self, x):
+        assert x.ndim == 1 and x.flags.c_contiguous
+        _capi._check(self._call(self._key.ctypes.data, ctypes.byref(self._pos), x.ctypes.data, len(x), x.itemsize),
+                     'mbx_mt19937_shuffle')
+
+    def permutation(self, x):
+        x = np.arange(x) if np.ndim(x) == 0 else np.array(x)
+        self.shuffle(x)
+        return x
+
+    def choice(self, a, size, replace):
+        assert not replace and size <= len(a)
+        return a[self.permutation(len(a))[:size]]
+
+    def get_state(self):
+        return 'MT19937', self._key, self._pos.value, self._has_gauss, self._gauss
 
 
 class BatchedVCD:
@@ -118,9 +149,9 @@ class BatchedVCD:
     def _host_draws(self, max_iterations, small, small_w):
         """The host part of every scan (see _scan_draws).  With per-scan seeds each scan draws from its own
         RandomState, which is the stream np.random.seed(seed) gives, so the scans run on a pool of host threads
-        and the global stream is left where the plain path leaves it, after the last scan's draws.  (The legacy
-        shuffles, most of this time, hold the GIL, so the threads overlap only the sorts and array work; the
-        whole host part runs while the set-up graph runs on the device.)  Without seeds the scans draw from the
+        and the global stream is left where the plain path leaves it, after the last scan's draws.  (The shuffles, most
+        of this time, run without the interpreter lock; the whole host part runs while the set-up graph runs on
+        the device.)  Without seeds the scans draw from the
         global stream one after another.
         Returns (regularisation dicts, partitions, schedule (steps, scans), fm constants, qGGMRF records, sigmas)."""
         n = len(self.models)
@@ -130,7 +161,7 @@ class BatchedVCD:
         if self.seeds is None:
             out = [self._scan_draws(i, max_iterations, small, small_w, None) for i in range(n)]
         else:
-            rngs = [np.random.RandomState(int(sd)) for sd in self.seeds]
+            rngs = [_SeededStream(sd) for sd in self.seeds]
             out = list(_draw_pool().map(
                 lambda i: self._scan_draws(i, max_iterations, small, small_w, rngs[i]), range(n)))
             np.random.set_state(rngs[-1].get_state())

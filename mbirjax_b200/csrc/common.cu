@@ -173,6 +173,67 @@ extern "C" const char *mbx_error_string(int code) {
 
 extern "C" int mbx_last_cuda_error(void) { return mbx::t_last_cuda_error; }
 
+namespace {
+
+// MT19937 (Matsumoto and Nishimura, 1998): 624 words of state, the recurrence of their paper and its tempering.
+struct Mt19937 {
+    uint32_t *key;
+    int pos;
+    void refill() {
+        constexpr int N = 624, M = 397;
+        auto twist = [](uint32_t hi, uint32_t lo) {
+            const uint32_t y = (hi & 0x80000000u) | (lo & 0x7fffffffu);
+            return (y >> 1) ^ ((0u - (lo & 1u)) & 0x9908b0dfu);
+        };
+        for (int i = 0; i < N - M; ++i) key[i] = key[i + M] ^ twist(key[i], key[i + 1]);
+        for (int i = N - M; i < N - 1; ++i) key[i] = key[i + M - N] ^ twist(key[i], key[i + 1]);
+        key[N - 1] = key[M - 1] ^ twist(key[N - 1], key[0]);
+        pos = 0;
+    }
+    uint32_t next() {
+        if (pos >= 624) refill();
+        uint32_t y = key[pos++];
+        y ^= y >> 11;
+        y ^= (y << 7) & 0x9d2c5680u;
+        y ^= (y << 15) & 0xefc60000u;
+        return y ^ (y >> 18);
+    }
+};
+
+template <typename T>
+void shuffle_items(Mt19937 &mt, T *x, int64_t n) {
+    uint32_t mask = 0;
+    for (int64_t i = n - 1; i > 0;) {
+        // all i of one bit length share the mask
+        mask = 0xffffffffu >> __builtin_clz((uint32_t)i);
+        const int64_t stop = (int64_t)(mask >> 1);
+        for (; i > stop; --i) {
+            uint32_t j;
+            do {
+                j = mt.next() & mask;
+            } while (j > (uint32_t)i);
+            const T t = x[i];
+            x[i] = x[j];
+            x[j] = t;
+        }
+    }
+}
+
+}  // namespace
+
+extern "C" int mbx_mt19937_shuffle(uint32_t *key, int32_t *pos, void *x, int64_t n, int32_t item_bytes) {
+    if (!key || !pos || *pos < 0 || *pos > 624 || n < 0 || n > (1LL << 31) - 1 || (n > 1 && !x) ||
+        (item_bytes != 4 && item_bytes != 8))
+        return MBX_ERR_INVALID_ARG;
+    Mt19937 mt{key, *pos};
+    if (item_bytes == 4)
+        shuffle_items(mt, static_cast<uint32_t *>(x), n);
+    else
+        shuffle_items(mt, static_cast<uint64_t *>(x), n);
+    *pos = mt.pos;
+    return MBX_OK;
+}
+
 extern "C" uint64_t mbx_launch_count(void) { return mbx::g_launches.load(std::memory_order_relaxed); }
 
 extern "C" int mbx_set_autotune(int mode) {

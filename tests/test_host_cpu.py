@@ -398,3 +398,21 @@ def test_batched_host_draws_on_threads_match_the_sequential_stream():
         np.testing.assert_array_equal(sched.reshape(4, 4, len(models))[:, :, i], order)
         assert fms[i] == pytest.approx(1.0 / reg['sigma_y'] ** 2)
     np.testing.assert_array_equal(np.random.get_state()[1], end_state)
+
+
+@pytest.mark.parametrize('seed', [0, 7, 2 ** 32 - 1])
+def test_seeded_stream_draws_what_randomstate_draws(seed):
+    """The library's shuffles against numpy's legacy ones, draw after draw: sizes around the powers of two where the
+    rejection mask changes and over the generator's refills, both item sizes, and the state that is left."""
+    from mbirjax_b200.batched import _SeededStream
+    want, got = np.random.RandomState(seed), _SeededStream(seed)
+    for n in (0, 1, 2, 3, 4, 5, 7, 8, 9, 623, 624, 625, 1023, 1024, 1025, 70001):
+        x = np.arange(n, dtype=np.int32)[::-1]
+        np.testing.assert_array_equal(got.permutation(x), want.permutation(x))
+        np.testing.assert_array_equal(got.permutation(n), want.permutation(n))
+        if n:
+            np.testing.assert_array_equal(got.choice(x, n // 3, replace=False), want.choice(x, n // 3, replace=False))
+    a, b = got.get_state(), want.get_state()
+    assert a[0] == b[0] and a[2:] == b[2:]
+    np.testing.assert_array_equal(a[1], b[1])
+    assert not x.flags.writeable or x[0] == 70000  # the inputs of permutation stay as they were
