@@ -305,7 +305,11 @@ class _Session:
             self.flat.append(torch.empty((nr * nc, ns), dtype=torch.float32, device=dev))
             self.hess.append(torch.empty((nr * nc, ns), dtype=torch.float32, device=dev))
             self.part.append(torch.as_tensor(np.ascontiguousarray(parts[i], dtype=np.int32), device=dev))
+            # in Z-order, like the subsets: whole chunks of the list miss a channel block, and the windows of the
+            # back projector's pixel groups are compact (with the 4-CTA forward variant,
+            # six scans: set-up graph 26.9 -> 21.7 ms)
             full = gen_full_indices_no_draw(self.recon_shapes[i], model.use_ror_mask)
+            full = morton_sorted_partition(full[None], nc)[0]
             self.full.append(torch.as_tensor(full, dtype=torch.int32, device=dev))
             rec = _scan_record(g, self.flat[i], self.err[i], self.w[i], self.hess[i], self.part[i], fms[i], qps[i])
             rec.sinogram = self.y[i].data_ptr()

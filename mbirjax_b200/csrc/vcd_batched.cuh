@@ -98,6 +98,7 @@ struct BatchedPlanHost {
     int transposed;       // the back projections read transposed copies (PL_HESS: when hess_transposed)
     int hess_transposed;
     size_t flt_smem;
+    int init_minb;  // b_fp variant of the initial projection: cb_many for parallel beam, else 2
     int fp_minb;  // b_fp variant of the subset stage: 2 or cb_many resident CTAs per SM
     size_t fp_smem_replay;  // shared memory of the replay kernel (the replay layouts of the subset plans)
     int magic;
