@@ -990,8 +990,9 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     int *hoff = reinterpret_cast<int *>(host.data() + L.offs);
     int *hbox_first = reinterpret_cast<int *>(host.data() + L.box_first);
     int *o_el = hoff, *o_sn = hoff + n1, *o_rc = hoff + 2 * n1, *o_flt = hoff + 3 * n1, *o_tr = hoff + 4 * n1;
-    // one tensor map per scan serves all its back projections: the window's rows depend on the geometry alone
-    bool transposed = L.transposed;
+    // one tensor map per scan serves all its back projections: the window's rows depend on the geometry alone; the TMA
+    // reads maps from 64-byte boundaries only, so in a workspace that starts off one the windows are copied by loads
+    bool transposed = L.transposed && (reinterpret_cast<uintptr_t>(base + L.maps) & 63) == 0;
     for (int s = 0; s < n && transposed; ++s) {
         CUtensorMap map = {};
         transposed = bpf_window_map(map, reinterpret_cast<const float *>(base + L.buf_off[4 * s + 3]), scans[s].geom,

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 import torch
 
+import mbirjax_b200 as mb
 import oracle as O
 from mbirjax_b200 import _capi
 from mbirjax_b200.vcd_utils import gen_full_indices, gen_pixel_partition, morton_sorted_partition
@@ -108,3 +109,35 @@ def test_workspace_off_a_16_byte_boundary(cuda):
     assert rc == 0
     torch.cuda.synchronize()
     assert rel_l2(out.cpu().numpy(), ref.cpu().numpy()) <= 1e-6
+
+
+def test_batched_workspace_off_the_tensor_map_boundary(cuda, monkeypatch):
+    """A batch whose workspace starts 16 bytes past a 64-byte boundary copies its windows by plain loads (the same sums
+    in the same order), and reconstructs what the aligned one does."""
+    from mbirjax_b200 import _capi, batched as B
+
+    class Shifted:
+        def __getattr__(self, name):
+            return getattr(torch, name)
+
+        def empty(self, *size, **kw):
+            if kw.get('dtype') is torch.uint8:
+                return torch.empty(size[0] + 64, **kw)[16:16 + size[0]]
+            return torch.empty(*size, **kw)
+
+    models, sinos = [], []
+    for v, r, c in ((40, 12, 64), (30, 8, 50)):
+        m = mb.ParallelBeamModel((v, r, c), np.linspace(0, np.pi, v, endpoint=False).astype(np.float32))
+        m.set_params(sharpness=0.0, granularity=[4], partition_sequence=[0], verbose=0)
+        models.append(m)
+        sinos.append(np.random.default_rng(v).random((v, r, c)).astype(np.float32))
+    out = []
+    for shift in (False, True):
+        B.release_batched_sessions()
+        if shift:
+            monkeypatch.setattr(_capi, 'torch', Shifted())
+        recons, _ = B.BatchedVCD(models, sinos, seeds=[1, 2]).recon(max_iterations=2)
+        out.append([x.cpu().numpy() for x in recons])
+    B.release_batched_sessions()
+    for a, b in zip(*out):
+        assert rel_l2(b, a) <= 1e-5
