@@ -22,6 +22,7 @@
 
 #include "back_project.cuh"
 #include "bp_fast.cuh"
+#include "bp_gather.cuh"
 
 namespace mbx {
 
@@ -56,14 +57,38 @@ bool bpf_window_map(CUtensorMap &map, const float *copy, const mbx_geom &g, int 
 
 size_t bp_workspace_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
     const BpfPlan fp = plan_bp_fast(g, num_pixels, num_views_sel);
-    if (fp.ok)
-        return fp.workspace + (bp_transposes(g, num_pixels, num_views_sel) ? bpf_transposed_bytes(g, num_views_sel) : 0);
-    return plan_bp(g, num_pixels, num_views_sel).workspace;
+    if (!fp.ok) return plan_bp(g, num_pixels, num_views_sel).workspace;
+    if (bp_gathers(g, num_pixels, true))  // with values; without any, windows and no transposed copy
+        return std::max(fp.workspace, plan_bp_gather(g, num_pixels, num_views_sel).workspace);
+    return fp.workspace + (bp_transposes(g, num_pixels, num_views_sel) ? bpf_transposed_bytes(g, num_views_sel) : 0);
 }
 
 size_t bp_noalloc_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
     const BpfPlan fp = plan_bp_fast(g, num_pixels, num_views_sel, 1);
-    return fp.ok ? fp.workspace : plan_bp(g, num_pixels, num_views_sel).workspace;
+    if (!fp.ok) return plan_bp(g, num_pixels, num_views_sel).workspace;
+    return bp_gathers(g, num_pixels, true)
+               ? std::max(fp.workspace, plan_bp_gather(g, num_pixels, num_views_sel).workspace)
+               : fp.workspace;
+}
+
+static int back_project_gather(const mbx_geom &g, const float *sino, const float *w, const int32_t *pix,
+                               long long num_pixels, const int32_t *views, int num_views_sel, int coeff_power,
+                               float scale, float *out, void *ws, size_t ws_bytes, cudaStream_t st) {
+    const BpgPlan pl = plan_bp_gather(g, num_pixels, num_views_sel);
+    if (pl.workspace > 0 && (ws == nullptr || ws_bytes < pl.workspace)) return MBX_ERR_WORKSPACE;
+    const long long stride = num_pixels * (long long)g.num_recon_slices;
+    const bool split = pl.splits > 1;
+    float *dst = split ? static_cast<float *>(ws) : out;
+    const BpgArgs A = {g,     sino, w,   pix, views, num_pixels, num_views_sel, coeff_power,
+                       scale, dst,  split ? stride : 0, pl};
+    bp_gather_kernel<<<dim3((unsigned)pl.gx, (unsigned)pl.gy, (unsigned)pl.splits), 256, 0, st>>>(A, device_error_ptr());
+    note_launch();
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && split) {
+        launch_split_sum(dst, stride, pl.splits, scale, out, stride, st);
+        e = cudaGetLastError();
+    }
+    return e == cudaSuccess ? MBX_OK : set_cuda_error(e);
 }
 
 __global__ void __launch_bounds__(256) bp_transpose_kernel(const float *__restrict__ src, const float *__restrict__ wts,
@@ -73,8 +98,10 @@ __global__ void __launch_bounds__(256) bp_transpose_kernel(const float *__restri
     const int j = first + blockIdx.y;
     const int vi = views ? views[j] : j;
     if (vi < 0 || vi >= num_views) return;  // flagged and skipped by the projection
+    const int rows = 32 * ceil_div(ceil_div(rp, 32), (int)gridDim.z);  // per block: 32, in all but absurdly tall views
     bpf_transpose_block(src, wts, dst, (long long)vi * num_rows * num_channels,
-                        (long long)j * (num_channels + 2 * BPF_EDGE) * rp, blockIdx.x * 32, num_rows, num_channels, rp);
+                        (long long)j * (num_channels + 2 * BPF_EDGE) * rp, blockIdx.x * 32, blockIdx.z * rows,
+                        min(rp, ((int)blockIdx.z + 1) * rows), num_rows, num_channels, rp);
 }
 
 template <int KIND, bool TR>
@@ -125,6 +152,9 @@ int back_project(const mbx_geom &g, const float *sino, const float *w, const int
         A.g = g;
     }
     A.plan = plan_bp_fast(g, num_pixels, num_views_sel, noalloc);
+    if (A.plan.ok && bp_gathers(g, num_pixels, sino != nullptr))
+        return back_project_gather(g, sino, w, pix, num_pixels, views, num_views_sel, coeff_power, scale, out, ws,
+                                   ws_bytes, st);
     if (A.plan.ok) {
         bool tr = !noalloc && sino && bp_transposes(g, num_pixels, num_views_sel);
         const size_t need = A.plan.workspace + (tr ? bpf_transposed_bytes(g, num_views_sel) : 0);
@@ -146,7 +176,8 @@ int back_project(const mbx_geom &g, const float *sino, const float *w, const int
             const int32_t *tv = A.tsino_all ? nullptr : views;
             // views in grid.y, at most 65535 per launch
             for (int j0 = 0; j0 < nt && e == cudaSuccess; j0 += 65535) {
-                bp_transpose_kernel<<<dim3((unsigned)ceil_div(g.num_det_channels + 2 * BPF_EDGE, 32), (unsigned)std::min(nt - j0, 65535)),
+                bp_transpose_kernel<<<dim3((unsigned)ceil_div(g.num_det_channels + 2 * BPF_EDGE, 32), (unsigned)std::min(nt - j0, 65535),
+                                           (unsigned)std::min((long long)ceil_div(A.rp, 32), 65535LL)),
                                       256, 0, st>>>(sino, w, tv, g.num_views, j0, copy, g.num_det_rows,
                                                     g.num_det_channels, A.rp);
                 note_launch();

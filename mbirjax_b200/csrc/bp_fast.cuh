@@ -936,13 +936,15 @@ inline size_t bpf_transposed_bytes(const mbx_geom &g, int num_views_sel) {
 bool bpf_window_map(CUtensorMap &map, const float *copy, const mbx_geom &g, int num_views_sel, int boxq);
 
 // Channels c0 .. c0 + 31 (counted with the edge channels) of one view of the transposed copy, by a block of 256 threads:
-// weights x values of src (view offset soff, num_rows x num_channels) to dst (view offset doff).
+// weights x values of src (view offset soff, num_rows x num_channels), rows r_begin (a multiple of 32) .. r_end - 1, to
+// dst (view offset doff).  A plain call gives each 32 rows a block of their own (views of 128 rows: a quarter of the
+// serial steps).
 __device__ __forceinline__ void bpf_transpose_block(const float *__restrict__ src, const float *__restrict__ wts,
                                                     float *__restrict__ dst, long long soff, long long doff, int c0,
-                                                    int num_rows, int num_channels, int rp) {
+                                                    int r_begin, int r_end, int num_rows, int num_channels, int rp) {
     __shared__ float tile[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-    for (int r0 = 0; r0 < rp; r0 += 32) {
+    for (int r0 = r_begin; r0 < r_end; r0 += 32) {
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
@@ -975,6 +977,10 @@ inline int bpf_tile_height(int S, int most) {
 // allocates nothing), or twice the sinogram unless `small`.
 constexpr size_t BPF_PARTIAL_BYTES = MBX_NOALLOC_SCRATCH_BYTES / 4 * 3;
 
+// Fewest views per split: a warp's views follow one another, so a small call takes as long as one warp's views
+// (24 x 20 x 64 cone, subset of 4: 30 us with 8, 20 with 4, 14 with 2).
+constexpr int BPF_SPLIT_VIEWS = 2;
+
 inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_views_sel, int small = 0) {
     BpfPlan pl;
     pl.inline_fp = 1;
@@ -1001,6 +1007,15 @@ inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_vie
         while (most > 4 && most * slope + 4 > BPF_CACHE_ROWS) most -= 4;
         if (bpf_tile_height(S, most) * slope + 4 > BPF_CACHE_ROWS) pl.ok = false;
     }
+    const long long slots = (long long)bpf_min_blocks(g.kind) * BPF_LAUNCH_WARPS * num_sms() / BPF_WARPS;
+    // translation: a pixel's magnification follows its row, so the footprints of a warp spread over more channels and
+    // rows than a low tile's windows have (all pixels of 49 x 128 x 128: 121 us with 32 slices, 130 with 16, 105 with 12,
+    // 132 with 8; subset of 4 of 49 x 85 x 96: 60, 46 and 41 us)
+    if (g.kind == MBX_GEOM_TRANSLATION) most = std::min(most, 12);
+    // cone: tiles of half the height for calls whose units could not fill the chip (101 x 18 x 51, subset of 4: 20 -> 16)
+    if (g.kind == MBX_GEOM_CONE && (num_pixels + 31) / 32 * ceil_div(S, most) *
+                                           std::max(1, num_views_sel / BPF_SPLIT_VIEWS) < BPF_WARPS * slots)
+        most = std::min(most, BPF_ST / 2);
     pl.ts = bpf_tile_height(S, most);
     pl.tiles = ceil_div(S, pl.ts);
     // rows of a window: the tile's (parallel); its rows at the steepest slope, their rounding and some spread (fan)
@@ -1019,10 +1034,9 @@ inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_vie
     // views split over CTAs when there are few: the fewest splits (partial sums cost memory traffic) whose last wave
     // is full enough, as the time of a call is about waves / splits
     const long long base = (long long)pl.gx * pl.gy;
-    const long long slots = (long long)bpf_min_blocks(g.kind) * BPF_LAUNCH_WARPS * num_sms() / BPF_WARPS;
     long long splits = 1;
     if (base < 2 * slots && num_views_sel >= 16) {
-        long long maxs = num_views_sel / 8;
+        long long maxs = num_views_sel / BPF_SPLIT_VIEWS;
         if (maxs > 64) maxs = 64;
         size_t most_bytes = BPF_PARTIAL_BYTES;
         if (!small) most_bytes = std::max(most_bytes, (size_t)g.num_views * g.num_det_rows * g.num_det_channels * 8);

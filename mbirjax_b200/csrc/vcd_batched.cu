@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) b_transpose(BatchedTables T, int num_scan
         const int v = local / blocks;
         bpf_transpose_block(mode == 2 ? sc.wts : sc.err, mode == 0 ? sc.wts : nullptr, sc.tsino,
                             (long long)v * sc.R * sc.C, (long long)v * (sc.C + 2 * BPF_EDGE) * sc.rp,
-                            (local - v * blocks) * 32, sc.R, sc.C, sc.rp);
+                            (local - v * blocks) * 32, 0, sc.rp, sc.R, sc.C, sc.rp);
     }
 }
 
