@@ -45,11 +45,13 @@ struct FiltShape {
     int taps;     // padded doubles of one tap table
 };
 
-__host__ __device__ inline FiltShape filter_shape(int C) {
+// groups: fewer groups of rows per block than the default (0), for calls of few rows.
+__host__ __device__ inline FiltShape filter_shape(int C, int groups = 0) {
     FiltShape f;
     f.outs = (C + 1) / 2;
     f.tiles = (f.outs + 63) / 64;
     f.groups = f.tiles >= 3 ? 1 : (f.tiles == 2 ? 2 : 4);
+    if (groups > 0 && groups < f.groups) f.groups = groups;
     f.rows = 16 * f.groups;
     f.kc = 2048 / f.rows;
     f.kp = (f.outs + f.kc - 1) / f.kc * f.kc;
@@ -58,8 +60,8 @@ __host__ __device__ inline FiltShape filter_shape(int C) {
     return f;
 }
 
-inline size_t filter_smem_bytes(int C) {
-    const FiltShape f = filter_shape(C);
+inline size_t filter_smem_bytes(int C, int groups = 0) {
+    const FiltShape f = filter_shape(C, groups);
     return sizeof(double) * (2 * (size_t)f.kc * f.pitch + 2 * (size_t)f.taps);
 }
 
@@ -73,13 +75,14 @@ inline size_t filter_smem_bytes(int C) {
 // one place, so a sample costs one tap load, two 16-byte loads of 4 rows (staged as float64, [sample][row]) and 32 FMAs,
 // and the loop is bound by the float64 pipe (half the float32 rate).  The tap tables (one per parity) are padded to 9
 // doubles per 8 taps, which keeps the lanes' loads, 8 taps apart, in different banks.  Measured on 360 x 256 x 512 (FDK):
-// 5.53 -> 1.51 ms against one output and 8 rows per thread, whose samples were converted to float64 at every use.
+// 5.53 -> 1.59 ms against one output and 8 rows per thread, whose samples were converted to float64 at every use.
 __device__ __forceinline__ void direct_filter_rows(const float *__restrict__ sino, float *__restrict__ out,
                                                    long long row0, long long num_rows_total, int R, int C,
                                                    double filter_scale, double out_scale, int fdk, double D,
                                                    double delta_det_channel, double delta_det_row,
-                                                   double det_channel_offset, double det_row_offset, double *sm) {
-    const FiltShape f = filter_shape(C);
+                                                   double det_channel_offset, double det_row_offset, double *sm,
+                                                   int groups = 0) {
+    const FiltShape f = filter_shape(C, groups);
     double *xs = sm;                              // [2][kc][pitch]: staged samples by parity
     double *taps = sm + 2 * f.kc * f.pitch;       // [2][f.taps]
     float *ot = reinterpret_cast<float *>(sm);    // finished outputs, [rows][128 * tiles of a pass] (after the last sample)
@@ -111,8 +114,9 @@ __device__ __forceinline__ void direct_filter_rows(const float *__restrict__ sin
             for (int r = 0; r < 4; ++r) acc[u][r] = 0.0;
         for (int k0 = 0; k0 < f.kp; k0 += f.kc) {
             __syncthreads();  // the last samples (and, at the start of a pass, its predecessor's outputs) are read
-            for (int t = tid; t < 2 * f.kc * f.rows; t += FILT_THREADS) {
-                const int rr = t / (2 * f.kc), cc = t - rr * 2 * f.kc, j = 2 * k0 + cc;
+            const int kn = min(f.kc, (f.outs - k0 + 7) & ~7);  // samples of the chunk, in eights
+            for (int t = tid; t < 2 * kn * f.rows; t += FILT_THREADS) {
+                const int rr = t / (2 * kn), cc = t - rr * 2 * kn, j = 2 * k0 + cc;
                 double v = 0.0;
                 if (rr < nrows && j < C) {
                     const long long row = row0 + rr;
@@ -131,7 +135,7 @@ __device__ __forceinline__ void direct_filter_rows(const float *__restrict__ sin
 #pragma unroll
                 for (int u = 1; u < 8; ++u) g[u] = tap[9 + u - 1];
             }
-            if (o0 >= k0 && o0 < k0 + f.kc) {  // the centre tap
+            if (o0 >= k0 && o0 < k0 + kn) {  // the centre tap
                 const double h0 = 0.25 * filter_scale;
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
@@ -144,7 +148,7 @@ __device__ __forceinline__ void direct_filter_rows(const float *__restrict__ sin
                 }
             }
             const double *x = xrow;
-            for (int k = 0; k < f.kc; k += 8) {
+            for (int k = 0; k < kn; k += 8) {
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {  // tap of output u at sample k + s: g[(u - s) & 7]
                     g[(8 - s) & 7] = tap[7 - s];
