@@ -28,7 +28,6 @@
 #include <cstring>
 #include <vector>
 
-#include "direct_filter.cuh"
 #include "vcd_batched.cuh"
 
 namespace mbx {
@@ -378,68 +377,6 @@ __global__ void __launch_bounds__(CB_CHUNK) b_chunk_bounds(BatchedTables T, int 
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-struct ScanSizes {
-    long long ncyl, nsino, nrecon, npix;
-    int el_tiles, sn_tiles, rc_tiles, flt_tiles;
-    BpfPlan bpp;  // subset back projection
-    CbPlan fpp;   // subset forward projection
-    CbPlan ifp;   // initial forward projection, on the same channel blocks
-    BpfPlan ibp;  // initial back projection over the region of reconstruction
-    BpfPlan hbp;  // Hessian back projection over every pixel
-    int hbp_slices;  // > 0: hbp is planned on one slice and broadcast to this many (unit-weight parallel beam)
-    bool setup;   // the scan carries the set-up inputs
-    int tr_tiles; // 32-channel blocks of the transposed copy over all views
-};
-
-static int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
-    const mbx_geom &g = sc.geom;
-    int rc = validate_geom(&g);
-    if (rc != MBX_OK) return rc;
-    if (!sc.flat_recon || !sc.error_sinogram || !sc.fm_hessian || !sc.partition) return MBX_ERR_INVALID_ARG;
-    if (sc.num_subsets <= 0 || sc.subset_size <= 0) return MBX_ERR_INVALID_ARG;
-    if (!(sc.qp.sigma_x > 0.0f) || !(sc.qp.T > 0.0f) || !(sc.qp.p > 0.0f)) return MBX_ERR_INVALID_ARG;
-    z.bpp = plan_bp_fast(g, sc.subset_size, g.num_views);
-    // the channel blocks of either kernel variant (the tuner keeps the faster): the second's are the narrower
-    z.fpp = plan_fp_cb(g, 0, 0, 2, cb_many(g.kind) >= 4 ? CB_MANY_CHANNELS : 128, 0, MBX_BATCHED_FP_CAP);
-    z.ifp = z.fpp;
-    if (!z.bpp.ok || !z.fpp.ok) return MBX_ERR_UNSUPPORTED;  // batched path needs the radius-1 kernels
-    if ((long long)sc.subset_size * g.num_recon_slices >= (1LL << 31)) return MBX_ERR_UNSUPPORTED;
-    if (sc.subset_size > (1 << 24)) return MBX_ERR_UNSUPPORTED;  // list positions share a word with the bin
-    z.ncyl = (long long)sc.subset_size * g.num_recon_slices;
-    z.nsino = (long long)g.num_views * g.num_det_rows * g.num_det_channels;
-    z.npix = (long long)g.num_recon_rows * g.num_recon_cols;
-    z.nrecon = z.npix * g.num_recon_slices;
-    z.el_tiles = (int)((z.ncyl + BT_ELEM_TILE - 1) / BT_ELEM_TILE);
-    z.sn_tiles = (int)((z.nsino + BT_SINO_TILE - 1) / BT_SINO_TILE);
-    z.rc_tiles = (int)((z.nrecon + BT_SINO_TILE - 1) / BT_SINO_TILE);
-    z.tr_tiles = g.num_views * ceil_div(g.num_det_channels + 2 * BPF_EDGE, 32);
-    z.setup = sc.sinogram != nullptr || sc.full_indices != nullptr || sc.num_full_indices != 0;
-    z.flt_tiles = 0;
-    if (z.setup) {
-        if (!sc.sinogram || !sc.full_indices || sc.num_full_indices <= 0 || sc.num_full_indices > z.npix)
-            return MBX_ERR_INVALID_ARG;
-        // the initial forward projection reads voxels by pixel index, which shares a word with the bin
-        if (z.npix > (1 << 24) || z.nrecon >= (1LL << 31)) return MBX_ERR_UNSUPPORTED;
-        z.hbp_slices = 0;
-        if (bp_unit_broadcast(g, nullptr, sc.weights)) {  // unit-weight parallel Hessian: one slice, broadcast
-            z.hbp = plan_bp_fast(one_slice_geometry(g), z.npix, g.num_views);
-            if (z.hbp.ok && z.hbp.splits == 1) z.hbp_slices = g.num_recon_slices;
-        }
-        if (z.hbp_slices == 0) z.hbp = plan_bp_fast(g, z.npix, g.num_views);
-        if (!z.hbp.ok) return MBX_ERR_UNSUPPORTED;
-        if (g.kind != MBX_GEOM_TRANSLATION) {  // translation geometry starts from zeros (no direct recon)
-            if (!filter_admits(g.num_det_channels, g.kind != MBX_GEOM_PARALLEL))
-                return MBX_ERR_UNSUPPORTED;
-            z.ibp = plan_bp_fast(g, sc.num_full_indices, g.num_views);
-            if (!z.ibp.ok) return MBX_ERR_UNSUPPORTED;
-            z.flt_tiles = ceil_div((long long)g.num_views * g.num_det_rows, filter_shape(g.num_det_channels).rows);
-        } else {
-            z.ibp = z.hbp;  // unused
-        }
-    }
-    return MBX_OK;
-}
-
 // Tiles of scan s in a projection work list, the list's per-scan dimension (gx or channel blocks) and the cost
 // of one of its tiles (to order the list: most expensive tiles first).
 static void list_dims(int which, const mbx_scan &sc, const ScanSizes &z, int &tiles, int &dim, double &cost,
@@ -586,7 +523,7 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
     L.pl_dim = take(sizeof(int) * PL_COUNT * n);
     L.pl_order = take(sizeof(int) * PL_COUNT * n);
     L.offs = take(sizeof(int) * 5 * (n + 1));
-    L.maps = take(sizeof(CUtensorMap) * n);
+    L.maps = take(sizeof(CUtensorMap) * SW_COUNT * n);
     L.box_first = take(sizeof(int) * (L.ksum + 1));
     L.counters = take(sizeof(int) * PL_COUNT);
     L.sched = take(sizeof(int) * (size_t)num_steps * n);  // the host-built tables end here
@@ -990,14 +927,16 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     int *hoff = reinterpret_cast<int *>(host.data() + L.offs);
     int *hbox_first = reinterpret_cast<int *>(host.data() + L.box_first);
     int *o_el = hoff, *o_sn = hoff + n1, *o_rc = hoff + 2 * n1, *o_flt = hoff + 3 * n1, *o_tr = hoff + 4 * n1;
-    // one tensor map per scan serves all its back projections: the window's rows depend on the geometry alone; the TMA
-    // reads maps from 64-byte boundaries only, so in a workspace that starts off one the windows are copied by loads
+    // the tensor maps of every scan's back projections; the TMA reads maps from 64-byte boundaries only, so in a
+    // workspace that starts off one the windows are copied by loads
     bool transposed = L.transposed && (reinterpret_cast<uintptr_t>(base + L.maps) & 63) == 0;
-    for (int s = 0; s < n && transposed; ++s) {
+    for (int m = 0; m < SW_COUNT * n && transposed; ++m) {
+        const int s = m / SW_COUNT, boxq = scan_window_box(zs[s], m % SW_COUNT);
+        if (boxq == 0) continue;
         CUtensorMap map = {};
         transposed = bpf_window_map(map, reinterpret_cast<const float *>(base + L.buf_off[4 * s + 3]), scans[s].geom,
-                                    scans[s].geom.num_views, zs[s].bpp.boxq);
-        std::memcpy(host.data() + L.maps + sizeof(map) * s, &map, sizeof(map));
+                                    scans[s].geom.num_views, boxq);
+        std::memcpy(host.data() + L.maps + sizeof(map) * m, &map, sizeof(map));
     }
     const bool hess_transposed = transposed && L.hess_transposed;
     fill_params(scans, n, reinterpret_cast<float *>(host.data() + L.fm), reinterpret_cast<QParams *>(host.data() + L.qp));
@@ -1043,11 +982,11 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         v.R = g.num_det_rows;
         v.C = g.num_det_channels;
         v.rp = bpf_padded_rows(g);
-        auto window_source = [&](BpArgs &a) {  // the scan's transposed copy
+        auto window_source = [&](BpArgs &a, int which) {  // the scan's transposed copy
             a.tsino = v.tsino;
             a.rp = v.rp;
             a.tsino_all = 1;
-            a.tmap = reinterpret_cast<const CUtensorMap *>(base + L.maps) + s;
+            a.tmap = reinterpret_cast<const CUtensorMap *>(base + L.maps) + SW_COUNT * s + which;
         };
         v.y = sc.sinogram;
         v.nsino = z.nsino;
@@ -1059,8 +998,9 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         v.ns = g.num_recon_slices;
         for (int k = 0; k < sc.num_subsets; ++k, ++ki) {
             const int32_t *pix = sc.partition + (size_t)k * sc.subset_size;
-            hb[ki] = bp_args(g, sc.error_sinogram, sc.weights, pix, sc.subset_size, 1, v.bp, 0, z.bpp);
-            if (transposed) window_source(hb[ki]);
+            hb[ki] = bp_args(g, sc.error_sinogram, sc.weights, pix, sc.subset_size, 1, v.bp, 0,
+                             scan_bp_plan(z, SW_SUBSET));
+            if (transposed) window_source(hb[ki], SW_SUBSET);
             if (sc.partition_order) hb[ki].order = sc.partition_order + (size_t)k * sc.subset_size;
             FpArgs &f = hf[ki];
             std::memset(&f, 0, sizeof(f));
@@ -1096,7 +1036,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         if (L.setup) {
             // x0: back projection of the filtered sinogram (held in the error sinogram) into the recon, by index
             hib[s] = bp_args(g, sc.error_sinogram, nullptr, sc.full_indices, sc.num_full_indices, 1, sc.flat_recon, 1,
-                             z.ibp);
+                             scan_bp_plan(z, SW_INIT));
             FpArgs &f = hif[s];
             std::memset(&f, 0, sizeof(f));
             f.g = g;
@@ -1111,10 +1051,10 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
             // Hessian: the weights (or ones: no sinogram) with squared coefficients over every pixel
             hhb[s] = bp_args(z.hbp_slices > 0 ? one_slice_geometry(g) : g, sc.weights, nullptr,
                              reinterpret_cast<const int32_t *>(base + L.arange), z.npix, 2,
-                             const_cast<float *>(sc.fm_hessian), 0, z.hbp);
+                             const_cast<float *>(sc.fm_hessian), 0, scan_bp_plan(z, SW_HESS));
             hhb[s].out_slices = z.hbp_slices;
-            if (transposed) window_source(hib[s]);
-            if (hess_transposed) window_source(hhb[s]);
+            if (transposed) window_source(hib[s], SW_INIT);
+            if (hess_transposed) window_source(hhb[s], SW_HESS);
             FiltScan &fl = hfl[s];
             fl.in = sc.sinogram;
             fl.out = sc.error_sinogram;

@@ -5,6 +5,7 @@
 
 #include "back_project.cuh"
 #include "bp_fast.cuh"
+#include "direct_filter.cuh"
 #include "fp_cb.cuh"
 #include "mbx_common.cuh"
 #include "mbx_host.hpp"
@@ -170,6 +171,80 @@ template <class A>
 __device__ __forceinline__ const A &list_record(const A *recs, const ProjList &L, int num_scans, int step, int s) {
     const int r = L.schedule ? __ldg(L.schedule + step * num_scans + s) : 0;
     return recs[s * L.stride + r];
+}
+
+// Sizes and plans of one scan of a batch (host side).
+struct ScanSizes {
+    long long ncyl, nsino, nrecon, npix;
+    int el_tiles, sn_tiles, rc_tiles, flt_tiles;
+    BpfPlan bpp;  // subset back projection
+    CbPlan fpp;   // subset forward projection
+    CbPlan ifp;   // initial forward projection, on the same channel blocks
+    BpfPlan ibp;  // initial back projection over the region of reconstruction
+    BpfPlan hbp;  // Hessian back projection over every pixel
+    int hbp_slices;  // > 0: hbp is planned on one slice and broadcast to this many (unit-weight parallel beam)
+    bool setup;   // the scan carries the set-up inputs
+    int tr_tiles; // 32-channel blocks of the transposed copy over all views
+};
+
+inline int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
+    const mbx_geom &g = sc.geom;
+    int rc = validate_geom(&g);
+    if (rc != MBX_OK) return rc;
+    if (!sc.flat_recon || !sc.error_sinogram || !sc.fm_hessian || !sc.partition) return MBX_ERR_INVALID_ARG;
+    if (sc.num_subsets <= 0 || sc.subset_size <= 0) return MBX_ERR_INVALID_ARG;
+    if (!(sc.qp.sigma_x > 0.0f) || !(sc.qp.T > 0.0f) || !(sc.qp.p > 0.0f)) return MBX_ERR_INVALID_ARG;
+    z.bpp = plan_bp_fast(g, sc.subset_size, g.num_views);
+    // the channel blocks of either kernel variant (the tuner keeps the faster): the second's are the narrower
+    z.fpp = plan_fp_cb(g, 0, 0, 2, cb_many(g.kind) >= 4 ? CB_MANY_CHANNELS : 128, 0, MBX_BATCHED_FP_CAP);
+    z.ifp = z.fpp;
+    if (!z.bpp.ok || !z.fpp.ok) return MBX_ERR_UNSUPPORTED;  // batched path needs the radius-1 kernels
+    if ((long long)sc.subset_size * g.num_recon_slices >= (1LL << 31)) return MBX_ERR_UNSUPPORTED;
+    if (sc.subset_size > (1 << 24)) return MBX_ERR_UNSUPPORTED;  // list positions share a word with the bin
+    z.ncyl = (long long)sc.subset_size * g.num_recon_slices;
+    z.nsino = (long long)g.num_views * g.num_det_rows * g.num_det_channels;
+    z.npix = (long long)g.num_recon_rows * g.num_recon_cols;
+    z.nrecon = z.npix * g.num_recon_slices;
+    z.el_tiles = (int)((z.ncyl + BT_ELEM_TILE - 1) / BT_ELEM_TILE);
+    z.sn_tiles = (int)((z.nsino + BT_SINO_TILE - 1) / BT_SINO_TILE);
+    z.rc_tiles = (int)((z.nrecon + BT_SINO_TILE - 1) / BT_SINO_TILE);
+    z.tr_tiles = g.num_views * ceil_div(g.num_det_channels + 2 * BPF_EDGE, 32);
+    z.setup = sc.sinogram != nullptr || sc.full_indices != nullptr || sc.num_full_indices != 0;
+    z.flt_tiles = 0;
+    if (z.setup) {
+        if (!sc.sinogram || !sc.full_indices || sc.num_full_indices <= 0 || sc.num_full_indices > z.npix)
+            return MBX_ERR_INVALID_ARG;
+        // the initial forward projection reads voxels by pixel index, which shares a word with the bin
+        if (z.npix > (1 << 24) || z.nrecon >= (1LL << 31)) return MBX_ERR_UNSUPPORTED;
+        z.hbp_slices = 0;
+        if (bp_unit_broadcast(g, nullptr, sc.weights)) {  // unit-weight parallel Hessian: one slice, broadcast
+            z.hbp = plan_bp_fast(one_slice_geometry(g), z.npix, g.num_views);
+            if (z.hbp.ok && z.hbp.splits == 1) z.hbp_slices = g.num_recon_slices;
+        }
+        if (z.hbp_slices == 0) z.hbp = plan_bp_fast(g, z.npix, g.num_views);
+        if (!z.hbp.ok) return MBX_ERR_UNSUPPORTED;
+        if (g.kind != MBX_GEOM_TRANSLATION) {  // translation geometry starts from zeros (no direct recon)
+            if (!filter_admits(g.num_det_channels, g.kind != MBX_GEOM_PARALLEL))
+                return MBX_ERR_UNSUPPORTED;
+            z.ibp = plan_bp_fast(g, sc.num_full_indices, g.num_views);
+            if (!z.ibp.ok) return MBX_ERR_UNSUPPORTED;
+            z.flt_tiles = ceil_div((long long)g.num_views * g.num_det_rows, filter_shape(g.num_det_channels).rows);
+        } else {
+            z.ibp = z.hbp;  // unused
+        }
+    }
+    return MBX_OK;
+}
+
+// The back projections of a scan.  The height of a list's slice tiles, and so of its windows, can follow its pixel count
+// (cone: plan_bp_fast), so each has a tensor map of its own, whose box holds the rows that its plan waits for.
+enum { SW_SUBSET = 0, SW_INIT, SW_HESS, SW_COUNT };
+inline const BpfPlan &scan_bp_plan(const ScanSizes &z, int which) {
+    return which == SW_SUBSET ? z.bpp : which == SW_INIT ? z.ibp : z.hbp;
+}
+// Rows of the box of that map, in fours (0: the scan has no such back projection).
+inline int scan_window_box(const ScanSizes &z, int which) {
+    return which == SW_SUBSET || z.setup ? scan_bp_plan(z, which).boxq : 0;
 }
 
 // The forward-projection stage kernels of one geometry kind: b_fp (walk), b_fp_replay (stored passes) and

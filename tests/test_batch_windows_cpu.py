@@ -1,0 +1,29 @@
+"""What a batch prepares for the windows of its back projections: host-only programs over the library's headers, compiled
+with nvcc and run on the CPU."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def _run(name, tmp_path):
+    nvcc = shutil.which('nvcc') or '/usr/local/cuda/bin/nvcc'
+    if not os.path.exists(nvcc):
+        pytest.skip('nvcc is not available')
+    exe = str(tmp_path / name)
+    subprocess.run([nvcc, '-std=c++17', '--expt-relaxed-constexpr', '-gencode', 'arch=compute_100a,code=sm_100a',
+                    '-o', exe, os.path.join(HERE, name + '.cu')], check=True, capture_output=True)
+    res = subprocess.run([exe], capture_output=True, text=True)
+    assert res.returncode == 0, res.stdout + res.stderr
+    assert res.stdout.startswith('ok ')
+    return [int(v) for v in res.stdout.split()[1:]]
+
+
+def test_each_back_projection_has_a_tensor_map_of_its_own_rows(tmp_path):
+    """Subset, initial and Hessian back projections of a scan can have slice tiles of different heights (cone scans whose
+    subsets leave the chip idle): each copies through a map whose box has its own rows."""
+    scans, differ = _run('batch_windows_check', tmp_path)
+    assert scans > 5000 and differ > 100  # the sweep holds scans that one map could not serve

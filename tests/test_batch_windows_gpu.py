@@ -1,0 +1,51 @@
+"""Batched reconstructions at the sizes where the windows of the batched back projections can go wrong, against the plain
+path (whose back projections make their plans and maps call by call)."""
+import numpy as np
+import pytest
+import torch
+
+import mbirjax_b200 as mb
+from mbirjax_b200 import _capi
+from mbirjax_b200.batched import BatchedVCD, release_batched_sessions
+from mbirjax_b200.utilities import gen_ellipsoid_phantom
+from cases import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _scan(kind, views, rows, channels, seed, subsets=4):
+    ang = np.linspace(0, np.pi if kind == 'parallel' else 2 * np.pi, views, endpoint=False).astype(np.float32)
+    if kind == 'parallel':
+        model = mb.ParallelBeamModel((views, rows, channels), ang)
+    else:
+        model = mb.ConeBeamModel((views, rows, channels), ang, 4.0 * channels, 4.0 * channels)
+    model.set_params(sharpness=0.0, granularity=[subsets], partition_sequence=[0], verbose=0)
+    ph = gen_ellipsoid_phantom(tuple(model.get_params('recon_shape')), 5, seed).numpy()
+    np.random.seed(seed)
+    sino = model.forward_project(torch.as_tensor(ph, device='cuda')).cpu().numpy()
+    noise = np.random.default_rng(seed).normal(0, 0.01 * np.abs(sino).max(), sino.shape)
+    return model, (sino + noise).astype(np.float32)
+
+
+def _batch_matches_plain(items, weights, seeds, iters=2):
+    """Both paths add the same float32 terms in other orders: a few 1e-7 a projection, and some 1e-6 of the recon after
+    a few iterations; the bar is the one of the batched tests, 1e-5."""
+    release_batched_sessions()
+    _capi.get_device_error()
+    models, sinos = [m for m, _ in items], [s for _, s in items]
+    recons, _ = BatchedVCD(models, sinos, weights=weights, seeds=seeds).recon(max_iterations=iters)
+    assert _capi.get_device_error() == 0
+    for i, (model, sino) in enumerate(items):
+        np.random.seed(seeds[i])
+        plain, _ = model.recon(sino, weights=None if weights is None else weights[i], max_iterations=iters,
+                               stop_threshold_change_pct=0, logfile_path=None, print_logs=False)
+        assert rel_l2(recons[i].cpu().numpy(), plain.cpu().numpy()) <= 1e-5
+    release_batched_sessions()
+
+
+@pytest.mark.parametrize('weighted', [False, True])
+def test_cone_scans_whose_back_projections_differ_in_tile_height(cuda, weighted):
+    """The subsets of these scans take slice tiles of half the height that their set-up's back projections take."""
+    items = [_scan('cone', 60, 32, 64, 3), _scan('cone', 60, 32, 96, 4), _scan('cone', 60, 40, 64, 5)]
+    ws = [np.exp(-s / s.max()).astype(np.float32) for _, s in items] if weighted else None
+    _batch_matches_plain(items, ws, [3, 4, 5])
