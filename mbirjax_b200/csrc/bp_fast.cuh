@@ -423,6 +423,11 @@ __device__ __forceinline__ float4 bpf_view(const BpArgs &A, int v, bool flag, in
     return vw;
 }
 
+// Channels that a window of 4 boxq rows holds, in whole boxes.
+__host__ __device__ constexpr int bpf_window_channels(int kind, int boxq) {
+    return (kind == MBX_GEOM_PARALLEL ? BPF_WIN_PARALLEL : BPF_WIN_FAN) / (4 * boxq) & ~(BPF_BOX - 1);
+}
+
 // Parallel beam: the window of one view for every pixel of a box of grid rows and columns (x, y and z, w of box), as first
 // channel and channels (0: the view misses the box).  The channel is linear in the position, so the corners bound it; the
 // slack covers the rounding of either side.
@@ -431,15 +436,23 @@ struct BpfBounds {
     bool wide;  // larger than a window (or not a number)
 };
 
-__device__ __forceinline__ BpfBounds bpf_bounds(const mbx_geom &g, const float4 &vw, int4 box, int cap) {
+// The same in one word (of a window that is not wide).
+constexpr int BPF_NCH_BITS = 9;
+static_assert(BPF_WIN_PARALLEL / 4 < (1 << BPF_NCH_BITS), "the widest window's channels do not fit their bits");
+__host__ __device__ constexpr int bpf_pack_window(int c_lo, int nch) { return (c_lo + BPF_EDGE) << BPF_NCH_BITS | nch; }
+__host__ __device__ constexpr int bpf_packed_first(int w) { return (w >> BPF_NCH_BITS) - BPF_EDGE; }
+__host__ __device__ constexpr int bpf_packed_channels(int w) { return w & ((1 << BPF_NCH_BITS) - 1); }
+
+// cs, sn: the view's angle; ok: it is a view of the sinogram.
+__host__ __device__ __forceinline__ BpfBounds bpf_bounds(const mbx_geom &g, float cs, float sn, bool ok, int4 box,
+                                                         int cap) {
     const float inv_dc = 1.0f / g.delta_det_channel;
     const float det_center_channel = 0.5f * (float)(g.num_det_channels - 1);
     float n_lo = 3.0e38f, n_hi = -3.0e38f, sum = 0.0f;
-#pragma unroll
     for (int corner = 0; corner < 4; ++corner) {
         const float yt = g.delta_voxel * ((float)((corner & 1) ? box.y : box.x) - 0.5f * (float)(g.num_recon_rows - 1));
         const float xt = g.delta_voxel * ((float)((corner & 2) ? box.w : box.z) - 0.5f * (float)(g.num_recon_cols - 1));
-        const float n = ((vw.x * xt - vw.y * yt) + g.det_channel_offset) * inv_dc + det_center_channel;
+        const float n = ((cs * xt - sn * yt) + g.det_channel_offset) * inv_dc + det_center_channel;
         n_lo = fminf(n_lo, n);
         n_hi = fmaxf(n_hi, n);
         sum += n;
@@ -451,7 +464,7 @@ __device__ __forceinline__ BpfBounds bpf_bounds(const mbx_geom &g, const float4 
     b.c_lo = max((int)rintf(n_lo - slack) - 1, -BPF_EDGE);
     b.nch = max(min((int)rintf(n_hi + slack) + 1, g.num_det_channels + BPF_EDGE - 1) - b.c_lo + 1, 0);
     b.wide = b.wide || b.nch > cap;
-    if (__float_as_int(vw.w) < 0) {  // an invalid view
+    if (!ok) {  // an invalid view
         b.wide = false;
         b.nch = 0;
     }
@@ -582,7 +595,7 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
     const int lane = threadIdx.x & 31;
     float *cache = smw + WIN + lane;                           // fan: row buffer [row][lane]
     const int pitch = 4 * P.boxq;                              // of a window's channels
-    const int cap = WIN / pitch & ~(BPF_BOX - 1);              // channels of a window
+    const int cap = bpf_window_channels(KIND, P.boxq);         // channels of a window
 
     const long long slot = (long long)pg * 32 + lane;
     const long long p = (A.order && slot < num_pixels) ? A.order[slot] : slot;  // list entry of this thread
@@ -786,15 +799,15 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         cur.in = false;
         cur.tma = false;
         if constexpr (TR && !FAN) {
-            const BpfBounds mb = bpf_bounds(g, mine, box, cap);
+            const BpfBounds mb = bpf_bounds(g, mine.x, mine.y, __float_as_int(mine.w) >= 0, box, cap);
             if (!__any_sync(ALL, mb.wide)) {
-                const int pc = (mb.c_lo + BPF_EDGE) << 8 | mb.nch;
+                const int pc = bpf_pack_window(mb.c_lo, mb.nch);
                 const int nv = v_stop - vb;
                 for (int t = 0; t <= nv; ++t) {
                     nxt.in = nxt.tma = false;
                     if (t < nv) {
                         const float4 vw = view_constants(t);
-                        const int c = __shfl_sync(ALL, pc, t), nch = c & 255, c_lo = (c >> 8) - BPF_EDGE;
+                        const int c = __shfl_sync(ALL, pc, t), nch = bpf_packed_channels(c), c_lo = bpf_packed_first(c);
                         nxt.tma = nch > 0;
                         if (nxt.tma)
                             bpf_stage_tma(smw + (t & 1) * WIN, A, tmap, pipe, t & 1, s0, __float_as_int(vw.w) + c_lo + BPF_EDGE, nch);

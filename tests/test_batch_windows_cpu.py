@@ -27,3 +27,9 @@ def test_each_back_projection_has_a_tensor_map_of_its_own_rows(tmp_path):
     subsets leave the chip idle): each copies through a map whose box has its own rows."""
     scans, differ = _run('batch_windows_check', tmp_path)
     assert scans > 5000 and differ > 100  # the sweep holds scans that one map could not serve
+
+
+def test_windows_of_few_slices_keep_their_width(tmp_path):
+    """With at most 4 slices a window holds up to 288 channels: its width and first channel survive the word they share."""
+    windows, big = _run('bp_window_check', tmp_path)
+    assert windows > 100000 and big > 1000

@@ -49,3 +49,12 @@ def test_cone_scans_whose_back_projections_differ_in_tile_height(cuda, weighted)
     items = [_scan('cone', 60, 32, 64, 3), _scan('cone', 60, 32, 96, 4), _scan('cone', 60, 40, 64, 5)]
     ws = [np.exp(-s / s.max()).astype(np.float32) for _, s in items] if weighted else None
     _batch_matches_plain(items, ws, [3, 4, 5])
+
+
+@pytest.mark.parametrize('channels', [256, 260, 300])
+@pytest.mark.parametrize('subsets', [4, 48])
+def test_parallel_scans_of_few_slices(cuda, channels, subsets):
+    """With at most 4 slices a window holds up to 288 channels, and warps whose pixels lie across the grid (where the
+    Z-order jumps) take windows of that width."""
+    items = [_scan('parallel', 90, rows, channels, rows, subsets) for rows in (1, 3, 4)]
+    _batch_matches_plain(items, None, [1, 3, 4], iters=1 if subsets == 48 else 2)
