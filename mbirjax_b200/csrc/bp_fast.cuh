@@ -313,6 +313,13 @@ __device__ __forceinline__ bool bpf_elect() {
     return one != 0;
 }
 
+// Before a warp's first copies through a tensor map in global memory: the map was written by a copy to the device, and
+// the TMA unit reads maps through a cache of its own, which may hold what stood there before.
+__device__ __forceinline__ void bpf_acquire_map(const CUtensorMap *tmap) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(tmap) : "memory");
+    __syncwarp();
+}
+
 // Starts the TMA copy of channels c .. c + nch - 1 (rows of the transposed copy, counted over views and edge channels)
 // and rows r0 .. (a multiple of 4) into buffer b at win; rows outside the copy arrive as zeros.  c, nch, r0 and b are the
 // warp's.

@@ -40,6 +40,7 @@ b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
     float *smw = smb + (threadIdx.x >> 5) * bpf_warp_floats(KIND);
     BpfPipe pipe = {0, 0};
     if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND) - 32);
+    const CUtensorMap *acquired = nullptr;  // the map this warp copies through
     for (;;) {
         int u = 0;
         if ((threadIdx.x & 31) == 0) u = atomicAdd(L.counter, 1);
@@ -49,6 +50,10 @@ b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
         const int k = find_scan(L.off, num_scans, t);
         const int s = __ldg(L.order + k);
         const BpArgs &A = list_record(L.bp, L, num_scans, step, s);
+        if (TR && A.tmap != acquired) {
+            acquired = A.tmap;
+            bpf_acquire_map(acquired);
+        }
         bp_fast_run<KIND, TR>(A, A.tmap, t - __ldg(L.off + k), u & 7, 0, smw, pipe, err);
     }
 }

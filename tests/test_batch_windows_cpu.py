@@ -33,3 +33,14 @@ def test_windows_of_few_slices_keep_their_width(tmp_path):
     """With at most 4 slices a window holds up to 288 channels: its width and first channel survive the word they share."""
     windows, big = _run('bp_window_check', tmp_path)
     assert windows > 100000 and big > 1000
+
+
+def test_maps_in_global_memory_are_acquired_before_their_first_copy():
+    """The batched stages read their tensor maps from the workspace, where older maps may have stood: the kernel that hands
+    a record's map on acquires it first (a stale map can not be brought about on demand, so this reads the source)."""
+    with open(os.path.join(HERE, os.pardir, 'mbirjax_b200', 'csrc', 'vcd_batched.cu')) as f:
+        text = f.read()
+    for use in [i for i in range(len(text)) if text.startswith('bp_fast_run<', i)]:
+        kernel = text[text.rindex('__global__', 0, use):use]
+        assert 'bpf_acquire_map(' in kernel
+    assert 'bp_fast_run<' in text

@@ -58,3 +58,10 @@ def test_parallel_scans_of_few_slices(cuda, channels, subsets):
     Z-order jumps) take windows of that width."""
     items = [_scan('parallel', 90, rows, channels, rows, subsets) for rows in (1, 3, 4)]
     _batch_matches_plain(items, None, [1, 3, 4], iters=1 if subsets == 48 else 2)
+
+
+def test_batches_of_different_shapes_one_after_another(cuda):
+    """Each batch's tensor maps stand where those of the batch before may have stood."""
+    for kind, shapes in (('cone', [(40, 28, 64), (30, 20, 48)]), ('parallel', [(60, 30, 80), (50, 12, 60)]),
+                         ('cone', [(30, 20, 48), (40, 28, 64)]), ('parallel', [(50, 12, 60), (60, 30, 80)])):
+        _batch_matches_plain([_scan(kind, *s, i) for i, s in enumerate(shapes)], None, [0, 1])
