@@ -96,9 +96,13 @@ MBX_API const char *mbx_error_string(int code);
 /* The CUDA error code behind the last MBX_ERR_CUDA returned on this host thread. */
 MBX_API int mbx_last_cuda_error(void);
 /* Reads and clears the device error word of the current device (synchronises the device).
- * Bit 0: a pixel index was out of range; bit 1: a view index was out of range; bit 2: a projector tile
- * exceeded its shared-memory row cache (the geometry check should make this impossible). */
+ * Bit 0: a pixel index was out of range; bit 1: a view index was out of range; bit 2 (MBX_DEVICE_ERROR_INTERNAL): a
+ * projection failed inside the library (a copy to shared memory that did not complete, or a tile that exceeded what its
+ * plan holds; the plans should make this impossible).  The back projector's sums of such a tile leave as NaN. */
+#define MBX_DEVICE_ERROR_INTERNAL 4
 MBX_API int mbx_get_device_error(int *flags_out);
+/* Reads the same word without clearing it, after the work queued on `stream` so far (synchronises that stream only). */
+MBX_API int mbx_peek_device_error(int *flags_out, void *stream);
 /* Number of kernel launches this library has submitted since it was loaded (host-side count, all devices and
  * streams; launches replayed from a captured CUDA graph are not re-counted). */
 MBX_API uint64_t mbx_launch_count(void);

@@ -59,6 +59,7 @@ _SIGNATURES = {
     'mbx_error_string': (ctypes.c_char_p, [ctypes.c_int]),
     'mbx_last_cuda_error': (ctypes.c_int, []),
     'mbx_get_device_error': (ctypes.c_int, [ctypes.POINTER(ctypes.c_int)]),
+    'mbx_peek_device_error': (ctypes.c_int, [ctypes.POINTER(ctypes.c_int), c_void_p]),
     'mbx_launch_count': (ctypes.c_uint64, []),
     'mbx_mt19937_shuffle': (c_int32, [c_void_p, ctypes.POINTER(c_int32), c_void_p, ctypes.c_int64, c_int32]),
     'mbx_set_autotune': (ctypes.c_int, [ctypes.c_int]),
@@ -188,6 +189,26 @@ def get_device_error():
     flags = ctypes.c_int(0)
     _check(load_library().mbx_get_device_error(ctypes.byref(flags)), 'mbx_get_device_error')
     return flags.value
+
+
+MBX_DEVICE_ERROR_INTERNAL = 4
+
+
+def peek_device_error(device):
+    """The device error word after the work queued on the current stream so far, not cleared (0 on a host device)."""
+    if device.type != 'cuda':
+        return 0
+    flags = ctypes.c_int(0)
+    _check(load_library().mbx_peek_device_error(ctypes.byref(flags), _stream()), 'mbx_peek_device_error')
+    return flags.value
+
+
+def raise_on_failed_projection(device):
+    """For the ends of reconstructions, which wait for the device anyway: raises when a projection failed inside the
+    library (and clears the error word), so that its result is not taken for a reconstruction."""
+    if peek_device_error(device) & MBX_DEVICE_ERROR_INTERNAL:
+        get_device_error()
+        raise MbxError('a projection failed on the device (device error word, bit 2): the reconstruction is not valid')
 
 
 def forward_project(geom, voxel_values, pixel_indices, view_indices=None, out=None):

@@ -394,6 +394,7 @@ class _Session:
 
 
 def _results(models, flats, sino_sizes, weights, sigmas, regs, step, it, max_iterations, K, clone):
+    _capi.raise_on_failed_projection(flats[0].device)
     recons, dicts = [], []
     for s, model in enumerate(models):
         recon_shape = model.get_params('recon_shape')

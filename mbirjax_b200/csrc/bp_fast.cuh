@@ -277,12 +277,14 @@ __device__ __forceinline__ float bpf_ldg(const float *p, bool ok) {
 struct BpfPipe {
     unsigned bar;
     unsigned parity;  // bit b: parity that buffer b waits for next
+    bool failed;      // a copy did not complete: the warp's work ends
 };
 
 __device__ __forceinline__ BpfPipe bpf_pipe_init(float *at) {
     BpfPipe p;
     p.bar = (unsigned)__cvta_generic_to_shared(at);
     p.parity = 0;
+    p.failed = false;
     if ((threadIdx.x & 31) == 0) {
         asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(p.bar) : "memory");
         asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(p.bar + 8) : "memory");
@@ -292,17 +294,40 @@ __device__ __forceinline__ BpfPipe bpf_pipe_init(float *at) {
     return p;
 }
 
-// Waits for buffer b's copy (bounded: a copy that never completes is flagged, not waited for).
-__device__ __forceinline__ void bpf_pipe_wait(BpfPipe &p, int b, int *err) {
+__device__ __forceinline__ bool bpf_try_wait(unsigned bar, unsigned parity) {
+    unsigned done;
+    asm volatile("{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return done != 0;
+}
+
+__device__ __forceinline__ unsigned long long bpf_now_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Waits for buffer b's copy; the same answer in every lane.  A copy takes some microseconds; one that has not completed
+// after BPF_WAIT_NS (BPF_WAIT_AGAIN_NS once the device error word says that another failed, so that a launch of many warps
+// ends soon) never will: the error is flagged, and the caller ends its unit.
+constexpr unsigned long long BPF_WAIT_NS = 250000000, BPF_WAIT_AGAIN_NS = 2000000;
+__device__ __forceinline__ bool bpf_pipe_wait(BpfPipe &p, int b, int *err) {
     const unsigned bar = p.bar + 8u * (unsigned)b, par = (p.parity >> b) & 1u;
-    unsigned done = 0;
-    for (int i = 0; i < (1 << 22) && !done; ++i)
-        asm volatile("{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                     : "=r"(done)
-                     : "r"(bar), "r"(par)
-                     : "memory");
-    if (!done) flag_error(err, MBX_ERRFLAG_CACHE);
     p.parity ^= 1u << b;
+    bool done = bpf_try_wait(bar, par);
+    if (__all_sync(0xffffffffu, done)) return true;
+    const unsigned long long t0 = bpf_now_ns();
+    for (;;) {
+        for (int i = 0; i < 64 && !done; ++i) done = bpf_try_wait(bar, par);
+        if (__all_sync(0xffffffffu, done)) return true;
+        const bool again = err && (*reinterpret_cast<volatile int *>(err) & MBX_ERRFLAG_CACHE);
+        if (__any_sync(0xffffffffu, bpf_now_ns() - t0 > (again ? BPF_WAIT_AGAIN_NS : BPF_WAIT_NS))) break;
+    }
+    flag_error(err, MBX_ERRFLAG_CACHE);
+    p.failed = true;
+    return false;
 }
 
 // True in one lane of the (converged) warp, by elect.sync, which the compiler knows to leave a single thread: it then
@@ -639,6 +664,7 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
     // fan, current view: the rows of the warp's window
     int r0 = 0, nq = 0;
     bool fits = true;
+    bool bad = false;  // a sum is not to be trusted: it leaves as NaN, and the error is flagged
 
     auto view_constants = [&](int t) {
         return make_float4(__shfl_sync(ALL, mine.x, t), __shfl_sync(ALL, mine.y, t), __shfl_sync(ALL, mine.z, t),
@@ -686,7 +712,7 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
                     r0 = m_lo & ~3;
                     nq = (m_hi - r0 + 4) >> 2;
                     if (todo && nq > P.boxq) {  // excluded by plan_bp_fast
-                        flag_error(err, MBX_ERRFLAG_CACHE);
+                        bad = true;
                         todo = false;
                     }
                 }
@@ -781,7 +807,7 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
     }
     const bool none = !__any_sync(ALL, active);
 
-    for (; vb < v_end && !none; vb = v_stop) {
+    for (; vb < v_end && !none && !(TR && pipe.failed); vb = v_stop) {
         v = vb;
         v_stop = (TR && !FAN) ? min(vb + 32, v_end) : v_end;
         mine = bpf_view<KIND, TR>(A, min(vb + lane, v_stop - 1), pg == 0 && st == 0, err);
@@ -821,11 +847,14 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
                         bpf_footprint<KIND>(g, vw, xt, yt, coeff_power, TWO, f);
                         const bool any = active && nxt.tma && (f.a[0] != 0.0f || f.a[1] != 0.0f || f.a[2] != 0.0f);
                         nxt.in = any && f.ch >= c_lo && f.ch + TAPS <= c_lo + nch;
-                        if (any && !nxt.in) flag_error(err, MBX_ERRFLAG_CACHE);  // excluded by the bounds' slack
+                        if (any && !nxt.in) bad = true;  // excluded by the bounds' slack
                         fill(nxt, c_lo);
                     }
                     if (cur.tma) {
-                        bpf_pipe_wait(pipe, (t & 1) ^ 1, err);
+                        if (!bpf_pipe_wait(pipe, (t & 1) ^ 1, err)) {
+                            if (nxt.tma) bpf_pipe_wait(pipe, t & 1, err);  // (no copy is left in flight)
+                            break;
+                        }
                         if (cur.in) gather(cur, (t & 1) ^ 1);
                         __syncwarp();  // this buffer takes the window after the next
                     }
@@ -838,10 +867,11 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         if constexpr (FAN) {
             for (;;) {
                 if (have) {
-                    if (TR && cur.tma)
-                        bpf_pipe_wait(pipe, 0, err);
-                    else
+                    if (TR && cur.tma) {
+                        if (!bpf_pipe_wait(pipe, 0, err)) break;
+                    } else {
                         bpf_private_wait<TR>();
+                    }
                     __syncwarp();
                     if (cur.in) horizontal(cur);
                     __syncwarp();  // the window may be overwritten
@@ -856,10 +886,14 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
             for (int b = 0;; b ^= 1) {
                 const bool more = next(nxt, smw + b * WIN, b);
                 if (have) {
-                    if (TR && cur.tma)
-                        bpf_pipe_wait(pipe, b ^ 1, err);
-                    else
+                    if (TR && cur.tma) {
+                        if (!bpf_pipe_wait(pipe, b ^ 1, err)) {
+                            if (more && nxt.tma) bpf_pipe_wait(pipe, b, err);  // (no copy is left in flight)
+                            break;
+                        }
+                    } else {
                         bpf_private_wait<TR>();
+                    }
                     __syncwarp();
                     if (cur.in) gather(cur, b ^ 1);
                     __syncwarp();  // this buffer takes the window after the next
@@ -871,6 +905,12 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         }
     }
     __syncwarp();  // the warp's next unit may use the shared memory
+    if (bad) flag_error(err, MBX_ERRFLAG_CACHE);
+    if (bad || (TR && pipe.failed)) {
+        const float nan = __int_as_float(0x7fc00000);
+#pragma unroll
+        for (int s = 0; s < BPF_ST / 2; ++s) acc[s] = bpf_pair(nan, nan);
+    }
     if (p >= num_pixels) return;
     long long row_of_out = p;
     if (A.out_by_index) {  // write into a flat recon at the pixel's index (skipped for invalid indices)
@@ -932,7 +972,7 @@ bp_fast_kernel(const BpArgs args, const __grid_constant__ CUtensorMap map, int *
     const int warp = threadIdx.x >> 5;
     const int unit = blockIdx.x * BPF_LAUNCH_WARPS + warp;
     float *smw = smf + warp * bpf_warp_floats(KIND);
-    BpfPipe pipe = {0, 0};
+    BpfPipe pipe = {0, 0, false};
     if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND) - 32);
     bp_fast_run<KIND, TR>(args, TR ? &map : nullptr, unit >> 3, unit & 7, blockIdx.y, smw, pipe, err);
 }

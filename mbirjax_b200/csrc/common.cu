@@ -241,6 +241,18 @@ extern "C" int mbx_set_autotune(int mode) {
     return mbx::g_autotune.exchange(mode);
 }
 
+extern "C" int mbx_peek_device_error(int *flags_out, void *stream) {
+    int *word = mbx::device_error_ptr();
+    if (!flags_out || !word) return MBX_ERR_INVALID_ARG;
+    int value = 0;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t e = cudaMemcpyAsync(&value, word, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return mbx::set_cuda_error(e);
+    *flags_out = value;
+    return MBX_OK;
+}
+
 extern "C" int mbx_get_device_error(int *flags_out) {
     if (!flags_out) return MBX_ERR_INVALID_ARG;
     int value = 0;

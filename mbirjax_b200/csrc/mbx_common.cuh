@@ -20,7 +20,7 @@
 
 #define MBX_ERRFLAG_PIXEL 1
 #define MBX_ERRFLAG_VIEW 2
-#define MBX_ERRFLAG_CACHE 4
+#define MBX_ERRFLAG_CACHE MBX_DEVICE_ERROR_INTERNAL
 
 namespace mbx {
 

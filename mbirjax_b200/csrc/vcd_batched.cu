@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(32 * BPF_LAUNCH_WARPS, 8)
 b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
     extern __shared__ __align__(128) float smb[];
     float *smw = smb + (threadIdx.x >> 5) * bpf_warp_floats(KIND);
-    BpfPipe pipe = {0, 0};
+    BpfPipe pipe = {0, 0, false};
     if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND) - 32);
     const CUtensorMap *acquired = nullptr;  // the map this warp copies through
     for (;;) {
@@ -55,6 +55,7 @@ b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
             bpf_acquire_map(acquired);
         }
         bp_fast_run<KIND, TR>(A, A.tmap, t - __ldg(L.off + k), u & 7, 0, smw, pipe, err);
+        if (TR && pipe.failed) break;
     }
 }
 

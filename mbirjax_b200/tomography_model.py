@@ -482,6 +482,7 @@ class TomographyModel(ParameterHandler):
                 if self.logger is not None:
                     self.logger.warning('Change threshold stopping condition reached')
                 break
+        _capi.raise_on_failed_projection(dev)
         self.last_error_sinogram = error_sinogram
         return flat_recon.reshape(recon_shape), (fm_rmse[:num_iters], pm_loss[:num_iters], nmae_update[:num_iters],
                                                  alpha_values[:num_iters])

@@ -65,3 +65,32 @@ def test_batches_of_different_shapes_one_after_another(cuda):
     for kind, shapes in (('cone', [(40, 28, 64), (30, 20, 48)]), ('parallel', [(60, 30, 80), (50, 12, 60)]),
                          ('cone', [(30, 20, 48), (40, 28, 64)]), ('parallel', [(50, 12, 60), (60, 30, 80)])):
         _batch_matches_plain([_scan(kind, *s, i) for i, s in enumerate(shapes)], None, [0, 1])
+
+
+def test_a_copy_that_never_completes_is_given_up(cuda, tmp_path):
+    """One warp waits for a barrier that nothing completes: the wait ends within its limit, with the error flagged."""
+    import os
+    import shutil
+    import subprocess
+    nvcc = shutil.which('nvcc') or '/usr/local/cuda/bin/nvcc'
+    if not os.path.exists(nvcc):
+        pytest.skip('nvcc is not available')
+    exe = str(tmp_path / 'bp_wait_check')
+    subprocess.run([nvcc, '-std=c++17', '--expt-relaxed-constexpr', '-gencode', 'arch=compute_100a,code=sm_100a', '-o', exe,
+                    os.path.join(os.path.dirname(os.path.abspath(__file__)), 'bp_wait_check.cu')], check=True,
+                   capture_output=True)
+    res = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert res.returncode == 0 and res.stdout.startswith('ok '), res.stdout + res.stderr
+
+
+def test_peek_leaves_the_error_word(cuda):
+    """peek_device_error reads the word after the stream's work, and leaves it for get_device_error; a caller's bad index
+    (bit 0) is no failure of the library."""
+    model, sino = _scan('parallel', 8, 4, 32, 1)
+    _capi.get_device_error()
+    _capi.back_project(model._geometry(), torch.as_tensor(sino, device=cuda),
+                       torch.tensor([5, -1, 7], dtype=torch.int32, device=cuda))
+    assert _capi.peek_device_error(cuda) == 1
+    _capi.raise_on_failed_projection(cuda)
+    assert _capi.get_device_error() == 1
+    assert _capi.peek_device_error(cuda) == 0
