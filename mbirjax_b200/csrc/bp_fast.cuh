@@ -480,7 +480,7 @@ __host__ __device__ __forceinline__ BpfBounds bpf_bounds(const mbx_geom &g, floa
                                                          int cap) {
     const float inv_dc = 1.0f / g.delta_det_channel;
     const float det_center_channel = 0.5f * (float)(g.num_det_channels - 1);
-    float n_lo = 3.0e38f, n_hi = -3.0e38f, sum = 0.0f;
+    float n_lo = 3.0e38f, n_hi = -3.0e38f, sum = 0.0f, size = 0.0f;
     for (int corner = 0; corner < 4; ++corner) {
         const float yt = g.delta_voxel * ((float)((corner & 1) ? box.y : box.x) - 0.5f * (float)(g.num_recon_rows - 1));
         const float xt = g.delta_voxel * ((float)((corner & 2) ? box.w : box.z) - 0.5f * (float)(g.num_recon_cols - 1));
@@ -488,11 +488,12 @@ __host__ __device__ __forceinline__ BpfBounds bpf_bounds(const mbx_geom &g, floa
         n_lo = fminf(n_lo, n);
         n_hi = fmaxf(n_hi, n);
         sum += n;
+        size = fmaxf(size, (fabsf(cs * xt) + fabsf(sn * yt) + fabsf(g.det_channel_offset)) * inv_dc + det_center_channel);
     }
     BpfBounds b;
     b.wide = !(fabsf(sum) < 4.0e6f) || !(n_hi - n_lo < 1.0e6f);
     if (b.wide) n_lo = n_hi = 0.0f;
-    const float slack = 0.02f;
+    const float slack = fmaxf(0.02f, 8.0e-7f * size);  // six roundings on either side, of terms up to `size` channels
     b.c_lo = max((int)rintf(n_lo - slack) - 1, -BPF_EDGE);
     b.nch = max(min((int)rintf(n_hi + slack) + 1, g.num_det_channels + BPF_EDGE - 1) - b.c_lo + 1, 0);
     b.wide = b.wide || b.nch > cap;

@@ -1,7 +1,8 @@
 // Host-only check of the parallel back projector's search for windows by the box of a warp's pixels (bp_fast.cuh): over
 // recons of 1 to 40 slices, detectors up to 512 channels, grid boxes of every width and 180 views, a window that is not
-// wide comes back from its one-word form as it went in; and so do all windows up to the widest that a plan has; printing
-// "ok <windows> <of more than 255 channels>" or the first failure.  Runs on the CPU (no device call).
+// wide comes back from its one-word form as it went in; and so do all windows up to the widest that a plan has; and the taps
+// of a box's pixels, with their centre channel rounded one way or another, lie in its window, for detectors up to a million
+// channels; printing "ok <windows> <of more than 255 channels> <pixels>" or the first failure.  Runs on the CPU (no device call).
 #include <cmath>
 #include <cstdio>
 
@@ -53,6 +54,45 @@ int main() {
                     }
                 }
         }
-    std::printf("ok %ld %ld\n", windows, big);
+    long pixels = 0;
+    unsigned rnd = 1;
+    auto draw = [&rnd]() { return (rnd = rnd * 1664525u + 1013904223u) >> 8; };
+    for (int C : {300, 5000, 20000, 65536, 300000, 900000})
+        for (float offset : {0.0f, 0.37f, -0.25f * (float)C})
+            for (int it = 0; it < 20000; ++it) {
+                mbx_geom g = {};
+                g.kind = MBX_GEOM_PARALLEL;
+                g.num_views = 1;
+                g.num_det_rows = g.num_recon_slices = 28;
+                g.num_det_channels = g.num_recon_cols = C;
+                g.num_recon_rows = 64 + draw() % 2000;
+                g.delta_det_channel = 1.0f;
+                g.delta_voxel = 0.99f;
+                g.det_channel_offset = offset;
+                const int r0 = (int)(draw() % (unsigned)(g.num_recon_rows - 4)), c0 = (int)(draw() % (unsigned)(C - 20));
+                const int4 box = {r0, r0 + (int)(draw() % 4), c0, c0 + (int)(draw() % 16)};
+                const float a = 3.14159265f * (float)(draw() % 100000) / 100000.0f, cs = std::cos(a), sn = std::sin(a);
+                const BpfBounds b = bpf_bounds(g, cs, sn, true, box, 288);
+                if (b.wide) continue;
+                for (int row : {box.x, box.y})
+                    for (int col : {box.z, box.w}) {
+                        const float yt = g.delta_voxel * ((float)row - 0.5f * (float)(g.num_recon_rows - 1));
+                        const float xt = g.delta_voxel * ((float)col - 0.5f * (float)(C - 1));
+                        const float mid = 0.5f * (float)(C - 1);
+                        const float x[3] = {cs * xt - sn * yt, std::fma(cs, xt, -(sn * yt)), std::fma(-sn, yt, cs * xt)};
+                        for (int k = 0; k < 6; ++k) {
+                            const float n = k < 3 ? (x[k] + offset) + mid : std::fma(x[k - 3] + offset, 1.0f, mid);
+                            const int nc = (int)std::rint(n);
+                            if (nc + 1 < 0 || nc - 1 >= C) continue;
+                            ++pixels;
+                            const int first = nc - 1 < -BPF_EDGE ? -BPF_EDGE : nc - 1;
+                            if (first < b.c_lo || (nc + 1 < C ? nc + 1 : C - 1) >= b.c_lo + b.nch) {
+                                std::printf("FAIL %d channels: centre %d outside %d + %d\n", C, nc, b.c_lo, b.nch);
+                                return 1;
+                            }
+                        }
+                    }
+            }
+    std::printf("ok %ld %ld %ld\n", windows, big, pixels);
     return windows > 0 ? 0 : 1;
 }

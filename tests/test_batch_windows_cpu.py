@@ -30,9 +30,10 @@ def test_each_back_projection_has_a_tensor_map_of_its_own_rows(tmp_path):
 
 
 def test_windows_of_few_slices_keep_their_width(tmp_path):
-    """With at most 4 slices a window holds up to 288 channels: its width and first channel survive the word they share."""
-    windows, big = _run('bp_window_check', tmp_path)
-    assert windows > 100000 and big > 1000
+    """With at most 4 slices a window holds up to 288 channels: its width and first channel survive the word they share.
+    A box's window holds the taps of its pixels whichever way their centre channel is rounded."""
+    windows, big, pixels = _run('bp_window_check', tmp_path)
+    assert windows > 100000 and big > 1000 and pixels > 1000000
 
 
 def test_maps_in_global_memory_are_acquired_before_their_first_copy():
