@@ -26,10 +26,9 @@
 
 namespace mbx {
 
-// Whether a call makes a transposed copy of its views (bp_fast.cuh): the copy moves R C values per view, the projection
-// N S.
-static bool bp_transposes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
-    return num_pixels * g.num_recon_slices * BPF_TRANSPOSE_RATIO >= (long long)g.num_det_rows * g.num_det_channels &&
+// Whether a call makes a transposed copy of its views (bp_fast.cuh): the copy's rows are addressed in 32 bits.
+static bool bp_transposes(const mbx_geom &g, const BpfPlan &pl, long long num_pixels, int num_views_sel) {
+    return bp_windows(g, pl, num_pixels, num_views_sel) &&
            (long long)g.num_views * (g.num_det_channels + 2 * BPF_EDGE) * bpf_padded_rows(g) < (1LL << 31);
 }
 
@@ -55,26 +54,33 @@ bool bpf_window_map(CUtensorMap &map, const float *copy, const mbx_geom &g, int 
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Parallel-beam calls with values and no windows gather (bp_gather.cuh).
+static bool bp_gathers(const mbx_geom &g, const BpfPlan &pl, long long num_pixels, int num_views_sel) {
+    return g.kind == MBX_GEOM_PARALLEL && !bp_windows(g, pl, num_pixels, num_views_sel);
+}
+
 size_t bp_workspace_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
     const BpfPlan fp = plan_bp_fast(g, num_pixels, num_views_sel);
     if (!fp.ok) return plan_bp(g, num_pixels, num_views_sel).workspace;
-    if (bp_gathers(g, num_pixels, true))  // with values; without any, windows and no transposed copy
+    if (bp_gathers(g, fp, num_pixels, num_views_sel))  // (without values: the partial sums of the plan)
         return std::max(fp.workspace, plan_bp_gather(g, num_pixels, num_views_sel).workspace);
-    return fp.workspace + (bp_transposes(g, num_pixels, num_views_sel) ? bpf_transposed_bytes(g, num_views_sel) : 0);
+    return fp.workspace +
+           (bp_transposes(g, fp, num_pixels, num_views_sel) ? bpf_transposed_bytes(g, num_views_sel) : 0);
 }
 
 size_t bp_noalloc_bytes(const mbx_geom &g, long long num_pixels, int num_views_sel) {
     const BpfPlan fp = plan_bp_fast(g, num_pixels, num_views_sel, 1);
     if (!fp.ok) return plan_bp(g, num_pixels, num_views_sel).workspace;
-    return bp_gathers(g, num_pixels, true)
+    return bp_gathers(g, fp, num_pixels, num_views_sel)
                ? std::max(fp.workspace, plan_bp_gather(g, num_pixels, num_views_sel).workspace)
                : fp.workspace;
 }
 
 static int back_project_gather(const mbx_geom &g, const float *sino, const float *w, const int32_t *pix,
                                long long num_pixels, const int32_t *views, int num_views_sel, int coeff_power,
-                               float scale, float *out, void *ws, size_t ws_bytes, cudaStream_t st) {
-    const BpgPlan pl = plan_bp_gather(g, num_pixels, num_views_sel);
+                               float scale, float *out, void *ws, size_t ws_bytes, cudaStream_t st,
+                               int splits_of = 0) {
+    const BpgPlan pl = plan_bp_gather(g, num_pixels, num_views_sel, splits_of);
     if (pl.workspace > 0 && (ws == nullptr || ws_bytes < pl.workspace)) return MBX_ERR_WORKSPACE;
     const long long stride = num_pixels * (long long)g.num_recon_slices;
     const bool split = pl.splits > 1;
@@ -109,8 +115,9 @@ static cudaError_t launch_bp_fast_kind(const BpArgs &A, const CUtensorMap &map, 
     auto kern = bp_fast_kernel<KIND, TR>;
     const cudaError_t ea = set_max_dynamic_smem(reinterpret_cast<const void *>(kern), 100 * 1024);
     if (ea != cudaSuccess) return ea;
-    const dim3 grid((unsigned)(A.plan.gx * A.plan.gy * (BPF_WARPS / BPF_LAUNCH_WARPS)), A.plan.splits);
-    kern<<<grid, 32 * BPF_LAUNCH_WARPS, bpf_smem_bytes(KIND, BPF_LAUNCH_WARPS), st>>>(A, map, device_error_ptr());
+    constexpr int W = bpf_launch_warps(TR);
+    const dim3 grid((unsigned)(A.plan.gx * A.plan.gy * (BPF_WARPS / W)), A.plan.splits);
+    kern<<<grid, 32 * W, bpf_smem_bytes(KIND, W, TR), st>>>(A, map, device_error_ptr());
     note_launch();
     return cudaGetLastError();
 }
@@ -152,15 +159,20 @@ int back_project(const mbx_geom &g, const float *sino, const float *w, const int
         A.g = g;
     }
     A.plan = plan_bp_fast(g, num_pixels, num_views_sel, noalloc);
-    if (A.plan.ok && bp_gathers(g, num_pixels, sino != nullptr))
+    if (A.plan.ok && sino && bp_gathers(g, A.plan, num_pixels, num_views_sel))
         return back_project_gather(g, sino, w, pix, num_pixels, views, num_views_sel, coeff_power, scale, out, ws,
                                    ws_bytes, st);
     if (A.plan.ok) {
-        bool tr = !noalloc && sino && bp_transposes(g, num_pixels, num_views_sel);
+        bool tr = !noalloc && sino && bp_transposes(g, A.plan, num_pixels, num_views_sel);
         const size_t need = A.plan.workspace + (tr ? bpf_transposed_bytes(g, num_views_sel) : 0);
         if (need > 0 && (ws == nullptr || ws_bytes < need)) return MBX_ERR_WORKSPACE;
         float *copy = reinterpret_cast<float *>(static_cast<char *>(ws) + A.plan.workspace);
         tr = tr && bpf_window_map(map, copy, g, num_views_sel, A.plan.boxq);
+        // parallel with windows by its size, but no room or no map for them: the gather in the windows' splits, so that the
+        // sums are the same (720 x 64 x 512 subset of 4: the gather takes 2.26 ms, reading taps as bp_direct_unit does 4.5)
+        if (g.kind == MBX_GEOM_PARALLEL && sino && !tr)
+            return back_project_gather(g, sino, w, pix, num_pixels, views, num_views_sel, coeff_power, scale, out, ws,
+                                       ws_bytes, st, A.plan.splits);
         const long long stride = num_pixels * (long long)g.num_recon_slices;
         A.views_per_split = A.plan.views_per_split;
         if (A.plan.splits > 1) {

@@ -11,19 +11,20 @@
 //    It is trig-free: cos/sin(theta - theta_p) and 1/cos(theta_p) come from the per-view cos/sin and
 //    rsqrt(D^2 + u^2) instead of atan2/cos/sin per pixel.
 //  * The channels and rows that the warp's footprints touch (their exact range, by warp min/max) are a small window
-//    of the view, about 20 to 36 channels wide for a compact pixel list.  It is copied once into the warp's own shared
-//    memory, channels outermost ([channel][row], weights multiplied in, zeros off the detector), so that a lane reads
-//    four rows of a channel with one 16-byte load at a constant offset; the channel pitch is an odd number of 16-byte
-//    units, so lanes on neighbouring channels hit different banks.  Calls with enough pixels first make a transposed
-//    copy of their sinogram (view, channel, row), whose windows the TMA unit copies (boxes of 8 channels; no load or
-//    store instruction, and no share of the load/store pipe, which bounds the kernel); the others copy by plain loads.
+//    of the view, about 20 to 36 channels wide for a compact pixel list.  Calls that bp_windows() names first make a
+//    transposed copy of their sinogram (view, channel, row; weights multiplied in, zeros off the detector), whose windows
+//    the TMA unit copies into the warp's own shared memory, channels outermost (boxes of 8 channels; no load or store
+//    instruction, and no share of the load/store pipe, which bounds the kernel), so that a lane reads four rows of a
+//    channel with one 16-byte load at a constant offset; the channel pitch is an odd number of 16-byte units, so lanes on
+//    neighbouring channels hit different banks.  The other calls read their taps from the sinogram itself
+//    (bp_direct_unit, bp_gather.cuh).
 //  * Fan geometries: a lane first forms the horizontal sum of each window row in its own column of a row buffer
 //    ([row][lane], conflict-free), then the vertical fan reads three of its rows per slice with no bounds tests.
 //    plan_bp_fast admits a geometry only when the rows of a slice tile (ts * max |dm/dk| + 4) fit that buffer.
-//    Measured (B200, one subset of 4 unless said): parallel 652 x 57 x 437 1724 -> 895 us a call against the kernel that
+//    Measured (B200, one subset of 4 unless said): parallel 652 x 57 x 437 1724 -> 885 us a call against the kernel that
 //    gathered each tap from global memory (21 instructions per slice and view there, 12 here), cone 360 x 256 x 512
-//    (subset of 8) 11.98 -> 6.25 ms, translation 49 x 128 x 128 (all pixels) 197 -> 123 us, weighted squared cone
-//    180 x 61 x 203 2.41 -> 1.26 ms; with windows copied by 16-byte cp.async instead of the TMA the parallel call took
+//    (subset of 8) 11.98 -> 6.34 ms, translation 49 x 128 x 128 (all pixels) 197 -> 107 us, weighted squared cone
+//    180 x 61 x 203 2.41 -> 1.29 ms; with windows copied by 16-byte cp.async instead of the TMA the parallel call took
 //    975 us.
 //  * Pixels without locality, which would need many windows, are handled some lanes at a time, each with private
 //    columns of its own taps in the place of the window.
@@ -53,8 +54,6 @@ constexpr int BPF_FAN_QUADS = 13;   // most rows of a fan window and of the row 
 // BPF_WINDOWS stretches of BPF_SPLIT channels.
 constexpr int BPF_SPLIT = 32;
 constexpr int BPF_WINDOWS = 4;
-// A call copies its sinogram transposed when its pixels' slices are at least 1 / this of a view's elements.
-constexpr int BPF_TRANSPOSE_RATIO = 8;
 // Window floats: 32 channels of 36 rows (parallel, two buffers), 32 channels of 52 rows (fan geometries).
 constexpr int BPF_WIN_PARALLEL = 32 * 36;
 constexpr int BPF_WIN_FAN = 32 * 4 * BPF_FAN_QUADS;
@@ -365,69 +364,26 @@ __device__ __forceinline__ void bpf_stage_tma(float *win, const BpArgs &A, const
     }
 }
 
-// Copies rows r0 .. r0 + 4 nq - 1 of channels c_lo .. c_lo + nch - 1 of one view (element offset voff of the sinogram)
-// into win ([channel][row], channel pitch `pitch`), by one warp: lanes along channels, four rows per lane and 16-byte
-// store, the weights multiplied in, zeros off the detector; a NULL sinogram is all ones.
-__device__ __forceinline__ float4 bpf_four_rows(const BpArgs &A, int voff, int r, int n) {
-    const int num_channels = A.g.num_det_channels, num_rows = A.g.num_det_rows;
-    const bool cok = n >= 0 && n < num_channels;
-    const int o = voff + r * num_channels + n;
-    float v[4], w[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const bool ok = cok && r + j >= 0 && r + j < num_rows;
-        v[j] = A.sino ? bpf_ldg(A.sino + (o + j * num_channels), ok) : (ok ? 1.0f : 0.0f);
-    }
-    if (A.wts) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            w[j] = bpf_ldg(A.wts + (o + j * num_channels), cok && r + j >= 0 && r + j < num_rows);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] *= w[j];
-    }
-    return make_float4(v[0], v[1], v[2], v[3]);
-}
-
-__device__ __forceinline__ void bpf_stage(float *win, const BpArgs &A, int voff, int r0, int nq, int pitch, int c_lo,
-                                          int nch, int lane) {
-    const int items = nch * nq;  // at most 416; the quotients below are exact while items * nch < 2^18
-    const unsigned inv = ((1u << 18) + (unsigned)nch - 1u) / (unsigned)nch;
-#pragma unroll 2
-    for (int it = lane; it < items; it += 32) {
-        const int q = (int)(((unsigned)it * inv) >> 18);
-        const int c = it - q * nch;
-        *reinterpret_cast<float4 *>(win + c * pitch + 4 * q) = bpf_four_rows(A, voff, r0 + 4 * q, c_lo + c);
-    }
-}
-
-// A lane's own channels ch .. ch + taps - 1, rows r0 .. r0 + 4 nq - 1, into its private columns at win.
-template <bool TR>
+// A lane's own channels ch .. ch + taps - 1 (on the view or its edge channels), rows r0 .. r0 + 4 nq - 1, into its private
+// columns at win.
 __device__ __forceinline__ void bpf_stage_private(float *win, const BpArgs &A, int voff, int r0, int nq, int pitch,
                                                   int ch, int taps) {
     for (int k = 0; k < taps; ++k) {
         float *dst = win + k * pitch;
-        if constexpr (TR) {  // (a lane's taps lie on the view's channels or its edge channels)
-            const float *src = A.tsino + (long long)(voff + ch + k + BPF_EDGE) * A.rp;
-            for (int q = 0, r = r0; q < nq; ++q, r += 4) {
-                const bool ok = r >= 0 && r < A.rp;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;"
-                             ::"r"((unsigned)__cvta_generic_to_shared(dst + 4 * q)), "l"(ok ? src + r : A.tsino), "r"(ok ? 16 : 0)
-                             : "memory");
-            }
-        } else {
-            for (int q = 0; q < nq; ++q)
-                *reinterpret_cast<float4 *>(dst + 4 * q) = bpf_four_rows(A, voff, r0 + 4 * q, ch + k);
+        const float *src = A.tsino + (long long)(voff + ch + k + BPF_EDGE) * A.rp;
+        for (int q = 0, r = r0; q < nq; ++q, r += 4) {
+            const bool ok = r >= 0 && r < A.rp;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;"
+                         ::"r"((unsigned)__cvta_generic_to_shared(dst + 4 * q)), "l"(ok ? src + r : A.tsino), "r"(ok ? 16 : 0)
+                         : "memory");
         }
     }
 }
 
 // Waits for this warp's private columns.
-template <bool TR>
 __device__ __forceinline__ void bpf_private_wait() {
-    if (TR) {
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the next TMA copy into the buffer
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the next TMA copy into the buffer
 }
 
 // The constants of view v of a call, see bpf_footprint.
@@ -606,11 +562,55 @@ __device__ __forceinline__ void bpf_vertical(bpf2 (&acc)[BPF_ST / 2], const BpfI
     }
 }
 
+__device__ __forceinline__ void bpf_vertical_fan(bpf2 (&acc)[BPF_ST / 2], const BpfItem &it, const float *cache, float k_first,
+                                                 int nsq, float delta_voxel, int coeff_power) {
+    if (it.A1 > 2.0f)
+        bpf_vertical<true, true>(acc, it, cache, k_first, nsq, delta_voxel, coeff_power);
+    else if (coeff_power == 2)
+        bpf_vertical<true, false>(acc, it, cache, k_first, nsq, delta_voxel, 2);
+    else
+        bpf_vertical<false, false>(acc, it, cache, k_first, nsq, delta_voxel, 1);
+}
+
+// A lane's sums (list entry p, slices s0 .. s0 + ns - 1) into the output; `failed` ones leave as NaN, and `flag` says so.
+__device__ __forceinline__ void bpf_write(const BpArgs &A, bpf2 (&acc)[BPF_ST / 2], bool failed, bool flag, long long p,
+                                          bool active, int split, int s0, int ns, int *err) {
+    if (flag) flag_error(err, MBX_ERRFLAG_CACHE);
+    if (failed) {
+        const float nan = __int_as_float(0x7fc00000);
+#pragma unroll
+        for (int s = 0; s < BPF_ST / 2; ++s) acc[s] = bpf_pair(nan, nan);
+    }
+    if (p >= A.num_pixels) return;
+    long long row_of_out = p;
+    if (A.out_by_index) {  // write into a flat recon at the pixel's index (skipped for invalid indices)
+        if (!active) return;
+        row_of_out = A.pix[p];
+    }
+    const float sc = (A.split_stride == 0) ? A.scale : 1.0f;
+    if (A.out_slices > 0) {  // the one slice's value in every slice of the cylinder
+        float *out = A.out + row_of_out * (long long)A.out_slices;
+        float v, unused;
+        bpf_unpair(acc[0], v, unused);
+        v = active ? sc * v : 0.0f;
+        for (int s = 0; s < A.out_slices; ++s) out[s] = v;
+        return;
+    }
+    float *out = A.out + (long long)split * A.split_stride + row_of_out * (long long)A.g.num_recon_slices + s0;
+#pragma unroll
+    for (int s = 0; s < BPF_ST / 2; ++s) {
+        float x, y;
+        bpf_unpair(acc[s], x, y);
+        if (2 * s < ns) out[2 * s] = active ? sc * x : 0.0f;
+        if (2 * s + 1 < ns) out[2 * s + 1] = active ? sc * y : 0.0f;
+    }
+}
+
 // One warp's unit of work: pixel group pg (32 list entries), slice tile st, view split `split`; smw: bpf_warp_floats
 // of shared memory of its own.  No barrier beyond the warp.  The window of the next pass is copied while the current
 // one is used: into a second buffer (parallel), or into the one buffer once the horizontal sums have been taken from
 // it, during the vertical fan (fan geometries).
-template <int KIND, bool TR, bool TWO>
+template <int KIND, bool TWO>
 __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorMap *tmap, int pg, int st, int split, float *smw, BpfPipe &pipe,
                                              int *err) {
     constexpr bool FAN = KIND != MBX_GEOM_PARALLEL;
@@ -688,7 +688,7 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         while (!__any_sync(ALL, todo)) {
             if (v >= v_stop) return false;
             const int t = (v - vb) & 31;
-            if (t == 0 && v != vb) mine = bpf_view<KIND, TR>(A, min(v + lane, v_stop - 1), pg == 0 && st == 0, err);
+            if (t == 0 && v != vb) mine = bpf_view<KIND, true>(A, min(v + lane, v_stop - 1), pg == 0 && st == 0, err);
             const float4 vw = view_constants(t);
             ++v;
             voff = __float_as_int(vw.w);
@@ -725,20 +725,17 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
             const int bucket = todo ? min((f.ch - w.c_lo) / BPF_SPLIT, 31) : 31;
             window = __popc(__reduce_or_sync(ALL, todo ? 1u << bucket : 0u)) <= BPF_WINDOWS;
         }
-        it.tma = TR && window;
+        it.tma = window;
         it.in = w.in;
         fill(it, w.c_lo);
         if (window) {
-            if (TR)
-                bpf_stage_tma(win, A, tmap, pipe, b, FAN ? r0 : s0, voff + w.c_lo + BPF_EDGE, w.nch);
-            else
-                bpf_stage(win, A, voff, FAN ? r0 : s0, FAN ? nq : nsq, pitch, w.c_lo, w.nch, lane);
+            bpf_stage_tma(win, A, tmap, pipe, b, FAN ? r0 : s0, voff + w.c_lo + BPF_EDGE, w.nch);
         } else {  // as many lanes as there is room for, each with columns of its own
             const int rank = __popc(__ballot_sync(ALL, todo) & ((1u << lane) - 1u));
             it.in = todo && rank < WIN / (TAPS * pitch);
             it.off = rank * (TAPS * pitch);
             if (it.in)
-                bpf_stage_private<TR>(win + it.off, A, voff, FAN ? r0 : s0, FAN ? nq : nsq, pitch, f.ch, TAPS);
+                bpf_stage_private(win + it.off, A, voff, FAN ? r0 : s0, FAN ? nq : nsq, pitch, f.ch, TAPS);
         }
         it.row0 = r0;
         it.nq = nq;
@@ -790,49 +787,27 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         });
     };
     auto vertical = [&](const BpfItem &it) {
-        if (it.A1 > 2.0f)
-            bpf_vertical<true, true>(acc, it, cache, k_first, nsq, g.delta_voxel, coeff_power);
-        else if (coeff_power == 2)
-            bpf_vertical<true, false>(acc, it, cache, k_first, nsq, g.delta_voxel, 2);
-        else
-            bpf_vertical<false, false>(acc, it, cache, k_first, nsq, g.delta_voxel, 1);
+        bpf_vertical_fan(acc, it, cache, k_first, nsq, g.delta_voxel, coeff_power);
     };
     // parallel: the box of the warp's pixels; a box that fits one window in every view of 32 needs no search for the
     // window view by view (batched stage of 6 scans 2.16 -> 1.90 ms a step, a plain 652 x 57 x 437 subset
     // unchanged; for the fan geometries the second loop's code cost more than the searches, 6.25 -> 7.9 ms on the cone)
     int4 box = make_int4(0, 0, 0, 0);
-    if constexpr (TR && !FAN) {
+    if constexpr (!FAN) {
         const int idx = active ? pix[p] : 0, row = idx / g.num_recon_cols, col = idx - row * g.num_recon_cols;
         box = make_int4(__reduce_min_sync(ALL, active ? row : INT_MAX), __reduce_max_sync(ALL, active ? row : INT_MIN),
                         __reduce_min_sync(ALL, active ? col : INT_MAX), __reduce_max_sync(ALL, active ? col : INT_MIN));
     }
     const bool none = !__any_sync(ALL, active);
 
-    for (; vb < v_end && !none && !(TR && pipe.failed); vb = v_stop) {
+    for (; vb < v_end && !none && !pipe.failed; vb = v_stop) {
         v = vb;
-        v_stop = (TR && !FAN) ? min(vb + 32, v_end) : v_end;
-        mine = bpf_view<KIND, TR>(A, min(vb + lane, v_stop - 1), pg == 0 && st == 0, err);
-        if (!FAN && !TR && !A.sino) {
-            // unit sinogram: the same additions as gathering ones (the unit-weight Hessian, usually of one slice)
-            for (; v < v_stop; ++v) {
-                const int t = (v - vb) & 31;
-                if (t == 0 && v != vb) mine = bpf_view<KIND, TR>(A, min(v + lane, v_stop - 1), pg == 0 && st == 0, err);
-                const float4 vw = view_constants(t);
-                if (__float_as_int(vw.w) < 0) continue;
-                bpf_footprint<KIND>(g, vw, xt, yt, coeff_power, TWO, f);
-                if (active)
-#pragma unroll
-                    for (int s = 0; s < BPF_ST / 2; ++s)
-                        if (2 * s < ns)
-                            acc[s] = bpf_add(bpf_pair(f.a[0], f.a[0]),
-                                             bpf_add(bpf_pair(f.a[1], f.a[1]), bpf_add(bpf_pair(f.a[2], f.a[2]), acc[s])));
-            }
-            continue;
-        }
+        v_stop = !FAN ? min(vb + 32, v_end) : v_end;
+        mine = bpf_view<KIND, true>(A, min(vb + lane, v_stop - 1), pg == 0 && st == 0, err);
         BpfItem cur, nxt;
         cur.in = false;
         cur.tma = false;
-        if constexpr (TR && !FAN) {
+        if constexpr (!FAN) {
             const BpfBounds mb = bpf_bounds(g, mine.x, mine.y, __float_as_int(mine.w) >= 0, box, cap);
             if (!__any_sync(ALL, mb.wide)) {
                 const int pc = bpf_pack_window(mb.c_lo, mb.nch);
@@ -868,10 +843,10 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         if constexpr (FAN) {
             for (;;) {
                 if (have) {
-                    if (TR && cur.tma) {
+                    if (cur.tma) {
                         if (!bpf_pipe_wait(pipe, 0, err)) break;
                     } else {
-                        bpf_private_wait<TR>();
+                        bpf_private_wait();
                     }
                     __syncwarp();
                     if (cur.in) horizontal(cur);
@@ -887,13 +862,13 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
             for (int b = 0;; b ^= 1) {
                 const bool more = next(nxt, smw + b * WIN, b);
                 if (have) {
-                    if (TR && cur.tma) {
+                    if (cur.tma) {
                         if (!bpf_pipe_wait(pipe, b ^ 1, err)) {
                             if (more && nxt.tma) bpf_pipe_wait(pipe, b, err);  // (no copy is left in flight)
                             break;
                         }
                     } else {
-                        bpf_private_wait<TR>();
+                        bpf_private_wait();
                     }
                     __syncwarp();
                     if (cur.in) gather(cur, b ^ 1);
@@ -906,47 +881,166 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         }
     }
     __syncwarp();  // the warp's next unit may use the shared memory
-    if (bad) flag_error(err, MBX_ERRFLAG_CACHE);
-    if (bad || (TR && pipe.failed)) {
-        const float nan = __int_as_float(0x7fc00000);
-#pragma unroll
-        for (int s = 0; s < BPF_ST / 2; ++s) acc[s] = bpf_pair(nan, nan);
-    }
-    if (p >= num_pixels) return;
-    long long row_of_out = p;
-    if (A.out_by_index) {  // write into a flat recon at the pixel's index (skipped for invalid indices)
-        if (!active) return;
-        row_of_out = pix[p];
-    }
-    const float sc = (A.split_stride == 0) ? A.scale : 1.0f;
-    if (A.out_slices > 0) {  // the one slice's value in every slice of the cylinder
-        float *out = A.out + row_of_out * (long long)A.out_slices;
-        float v, unused;
-        bpf_unpair(acc[0], v, unused);
-        v = active ? sc * v : 0.0f;
-        for (int s = 0; s < A.out_slices; ++s) out[s] = v;
-        return;
-    }
-    float *out = A.out + (long long)split * A.split_stride + row_of_out * (long long)num_slices + s0;
-#pragma unroll
-    for (int s = 0; s < BPF_ST / 2; ++s) {
-        float x, y;
-        bpf_unpair(acc[s], x, y);
-        if (2 * s < ns) out[2 * s] = active ? sc * x : 0.0f;
-        if (2 * s + 1 < ns) out[2 * s + 1] = active ? sc * y : 0.0f;
-    }
+    bpf_write(A, acc, bad || pipe.failed, bad, p, active, split, s0, ns, err);
 }
 
-// Shared memory of one warp, in floats: window(s), row buffer, barriers; a multiple of the 128 bytes a TMA destination
-// is aligned to.
-__host__ __device__ constexpr int bpf_warp_floats(int kind) {
-    return (kind == MBX_GEOM_PARALLEL ? 2 * BPF_WIN_PARALLEL : BPF_WIN_FAN + 4 * BPF_FAN_QUADS * 32) + 32;
+// The same unit without a transposed copy to take windows of (calls whose scratch holds none, or that project ones): each
+// lane reads its taps from the sinogram itself, for the fan geometries each detector row once, four rows in flight, into
+// its column of the row buffer.  Bound by the load/store pipe and the latency of the gathers.  Measured where windows copied
+// by plain loads stood here before: cone 100 x 200 x 60 (subset of 8) 126 -> 45 us, 256 x 128 x 256 (subset of 8)
+// 1035 -> 598 us, translation 49 x 128 x 128 (subset of 4) 85 -> 42 us, unit-weight Hessian of cone 256 x 128 x 256
+// 4.66 -> 2.98 ms.
+template <int KIND, bool TWO>
+__device__ __forceinline__ void bp_direct_unit(const BpArgs &args, int pg, int st, int split, float *smw, int *err) {
+    constexpr bool FAN = KIND != MBX_GEOM_PARALLEL;
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int TAPS = TWO ? 2 : 3;
+    const BpArgs A = args;  // by value: a record in global memory is read once, not in the loops
+    const mbx_geom &g = A.g;
+    const int lane = threadIdx.x & 31;
+    float *cache = smw + lane;  // fan: row buffer [row][lane]
+    const long long slot = (long long)pg * 32 + lane;
+    const long long p = (A.order && slot < A.num_pixels) ? A.order[slot] : slot;
+    const int s0 = st * A.plan.ts, ns = min(A.plan.ts, g.num_recon_slices - s0);
+    if (ns <= 0) return;
+    const int nsq = (ns + 3) >> 2;
+    const float k_first = (float)s0, k_last = (float)(s0 + 4 * nsq - 1);
+    const int v_begin = split * A.views_per_split, v_end = min(A.num_views_sel, v_begin + A.views_per_split);
+    const int num_rows = g.num_det_rows, num_channels = g.num_det_channels;
+
+    bool active = p < A.num_pixels;
+    float xt = 0.0f, yt = 0.0f;
+    if (active) {
+        const int idx = A.pix[p];
+        active = idx >= 0 && idx < g.num_recon_rows * g.num_recon_cols;
+        if (active)
+            bpf_pixel<KIND>(g, idx, xt, yt);
+        else if (st == 0 && split == 0)
+            flag_error(err, MBX_ERRFLAG_PIXEL);
+    }
+
+    bpf2 acc[BPF_ST / 2];
+#pragma unroll
+    for (int s = 0; s < BPF_ST / 2; ++s) acc[s] = 0ull;
+    bool bad = false;
+
+    for (int vb = v_begin; vb < v_end; vb += 32) {
+        const float4 mine = bpf_view<KIND, false>(A, min(vb + lane, v_end - 1), pg == 0 && st == 0, err);
+        const int nv = min(32, v_end - vb);
+        for (int t = 0; t < nv; ++t) {
+            const float4 vw = make_float4(__shfl_sync(ALL, mine.x, t), __shfl_sync(ALL, mine.y, t),
+                                          __shfl_sync(ALL, mine.z, t), __shfl_sync(ALL, mine.w, t));
+            const int voff = __float_as_int(vw.w);
+            if (voff < 0) continue;
+            BpfFoot f;
+            bpf_footprint<KIND>(g, vw, xt, yt, A.coeff_power, TWO, f);
+            bool in = active && (f.a[0] != 0.0f || f.a[1] != 0.0f || f.a[2] != 0.0f);
+            bool on[TAPS];  // taps on the detector
+#pragma unroll
+            for (int k = 0; k < TAPS; ++k) on[k] = (unsigned)(f.ch + k) < (unsigned)num_channels;
+            if constexpr (FAN) {
+                const float m_a = rintf(fmaf(k_first, f.A1, f.A0)), m_b = rintf(fmaf(k_last, f.A1, f.A0));
+                if (in && !(fabsf(m_a) < 4.0e6f && fabsf(m_b) < 4.0e6f)) {  // as in bp_fast_unit
+                    const float nan_or_0 = 0.0f * (m_a + m_b);
+#pragma unroll
+                    for (int s = 0; s < BPF_ST / 2; ++s) acc[s] = bpf_add(acc[s], bpf_pair(nan_or_0, nan_or_0));
+                    in = false;
+                }
+                const int m_lo = (int)fminf(m_a, m_b) - 1, m_hi = (int)fmaxf(m_a, m_b) + 1;
+                if (in && m_hi - m_lo >= 4 * BPF_FAN_QUADS) {  // excluded by plan_bp_fast
+                    bad = true;
+                    in = false;
+                }
+                if (in) {
+                    const float ones = f.a[0] + (f.a[1] + f.a[2]);
+                    int o = voff + m_lo * num_channels + f.ch;
+                    float *dst = cache;
+                    for (int m = m_lo; m <= m_hi; m += 4, o += 4 * num_channels, dst += 4 * 32) {
+                        float x[4][TAPS];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+#pragma unroll
+                            for (int k = 0; k < TAPS; ++k)
+                                x[j][k] = bpf_ldg(A.sino + (o + j * num_channels + k),
+                                                  A.sino && on[k] && (unsigned)(m + j) < (unsigned)num_rows);
+                        if (A.wts) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                                for (int k = 0; k < TAPS; ++k)
+                                    x[j][k] *= bpf_ldg(A.wts + (o + j * num_channels + k),
+                                                       on[k] && (unsigned)(m + j) < (unsigned)num_rows);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            dst[j * 32] = A.sino ? fmaf(f.a[0], x[j][0], fmaf(f.a[1], x[j][1], f.a[2] * x[j][TAPS - 1]))
+                                                 : ((unsigned)(m + j) < (unsigned)num_rows ? ones : 0.0f);
+                    }
+                    BpfItem it;
+                    it.row0 = m_lo;
+                    it.A0 = f.A0;
+                    it.A1 = f.A1;
+                    it.c2 = f.c2;
+                    it.zv = f.zv;
+                    bpf_vertical_fan(acc, it, cache, k_first, nsq, g.delta_voxel, A.coeff_power);
+                }
+            } else if (!A.sino) {  // (the unit-weight Hessian, usually of one slice)
+                if (in) {
+#pragma unroll
+                    for (int s = 0; s < BPF_ST / 2; ++s)
+                        if (2 * s < ns)
+                            acc[s] = bpf_add(bpf_pair(f.a[0], f.a[0]),
+                                             bpf_add(bpf_pair(f.a[1], f.a[1]), bpf_add(bpf_pair(f.a[2], f.a[2]), acc[s])));
+                }
+            } else if (in) {
+                int o = voff + s0 * num_channels + f.ch;
+                const bpf2 a0 = bpf_pair(f.a[0], f.a[0]), a1 = bpf_pair(f.a[1], f.a[1]), a2 = bpf_pair(f.a[2], f.a[2]);
+#pragma unroll
+                for (int q = 0; q < BPF_ST / 4; ++q, o += 4 * num_channels) {
+                    if (q >= nsq) break;
+                    float x[TAPS][4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int k = 0; k < TAPS; ++k)
+                            x[k][j] = bpf_ldg(A.sino + (o + j * num_channels + k), on[k] && 4 * q + j < ns);
+                    if (A.wts) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+#pragma unroll
+                            for (int k = 0; k < TAPS; ++k)
+                                x[k][j] *= bpf_ldg(A.wts + (o + j * num_channels + k), on[k] && 4 * q + j < ns);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        bpf2 a = acc[2 * q + h];
+                        if constexpr (!TWO) a = bpf_fma(a2, bpf_pair(x[TAPS - 1][2 * h], x[TAPS - 1][2 * h + 1]), a);
+                        a = bpf_fma(a1, bpf_pair(x[1][2 * h], x[1][2 * h + 1]), a);
+                        acc[2 * q + h] = bpf_fma(a0, bpf_pair(x[0][2 * h], x[0][2 * h + 1]), a);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    bpf_write(A, acc, bad, bad, p, active, split, s0, ns, err);
+}
+
+// Shared memory of one warp, in floats: window(s) and barriers (of a call with a transposed copy), row buffer; a multiple
+// of the 128 bytes a TMA destination is aligned to.
+__host__ __device__ constexpr int bpf_warp_floats(int kind, bool tr) {
+    const int rows = kind == MBX_GEOM_PARALLEL ? 0 : 4 * BPF_FAN_QUADS * 32;
+    return rows + (tr ? (kind == MBX_GEOM_PARALLEL ? 2 * BPF_WIN_PARALLEL : BPF_WIN_FAN) + 32 : 0);
 }
 
 // CTAs of two warps: a warp whose pixels span a wide window takes longer, and holds back only one other.  Resident
 // CTAs per SM the kernels are compiled for (112 and 128 registers).
 constexpr int BPF_LAUNCH_WARPS = 2;
 __host__ __device__ constexpr int bpf_min_blocks(int kind) { return kind == MBX_GEOM_PARALLEL ? 9 : 8; }
+// Without windows: CTAs of four warps on neighbouring pixels, which share lines in L1 (128 registers, 4 resident).  Cone
+// 200 x 100 x 200 subset of 4, 256 x 128 x 256 subset of 8: 470 and 604 us, in CTAs of two 491 and 598, of eight 508 and 705.
+constexpr int BPF_DIRECT_WARPS = 4;
+__host__ __device__ constexpr int bpf_launch_warps(bool tr) { return tr ? BPF_LAUNCH_WARPS : BPF_DIRECT_WARPS; }
 
 // Unit u of a call: the 8 units of plan tile (bx, by) are its npg pixel groups x nsl slice tiles.
 template <int KIND, bool TR>
@@ -956,29 +1050,35 @@ __device__ __forceinline__ void bp_fast_run(const BpArgs &A, const CUtensorMap *
     const int by = tile / P.gx, bx = tile - by * P.gx;
     const int pg = w / P.nsl;
     const int group = bx * P.npg + pg, st = by * P.nsl + (w - pg * P.nsl);
+    auto unit = [&](auto two) {
+        if constexpr (TR)
+            bp_fast_unit<KIND, decltype(two)::value>(A, tmap, group, st, split, smw, pipe, err);
+        else
+            bp_direct_unit<KIND, decltype(two)::value>(A, group, st, split, smw, err);
+    };
     if constexpr (KIND == MBX_GEOM_PARALLEL) {
         // voxels no wider than a channel: two taps per footprint
         if (A.g.delta_voxel * (1.0f / A.g.delta_det_channel) <= 1.0f) {
-            bp_fast_unit<KIND, TR, true>(A, tmap, group, st, split, smw, pipe, err);
+            unit(std::true_type{});
             return;
         }
     }
-    bp_fast_unit<KIND, TR, false>(A, tmap, group, st, split, smw, pipe, err);
+    unit(std::false_type{});
 }
 
 template <int KIND, bool TR>
-__global__ void __launch_bounds__(32 * BPF_LAUNCH_WARPS, bpf_min_blocks(KIND))
+__global__ void __launch_bounds__(32 * bpf_launch_warps(TR), TR ? bpf_min_blocks(KIND) : 4)
 bp_fast_kernel(const BpArgs args, const __grid_constant__ CUtensorMap map, int *err) {
     extern __shared__ __align__(128) float smf[];
     const int warp = threadIdx.x >> 5;
-    const int unit = blockIdx.x * BPF_LAUNCH_WARPS + warp;
-    float *smw = smf + warp * bpf_warp_floats(KIND);
+    const int unit = blockIdx.x * bpf_launch_warps(TR) + warp;
+    float *smw = smf + warp * bpf_warp_floats(KIND, TR);
     BpfPipe pipe = {0, 0, false};
-    if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND) - 32);
+    if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND, TR) - 32);
     bp_fast_run<KIND, TR>(args, TR ? &map : nullptr, unit >> 3, unit & 7, blockIdx.y, smw, pipe, err);
 }
 
-inline size_t bpf_smem_bytes(int kind, int warps) { return 4 * (size_t)warps * bpf_warp_floats(kind); }
+inline size_t bpf_smem_bytes(int kind, int warps, bool tr) { return 4 * (size_t)warps * bpf_warp_floats(kind, tr); }
 
 // Transposed copy of a call's views (of every view of the geometry when the call selects more, that is repeats
 // some): per view, channel outermost with BPF_EDGE channels of zeros on either side, rows padded to a multiple of 4
@@ -1114,9 +1214,41 @@ inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_vie
     }
     pl.views_per_split = ceil_div(num_views_sel, splits);
     pl.splits = ceil_div(num_views_sel, pl.views_per_split);
-    pl.smem = bpf_smem_bytes(g.kind, BPF_LAUNCH_WARPS);
+    pl.smem = bpf_smem_bytes(g.kind, BPF_LAUNCH_WARPS, true);
     pl.workspace = pl.splits > 1 ? align256((size_t)pl.splits * num_pixels * S * 4) : 0;
     return pl;
+}
+
+// Whether a call's back projection reads windows of a transposed copy of its views, given the plan it would have.  The copy
+// and a warp's windows are paid once per view and serve 32 pixels x the slices of a tile, so small calls, lists that spread
+// a warp over more channels than a window has, and calls whose warps make less than about a wave (which then take as long as
+// the warp with the most windows) read their taps from the sinogram itself: the fan geometries by bp_direct_unit (the same
+// sums in the same order), parallel beam by bp_gather.cuh.  A batch fills the chip with its scans, and always takes windows.
+// Lines measured on 300 calls; us without / with windows:
+//  * parallel, slices: 13, every pixel 70 / 107; 9, subset of 4 109 / 168; 25 70 / 89;
+//    density: 35 slices, subset of 8 29 / 38; 60 slices, subset of 8 97 / 102; then by voxels x views:
+//    dense lists 59 M 95 / 103, 71 M 88 / 78, 130 M 129 / 128; subsets of 4 10 M 26 / 37, 83 M 101 / 109,
+//    131 M 149 / 192, 174 M 238 / 212, 322 M 405 / 370; under 0.7 waves 268 M 259 / 378, 125 M 105 / 130.
+//  * cone: under a wave 464 M 1183 / 2050, 116 M 339 / 594, 742 M 1833 / 2145, but whole grids, whose warps seldom lie
+//    across two rows' ends, 377 M 958 / 765, 452 M 1428 / 1203, 178 M 461 / 488; up to two waves 271 M 697 / 626,
+//    135 M 524 / 328, 228 M 584 / 661; from three 418 M 1164 / 866, 544 M 1610 / 1061; by voxels x views 45 M 153 / 144,
+//    66 M 208 / 240, 101 M 322 / 333, 111 M 298 / 337, 117 M 376 / 300; subset of 32 144 M 472 / 671, of 16
+//    304 M 1021 / 893.
+//  * translation, whose magnification differs from grid row to grid row: every pixel 23 M 64 / 65, 29 M 91 / 88,
+//    39 M 121 / 108, 153 M 408 / 370; half of them 132 M 305 / 574.
+constexpr int BPF_FEW_SLICES = 27;
+inline bool bp_windows(const mbx_geom &g, const BpfPlan &pl, long long num_pixels, int num_views_sel) {
+    const double grid = (double)g.num_recon_rows * g.num_recon_cols, dense = (double)num_pixels / grid;
+    const double work = (double)num_pixels * g.num_recon_slices * num_views_sel * 1e-6;
+    const double waves = (double)pl.gx * pl.gy * pl.splits * BPF_WARPS /
+                         ((double)bpf_min_blocks(g.kind) * BPF_LAUNCH_WARPS * num_sms());
+    switch (g.kind) {
+        case MBX_GEOM_PARALLEL:
+            return g.num_recon_slices >= BPF_FEW_SLICES && dense >= 1.0 / 7 && work >= (dense >= 0.375 ? 48 : 160) &&
+                   waves >= 0.7;
+        case MBX_GEOM_CONE: return work >= 112 && dense >= 1.0 / 24 && (waves >= 1.05 || dense > 0.9);
+        default: return work >= 28 && dense > 0.5;
+    }
 }
 
 }  // namespace mbx

@@ -1,5 +1,5 @@
 // Parallel-beam back projection that gathers its taps from global memory (psf_radius == 1): the better kernel where a
-// window of the view (bp_fast.cuh) costs more than it saves, for lists and recons that bp_gathers() names.
+// window of the view (bp_fast.cuh) costs more than it saves, for lists and recons that bp_windows() leaves out.
 //
 // CTA = 256 threads = 8 warps; lanes run along 32 pixels, warps along slice tiles of at most BPG_ST slices, accumulators
 // in registers across all views.  A thread reads three taps per slice at constant offsets from one 32-bit element offset.
@@ -22,23 +22,10 @@ struct BpgPlan {
     size_t workspace;
 };
 
-// Whether a parallel-beam call with values takes this kernel.  A window is copied once per warp and view and serves 32
-// pixels x the slices of a tile: with few slices the copy is not paid back, and a list that holds few of its grid's
-// pixels (a subset of 8 holds a tenth) spreads a warp over more channels than a window has.  Measured (calls of 60 to 660
-// views, us, gathers / windows): 13 slices, every pixel 70 / 107; 9 slices, subset of 4 109 / 168; 25 slices 70 / 89;
-// 35 slices, subset of 8 29 / 38; 60 slices, subset of 8 97 / 102; against 28 slices, subset of 4 155 / 151; 34 slices,
-// every pixel 75 / 69; 57 slices, subset of 4 (437 channels) 1724 / 895.
-constexpr int BPG_FEW_SLICES = 27;
-constexpr int BPG_SPARSE = 7;  // a list of fewer than 1 / this of the grid's pixels
-inline bool bp_gathers(const mbx_geom &g, long long num_pixels, bool values) {
-    return g.kind == MBX_GEOM_PARALLEL && values &&
-           (g.num_recon_slices < BPG_FEW_SLICES ||
-            num_pixels * BPG_SPARSE < (long long)g.num_recon_rows * g.num_recon_cols);
-}
-
 // For geometries that plan_bp_fast admits.  Views are split over CTAs when there are fewer than two per SM; the partial
-// sums of the splits then hold at most 592 CTAs' accumulators (9.7 MB).
-inline BpgPlan plan_bp_gather(const mbx_geom &g, long long num_pixels, int num_views_sel) {
+// sums of the splits then hold at most 592 CTAs' accumulators (9.7 MB).  splits > 0: that many instead (of a call that
+// stands in for one with windows: the same sums in the same order).
+inline BpgPlan plan_bp_gather(const mbx_geom &g, long long num_pixels, int num_views_sel, int splits_of = 0) {
     BpgPlan pl;
     const int S = g.num_recon_slices;
     // the fewest tiles, rounded up to a power of two (at most 8) or a multiple of 8, then the slices spread evenly
@@ -60,7 +47,9 @@ inline BpgPlan plan_bp_gather(const mbx_geom &g, long long num_pixels, int num_v
     pl.gy = ceil_div(tiles, pl.nsl);
     const long long base = (long long)pl.gx * pl.gy, want = 2LL * num_sms();
     long long splits = 1;
-    if (base < want && num_views_sel >= 16)
+    if (splits_of > 0)
+        splits = splits_of;
+    else if (base < want && num_views_sel >= 16)
         splits = std::max(1LL, std::min({(want + base - 1) / base, (long long)num_views_sel / 8, 64LL}));
     pl.views_per_split = ceil_div(num_views_sel, splits);
     pl.splits = ceil_div(num_views_sel, pl.views_per_split);

@@ -37,9 +37,9 @@ template <int KIND, bool TR>
 __global__ void __launch_bounds__(32 * BPF_LAUNCH_WARPS, 8)
 b_bp(ProjList L, int num_scans, int step, int first, int total, int *err) {
     extern __shared__ __align__(128) float smb[];
-    float *smw = smb + (threadIdx.x >> 5) * bpf_warp_floats(KIND);
+    float *smw = smb + (threadIdx.x >> 5) * bpf_warp_floats(KIND, TR);
     BpfPipe pipe = {0, 0, false};
-    if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND) - 32);
+    if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND, TR) - 32);
     const CUtensorMap *acquired = nullptr;  // the map this warp copies through
     for (;;) {
         int u = 0;
@@ -934,7 +934,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     int *hbox_first = reinterpret_cast<int *>(host.data() + L.box_first);
     int *o_el = hoff, *o_sn = hoff + n1, *o_rc = hoff + 2 * n1, *o_flt = hoff + 3 * n1, *o_tr = hoff + 4 * n1;
     // the tensor maps of every scan's back projections; the TMA reads maps from 64-byte boundaries only, so in a
-    // workspace that starts off one the windows are copied by loads
+    // workspace that starts off one the taps are read from the sinograms
     bool transposed = L.transposed && (reinterpret_cast<uintptr_t>(base + L.maps) & 63) == 0;
     for (int m = 0; m < SW_COUNT * n && transposed; ++m) {
         const int s = m / SW_COUNT, boxq = scan_window_box(zs[s], m % SW_COUNT);
@@ -1091,7 +1091,9 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
             ord[s] = s;
             const ScanSizes &z = zs[s];
             const bool fp = w == PL_FP || w == PL_INIT_FP || w == PL_BUILD;
-            const size_t sm = fp ? (w == PL_INIT_FP ? z.ifp : z.fpp).walk.smem : bpf_smem_bytes(scans[s].geom.kind, BPF_LAUNCH_WARPS);
+            const bool tr = w == PL_HESS ? hess_transposed : transposed;
+            const size_t sm = fp ? (w == PL_INIT_FP ? z.ifp : z.fpp).walk.smem
+                                 : bpf_smem_bytes(scans[s].geom.kind, BPF_LAUNCH_WARPS, tr);
             pl_smem[w] = std::max(pl_smem[w], sm);
         }
         std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return cost[a] > cost[b]; });
