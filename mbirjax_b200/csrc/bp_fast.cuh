@@ -885,8 +885,10 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
 }
 
 // The same unit without a transposed copy to take windows of (calls whose scratch holds none, or that project ones): each
-// lane reads its taps from the sinogram itself, for the fan geometries each detector row once, four rows in flight, into
-// its column of the row buffer.  Bound by the load/store pipe and the latency of the gathers.  Measured where windows copied
+// lane reads its taps from the sinogram itself: for parallel beam those of 16 slices (8 with three taps) in flight together
+// (4 scans of 180 x 20 x 200 in 4 subsets, a batch's stage: 249 us with 4 slices in flight and tiles of 20, 182 so with
+// tiles of 12); for the fan geometries each detector row once, four rows in flight, into its column of the row buffer.
+// Bound by the load/store pipe and the latency of the gathers.  Measured where windows copied
 // by plain loads stood here before: cone 100 x 200 x 60 (subset of 8) 126 -> 45 us, 256 x 128 x 256 (subset of 8)
 // 1035 -> 598 us, translation 49 x 128 x 128 (subset of 4) 85 -> 42 us, unit-weight Hessian of cone 256 x 128 x 256
 // 4.66 -> 2.98 ms.
@@ -995,28 +997,29 @@ __device__ __forceinline__ void bp_direct_unit(const BpArgs &args, int pg, int s
             } else if (in) {
                 int o = voff + s0 * num_channels + f.ch;
                 const bpf2 a0 = bpf_pair(f.a[0], f.a[0]), a1 = bpf_pair(f.a[1], f.a[1]), a2 = bpf_pair(f.a[2], f.a[2]);
+                constexpr int N = TWO ? 16 : 8;  // slices whose taps are in flight together
 #pragma unroll
-                for (int q = 0; q < BPF_ST / 4; ++q, o += 4 * num_channels) {
-                    if (q >= nsq) break;
-                    float x[TAPS][4];
+                for (int c = 0; c < BPF_ST / N; ++c, o += N * num_channels) {
+                    if (c * N >= ns) break;
+                    float x[N][TAPS];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < N; ++j)
 #pragma unroll
                         for (int k = 0; k < TAPS; ++k)
-                            x[k][j] = bpf_ldg(A.sino + (o + j * num_channels + k), on[k] && 4 * q + j < ns);
+                            x[j][k] = bpf_ldg(A.sino + (o + j * num_channels + k), on[k] && c * N + j < ns);
                     if (A.wts) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
+                        for (int j = 0; j < N; ++j)
 #pragma unroll
                             for (int k = 0; k < TAPS; ++k)
-                                x[k][j] *= bpf_ldg(A.wts + (o + j * num_channels + k), on[k] && 4 * q + j < ns);
+                                x[j][k] *= bpf_ldg(A.wts + (o + j * num_channels + k), on[k] && c * N + j < ns);
                     }
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        bpf2 a = acc[2 * q + h];
-                        if constexpr (!TWO) a = bpf_fma(a2, bpf_pair(x[TAPS - 1][2 * h], x[TAPS - 1][2 * h + 1]), a);
-                        a = bpf_fma(a1, bpf_pair(x[1][2 * h], x[1][2 * h + 1]), a);
-                        acc[2 * q + h] = bpf_fma(a0, bpf_pair(x[0][2 * h], x[0][2 * h + 1]), a);
+                    for (int h = 0; h < N / 2; ++h) {
+                        bpf2 a = acc[c * N / 2 + h];
+                        if constexpr (!TWO) a = bpf_fma(a2, bpf_pair(x[2 * h][TAPS - 1], x[2 * h + 1][TAPS - 1]), a);
+                        a = bpf_fma(a1, bpf_pair(x[2 * h][1], x[2 * h + 1][1]), a);
+                        acc[c * N / 2 + h] = bpf_fma(a0, bpf_pair(x[2 * h][0], x[2 * h + 1][0]), a);
                     }
                 }
             }
@@ -1142,7 +1145,9 @@ constexpr size_t BPF_PARTIAL_BYTES = MBX_NOALLOC_SCRATCH_BYTES / 4 * 3;
 // (24 x 20 x 64 cone, subset of 4: 30 us with 8, 20 with 4, 14 with 2).
 constexpr int BPF_SPLIT_VIEWS = 2;
 
-inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_views_sel, int small = 0) {
+// most_slices > 0: tiles of at most that many slices, whatever the call's size (a batch's lists).
+inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_views_sel, int small = 0,
+                            int most_slices = 0) {
     BpfPlan pl;
     pl.inline_fp = 1;
     pl.chunk = 0;
@@ -1173,8 +1178,10 @@ inline BpfPlan plan_bp_fast(const mbx_geom &g, long long num_pixels, int num_vie
     // rows than a low tile's windows have (all pixels of 49 x 128 x 128: 121 us with 32 slices, 130 with 16, 105 with 12,
     // 132 with 8; subset of 4 of 49 x 85 x 96: 60, 46 and 41 us)
     if (g.kind == MBX_GEOM_TRANSLATION) most = std::min(most, 12);
+    if (most_slices > 0)
+        most = std::min(most, most_slices);
     // cone: tiles of half the height for calls whose units could not fill the chip (101 x 18 x 51, subset of 4: 20 -> 16)
-    if (g.kind == MBX_GEOM_CONE && (num_pixels + 31) / 32 * ceil_div(S, most) *
+    else if (g.kind == MBX_GEOM_CONE && (num_pixels + 31) / 32 * ceil_div(S, most) *
                                            std::max(1, num_views_sel / BPF_SPLIT_VIEWS) < BPF_WARPS * slots)
         most = std::min(most, BPF_ST / 2);
     pl.ts = bpf_tile_height(S, most);

@@ -454,7 +454,8 @@ struct Layout {
     std::vector<size_t> plan_off;  // per scan: its subsets' planned storage, [K][PlannedSizes::total]
     int pl_total[PL_COUNT];
     int el_total, sn_total, rc_total, flt_total, box_total, tr_total, ksum, max_npix;
-    bool setup, transposed, hess_transposed;
+    bool setup;
+    BatchBp bp;
     std::vector<size_t> buf_off;   // per scan: bp, delta, dsino, transposed copy
     std::vector<size_t> box_off;   // per scan: chunk boxes of its subsets, [K][chunks]
     std::vector<size_t> fbox_off;  // per scan: chunk boxes of its region-of-reconstruction list
@@ -478,14 +479,12 @@ static int plan_initial_fp(const mbx_scan *scans, int n, std::vector<ScanSizes> 
 static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::vector<ScanSizes> &zs,
                   int flags = 0) {
     L.plan_fp = (flags & MBX_BATCHED_PLAN_FORWARD) != 0;
-    zs.resize(n);
     for (int w = 0; w < PL_COUNT; ++w) L.pl_total[w] = 0;
     L.el_total = L.sn_total = L.rc_total = L.flt_total = L.box_total = L.tr_total = L.ksum = L.max_npix = 0;
-    L.transposed = L.hess_transposed = true;
     int kind = -1, nsetup = 0;
+    const int rc = batch_sizes(scans, n, zs, L.bp);
+    if (rc != MBX_OK) return rc;
     for (int s = 0; s < n; ++s) {
-        int rc = scan_sizes(scans[s], zs[s]);
-        if (rc != MBX_OK) return rc;
         if (kind >= 0 && scans[s].geom.kind != kind) return MBX_ERR_UNSUPPORTED;  // one geometry kind per batch
         if (scans[s].num_subsets != scans[0].num_subsets) return MBX_ERR_UNSUPPORTED;  // argument table is [scan][K]
         kind = scans[s].geom.kind;
@@ -500,11 +499,6 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
         L.rc_total += zs[s].rc_tiles;
         L.flt_total += zs[s].flt_tiles;
         L.tr_total += zs[s].tr_tiles;
-        // every scan's copy has to be addressable (32-bit offsets); the Hessian's needs weights to copy
-        const mbx_geom &g = scans[s].geom;
-        if ((long long)g.num_views * (g.num_det_channels + 2 * BPF_EDGE) * bpf_padded_rows(g) >= (1LL << 31))
-            L.transposed = false;
-        if (!scans[s].weights) L.hess_transposed = false;
         L.ksum += scans[s].num_subsets;
         L.box_total += scans[s].num_subsets * (int)((scans[s].subset_size + CB_CHUNK - 1) / CB_CHUNK);
         L.max_npix = std::max<int>(L.max_npix, (int)zs[s].npix);
@@ -512,7 +506,7 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
     }
     if (nsetup != 0 && nsetup != n) return MBX_ERR_INVALID_ARG;  // set-up inputs for every scan or for none
     L.setup = nsetup == n;
-    L.hess_transposed = L.hess_transposed && L.transposed;
+    const bool copies = L.bp.windows[SW_SUBSET] || (L.setup && (L.bp.windows[SW_INIT] || L.bp.windows[SW_HESS]));
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += align256(bytes); return o; };
     L.scans = take(sizeof(VcdScan) * n);
@@ -547,7 +541,7 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
         L.buf_off[4 * s] = take(4 * (size_t)zs[s].ncyl);
         L.buf_off[4 * s + 1] = take(4 * (size_t)zs[s].ncyl);
         L.buf_off[4 * s + 2] = take(4 * (size_t)zs[s].nsino);
-        L.buf_off[4 * s + 3] = take(L.transposed ? bpf_transposed_bytes(scans[s].geom, scans[s].geom.num_views) : 0);
+        L.buf_off[4 * s + 3] = take(copies ? bpf_transposed_bytes(scans[s].geom, scans[s].geom.num_views) : 0);
     }
     L.box_off.resize(n);
     L.fbox_off.assign(n, 0);
@@ -647,6 +641,8 @@ static void launch_bp_kernel(int kind, int grid, size_t smem, cudaStream_t st, c
         b_bp<MBX_GEOM_TRANSLATION, TR><<<grid, T, smem, st>>>(L, n, step, 0, total, err);
 }
 
+static int bp_of_list(int which) { return which == PL_BP ? SW_SUBSET : which == PL_INIT_BP ? SW_INIT : SW_HESS; }
+
 // One launch of a back-projection work list (resets the list's counter first), after the transposed copies of what it
 // projects.
 static cudaError_t launch_bp_list(const BatchedPlanHost &P, int which, int step, cudaStream_t st) {
@@ -654,7 +650,7 @@ static cudaError_t launch_bp_list(const BatchedPlanHost &P, int which, int step,
     L.stride = which == PL_BP ? P.ksum / P.num_scans : 1;
     cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    const bool tr = which == PL_HESS ? P.hess_transposed : P.transposed;
+    const bool tr = P.windows[bp_of_list(which)];
     if (tr) {
         b_transpose<<<P.tr_grid, 256, 0, st>>>(P.t, P.num_scans, P.tr_total,
                                                which == PL_BP ? 0 : which == PL_INIT_BP ? 1 : 2);
@@ -935,16 +931,17 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     int *o_el = hoff, *o_sn = hoff + n1, *o_rc = hoff + 2 * n1, *o_flt = hoff + 3 * n1, *o_tr = hoff + 4 * n1;
     // the tensor maps of every scan's back projections; the TMA reads maps from 64-byte boundaries only, so in a
     // workspace that starts off one the taps are read from the sinograms
-    bool transposed = L.transposed && (reinterpret_cast<uintptr_t>(base + L.maps) & 63) == 0;
-    for (int m = 0; m < SW_COUNT * n && transposed; ++m) {
-        const int s = m / SW_COUNT, boxq = scan_window_box(zs[s], m % SW_COUNT);
+    bool mapped = (reinterpret_cast<uintptr_t>(base + L.maps) & 63) == 0;
+    for (int m = 0; m < SW_COUNT * n && mapped; ++m) {
+        const int s = m / SW_COUNT, boxq = scan_window_box(zs[s], m % SW_COUNT, L.bp);
         if (boxq == 0) continue;
         CUtensorMap map = {};
-        transposed = bpf_window_map(map, reinterpret_cast<const float *>(base + L.buf_off[4 * s + 3]), scans[s].geom,
+        mapped = bpf_window_map(map, reinterpret_cast<const float *>(base + L.buf_off[4 * s + 3]), scans[s].geom,
                                     scans[s].geom.num_views, boxq);
         std::memcpy(host.data() + L.maps + sizeof(map) * m, &map, sizeof(map));
     }
-    const bool hess_transposed = transposed && L.hess_transposed;
+    bool windows[SW_COUNT];
+    for (int w = 0; w < SW_COUNT; ++w) windows[w] = mapped && L.bp.windows[w];
     fill_params(scans, n, reinterpret_cast<float *>(host.data() + L.fm), reinterpret_cast<QParams *>(host.data() + L.qp));
     o_el[0] = o_sn[0] = o_rc[0] = o_flt[0] = o_tr[0] = 0;
     hbox_first[0] = 0;
@@ -983,12 +980,13 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         v.bp = reinterpret_cast<float *>(base + L.buf_off[4 * s]);
         v.delta = reinterpret_cast<float *>(base + L.buf_off[4 * s + 1]);
         v.dsino = reinterpret_cast<float *>(base + L.buf_off[4 * s + 2]);
-        v.tsino = transposed ? reinterpret_cast<float *>(base + L.buf_off[4 * s + 3]) : nullptr;
+        v.tsino = reinterpret_cast<float *>(base + L.buf_off[4 * s + 3]);  // (of no size when nothing reads windows)
         v.V = g.num_views;
         v.R = g.num_det_rows;
         v.C = g.num_det_channels;
         v.rp = bpf_padded_rows(g);
         auto window_source = [&](BpArgs &a, int which) {  // the scan's transposed copy
+            if (!windows[which]) return;
             a.tsino = v.tsino;
             a.rp = v.rp;
             a.tsino_all = 1;
@@ -1006,7 +1004,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
             const int32_t *pix = sc.partition + (size_t)k * sc.subset_size;
             hb[ki] = bp_args(g, sc.error_sinogram, sc.weights, pix, sc.subset_size, 1, v.bp, 0,
                              scan_bp_plan(z, SW_SUBSET));
-            if (transposed) window_source(hb[ki], SW_SUBSET);
+            window_source(hb[ki], SW_SUBSET);
             if (sc.partition_order) hb[ki].order = sc.partition_order + (size_t)k * sc.subset_size;
             FpArgs &f = hf[ki];
             std::memset(&f, 0, sizeof(f));
@@ -1059,8 +1057,8 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
                              reinterpret_cast<const int32_t *>(base + L.arange), z.npix, 2,
                              const_cast<float *>(sc.fm_hessian), 0, scan_bp_plan(z, SW_HESS));
             hhb[s].out_slices = z.hbp_slices;
-            if (transposed) window_source(hib[s], SW_INIT);
-            if (hess_transposed) window_source(hhb[s], SW_HESS);
+            window_source(hib[s], SW_INIT);
+            window_source(hhb[s], SW_HESS);
             FiltScan &fl = hfl[s];
             fl.in = sc.sinogram;
             fl.out = sc.error_sinogram;
@@ -1091,7 +1089,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
             ord[s] = s;
             const ScanSizes &z = zs[s];
             const bool fp = w == PL_FP || w == PL_INIT_FP || w == PL_BUILD;
-            const bool tr = w == PL_HESS ? hess_transposed : transposed;
+            const bool tr = !fp && windows[bp_of_list(w)];
             const size_t sm = fp ? (w == PL_INIT_FP ? z.ifp : z.fpp).walk.smem
                                  : bpf_smem_bytes(scans[s].geom.kind, BPF_LAUNCH_WARPS, tr);
             pl_smem[w] = std::max(pl_smem[w], sm);
@@ -1170,8 +1168,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     P.flt_total = L.flt_total;
     P.box_total = L.box_total;
     P.tr_total = L.tr_total;
-    P.transposed = transposed ? 1 : 0;
-    P.hess_transposed = hess_transposed ? 1 : 0;
+    for (int w = 0; w < SW_COUNT; ++w) P.windows[w] = windows[w] ? 1 : 0;
     P.fp_minb = 2;
     P.init_minb = init_minb;
     size_t flt_smem = 0;
@@ -1192,11 +1189,12 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
     }
     if (e == cudaSuccess) e = set_max_dynamic_smem(reinterpret_cast<const void *>(b_filter), 200 * 1024);
     if (e != cudaSuccess) return set_cuda_error(e);
-    P.pl_grid[PL_BP] = bp_grid(P.kind, transposed, P.pl_smem[PL_BP], P.pl_total[PL_BP]);
+    P.pl_grid[PL_BP] = bp_grid(P.kind, windows[SW_SUBSET], P.pl_smem[PL_BP], P.pl_total[PL_BP]);
     P.pl_grid[PL_FP] = fp_grid(P.kind, 2, P.pl_smem[PL_FP], P.pl_total[PL_FP]);
-    P.pl_grid[PL_INIT_BP] = bp_grid(P.kind, transposed, P.pl_smem[PL_INIT_BP], std::max(1, P.pl_total[PL_INIT_BP]));
+    P.pl_grid[PL_INIT_BP] =
+        bp_grid(P.kind, windows[SW_INIT], P.pl_smem[PL_INIT_BP], std::max(1, P.pl_total[PL_INIT_BP]));
     P.pl_grid[PL_INIT_FP] = fp_grid(P.kind, P.init_minb, P.pl_smem[PL_INIT_FP], std::max(1, P.pl_total[PL_INIT_FP]));
-    P.pl_grid[PL_HESS] = bp_grid(P.kind, hess_transposed, P.pl_smem[PL_HESS], std::max(1, P.pl_total[PL_HESS]));
+    P.pl_grid[PL_HESS] = bp_grid(P.kind, windows[SW_HESS], P.pl_smem[PL_HESS], std::max(1, P.pl_total[PL_HESS]));
     {   // load every stage kernel now (lazy module loading must not happen inside a stream capture)
         cudaFuncAttributes fa;
         const void *ks[] = {reinterpret_cast<const void *>(b_delta), reinterpret_cast<const void *>(b_linquad),

@@ -3,6 +3,8 @@
 // (b_fp_parallel.cu, b_fp_cone.cu, b_fp_translation.cu) for build parallelism.
 #pragma once
 
+#include <vector>
+
 #include "back_project.cuh"
 #include "bp_fast.cuh"
 #include "direct_filter.cuh"
@@ -96,8 +98,7 @@ struct BatchedPlanHost {
     size_t pl_smem[PL_COUNT];
     int el_total, sn_total, rc_total, flt_total, box_total, tr_total;
     int el_grid, sn_grid, rc_grid, flt_grid, box_grid, tr_grid;
-    int transposed;       // the back projections read transposed copies (PL_HESS: when hess_transposed)
-    int hess_transposed;
+    int windows[3];       // by back projection (SW_SUBSET, SW_INIT, SW_HESS): reads windows of transposed copies
     size_t flt_smem;
     int init_minb;  // b_fp variant of the initial projection: cb_many for parallel beam, else 2
     int fp_minb;  // b_fp variant of the subset stage: 2 or cb_many resident CTAs per SM
@@ -187,14 +188,24 @@ struct ScanSizes {
     int tr_tiles; // 32-channel blocks of the transposed copy over all views
 };
 
-inline int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
+// The back projections of a scan: of a subset, of the region of reconstruction (from the filtered sinogram), of every pixel
+// (the Hessian).
+enum { SW_SUBSET = 0, SW_INIT, SW_HESS, SW_COUNT };
+
+// How a batch runs them, by list: whether they read windows of transposed copies, and the most slices of a tile.
+struct BatchBp {
+    bool windows[SW_COUNT];
+    int most[SW_COUNT];
+};
+
+inline int scan_sizes(const mbx_scan &sc, ScanSizes &z, const BatchBp &B) {
     const mbx_geom &g = sc.geom;
     int rc = validate_geom(&g);
     if (rc != MBX_OK) return rc;
     if (!sc.flat_recon || !sc.error_sinogram || !sc.fm_hessian || !sc.partition) return MBX_ERR_INVALID_ARG;
     if (sc.num_subsets <= 0 || sc.subset_size <= 0) return MBX_ERR_INVALID_ARG;
     if (!(sc.qp.sigma_x > 0.0f) || !(sc.qp.T > 0.0f) || !(sc.qp.p > 0.0f)) return MBX_ERR_INVALID_ARG;
-    z.bpp = plan_bp_fast(g, sc.subset_size, g.num_views);
+    z.bpp = plan_bp_fast(g, sc.subset_size, g.num_views, 0, B.most[SW_SUBSET]);
     // the channel blocks of either kernel variant (the tuner keeps the faster): the second's are the narrower
     z.fpp = plan_fp_cb(g, 0, 0, 2, cb_many(g.kind) >= 4 ? CB_MANY_CHANNELS : 128, 0, MBX_BATCHED_FP_CAP);
     z.ifp = z.fpp;
@@ -218,15 +229,15 @@ inline int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
         if (z.npix > (1 << 24) || z.nrecon >= (1LL << 31)) return MBX_ERR_UNSUPPORTED;
         z.hbp_slices = 0;
         if (bp_unit_broadcast(g, nullptr, sc.weights)) {  // unit-weight parallel Hessian: one slice, broadcast
-            z.hbp = plan_bp_fast(one_slice_geometry(g), z.npix, g.num_views);
+            z.hbp = plan_bp_fast(one_slice_geometry(g), z.npix, g.num_views, 0, B.most[SW_HESS]);
             if (z.hbp.ok && z.hbp.splits == 1) z.hbp_slices = g.num_recon_slices;
         }
-        if (z.hbp_slices == 0) z.hbp = plan_bp_fast(g, z.npix, g.num_views);
+        if (z.hbp_slices == 0) z.hbp = plan_bp_fast(g, z.npix, g.num_views, 0, B.most[SW_HESS]);
         if (!z.hbp.ok) return MBX_ERR_UNSUPPORTED;
         if (g.kind != MBX_GEOM_TRANSLATION) {  // translation geometry starts from zeros (no direct recon)
             if (!filter_admits(g.num_det_channels, g.kind != MBX_GEOM_PARALLEL))
                 return MBX_ERR_UNSUPPORTED;
-            z.ibp = plan_bp_fast(g, sc.num_full_indices, g.num_views);
+            z.ibp = plan_bp_fast(g, sc.num_full_indices, g.num_views, 0, B.most[SW_INIT]);
             if (!z.ibp.ok) return MBX_ERR_UNSUPPORTED;
             z.flt_tiles = ceil_div((long long)g.num_views * g.num_det_rows, filter_shape(g.num_det_channels).rows);
         } else {
@@ -236,15 +247,69 @@ inline int scan_sizes(const mbx_scan &sc, ScanSizes &z) {
     return MBX_OK;
 }
 
-// The back projections of a scan.  The height of a list's slice tiles, and so of its windows, can follow its pixel count
-// (cone: plan_bp_fast), so each has a tensor map of its own, whose box holds the rows that its plan waits for.
-enum { SW_SUBSET = 0, SW_INIT, SW_HESS, SW_COUNT };
+// Each back projection of a scan has a tensor map of its own, whose box holds the rows that its plan waits for: the height
+// of its slice tiles, and so of its windows, follows its list.
 inline const BpfPlan &scan_bp_plan(const ScanSizes &z, int which) {
     return which == SW_SUBSET ? z.bpp : which == SW_INIT ? z.ibp : z.hbp;
 }
-// Rows of the box of that map, in fours (0: the scan has no such back projection).
-inline int scan_window_box(const ScanSizes &z, int which) {
-    return which == SW_SUBSET || z.setup ? scan_bp_plan(z, which).boxq : 0;
+// Rows of the box of that map, in fours (0: no windows, or the scan has no such back projection).
+inline int scan_window_box(const ScanSizes &z, int which, const BatchBp &B) {
+    return B.windows[which] && (which == SW_SUBSET || z.setup) ? scan_bp_plan(z, which).boxq : 0;
+}
+
+// Sizes of every scan, and how the batch runs its back projections.  A unit's views follow one another, so a list whose
+// units make less than about two waves of the chip's warps takes as long as one or two units: it reads its taps from the
+// sinograms, in tiles as low (down to 8 slices) as still make one wave.  Stage of one step, us, gathering kernel of 16-slice
+// tiles / windows / taps from the sinograms, 4 scans unless said: parallel 180 x 5 x 200 in 4 subsets (0.4 waves)
+// 186 / 231 / 122, 360 x 64 x 300 in 8 (0.9) 1512 / 876 / 718, 16 scans of 360 x 28 x 300 in 8 (1.6) 2157 / 1336 / 1150,
+// 360 x 28 x 437 in 4 (1.9) 2020 / 1123 / 1303, 16 scans of 180 x 40 x 200 in 4 (2.7) 884 / 630 / 768; cone 100 x 200 x 60
+// in 8 (0.2) 510 / 798 / 189, 16 scans of 200 x 40 x 160 in 4 (1.6) 2540 / 1438 / 1397.  Translation geometry: as bp_windows.
+constexpr double BATCH_WINDOW_WAVES = 1.75;
+inline int batch_sizes(const mbx_scan *scans, int n, std::vector<ScanSizes> &zs, BatchBp &B) {
+    const double slots = 8.0 * BPF_LAUNCH_WARPS * num_sms();
+    for (int w = 0; w < SW_COUNT; ++w) {
+        B.windows[w] = true;
+        B.most[w] = BPF_ST;
+    }
+    zs.assign(n, ScanSizes{});
+    auto plan = [&]() {
+        for (int s = 0; s < n; ++s) {
+            const int rc = scan_sizes(scans[s], zs[s], B);
+            if (rc != MBX_OK) return rc;
+        }
+        return (int)MBX_OK;
+    };
+    auto waves = [&](int w) {
+        double units = 0.0;
+        for (int s = 0; s < n; ++s) {
+            const BpfPlan &p = scan_bp_plan(zs[s], w);
+            if (w != SW_SUBSET && !zs[s].setup) return 1e9;
+            units += (double)p.gx * p.gy * BPF_WARPS;
+        }
+        return units / slots;
+    };
+    int rc = plan();
+    for (int w = 0; w < SW_COUNT && rc == MBX_OK; ++w) {
+        B.windows[w] = waves(w) >= BATCH_WINDOW_WAVES;
+        for (int s = 0; s < n; ++s) {
+            if (scans[s].geom.kind == MBX_GEOM_TRANSLATION && w == SW_SUBSET && 2 * scans[s].subset_size <= zs[s].npix)
+                B.windows[w] = false;
+            // every copy has to be addressable (32-bit offsets); the Hessian's needs weights to copy
+            const mbx_geom &g = scans[s].geom;
+            if ((long long)g.num_views * (g.num_det_channels + 2 * BPF_EDGE) * bpf_padded_rows(g) >= (1LL << 31) ||
+                (w == SW_HESS && !scans[s].weights))
+                B.windows[w] = false;
+        }
+        while (rc == MBX_OK && !B.windows[w] && B.most[w] > 8) {
+            B.most[w] /= 2;
+            rc = plan();
+            if (rc != MBX_OK || waves(w) <= 1.1) continue;
+            B.most[w] *= 2;  // too many for a wave
+            rc = plan();
+            break;
+        }
+    }
+    return rc;
 }
 
 // The forward-projection stage kernels of one geometry kind: b_fp (walk), b_fp_replay (stored passes) and

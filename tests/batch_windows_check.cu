@@ -1,7 +1,8 @@
-// Host-only check of what a batch prepares for its back projections (vcd_batched.cuh): for a sweep of scans, the box of
-// each back projection's tensor map has the rows of that back projection's own plan, since a copy waits for as many bytes
-// as its plan's windows hold; printing "ok <scans> <scans whose plans differ>" or the first failure.  Runs on the CPU (no
-// device call).
+// Host-only check of what a batch prepares for its back projections (vcd_batched.cuh), for a sweep of batches: a back
+// projection that reads windows copies them through a map whose box has the rows of its own plan, since a copy waits for as
+// many bytes as its plan's windows hold; one that does not has no map; the tiles are no higher than the batch says and cover
+// the slices; and windows are read where the list fills the chip.  Prints "ok <scans> <scans whose plans differ> <batches
+// with windows> <without>" or the first failure.  Runs on the CPU (no device call).
 #include <cmath>
 #include <cstdio>
 
@@ -43,27 +44,48 @@ static mbx_scan make_scan(int kind, int V, int R, int C, int K, bool weighted) {
 }
 
 int main() {
-    long scans = 0, differ = 0;
+    long checked = 0, differ = 0, with = 0, without = 0;
     for (int kind : {MBX_GEOM_PARALLEL, MBX_GEOM_CONE, MBX_GEOM_TRANSLATION})
         for (int C : {48, 64, 96, 128, 192, 256})
-            for (int R : {4, 16, 17, 24, 32, 40, 64, 100, 128})
-                for (int V : {24, 60, 128, 180, 256})
-                    for (int K : {1, 2, 4, 8, 16})
-                        for (int weighted = 0; weighted < 2; ++weighted) {
-                            ScanSizes z = {};
-                            if (scan_sizes(make_scan(kind, V, R, C, K, weighted != 0), z) != MBX_OK) continue;
-                            ++scans;
-                            bool same = true;
-                            for (int w = 0; w < SW_COUNT; ++w) {
-                                if (scan_window_box(z, w) != scan_bp_plan(z, w).boxq) {
-                                    std::printf("FAIL map %d of kind %d, %d x %d x %d in %d: box %d, plan %d\n", w, kind, V,
-                                                R, C, K, scan_window_box(z, w), scan_bp_plan(z, w).boxq);
+            for (int R : {1, 4, 16, 17, 24, 32, 40, 64, 100, 128})
+                for (int V : {24, 60, 180})
+                    for (int K : {1, 2, 4, 16})
+                        for (int n : {1, 3, 20})
+                            for (int weighted = 0; weighted < 3; ++weighted) {  // 2: some scans of the batch
+                                std::vector<mbx_scan> scans;
+                                for (int s = 0; s < n; ++s)
+                                    scans.push_back(make_scan(kind, V, R + s % 3, C + s, K, weighted == 1 || (weighted == 2 && s % 2)));
+                                std::vector<ScanSizes> zs;
+                                BatchBp B;
+                                if (batch_sizes(scans.data(), n, zs, B) != MBX_OK) continue;
+                                double units[SW_COUNT] = {};
+                                auto fail = [&](const char *what, int w) {
+                                    std::printf("FAIL %s: list %d of kind %d, %d scans of %d x %d x %d in %d\n", what, w,
+                                                kind, n, V, R, C, K);
                                     return 1;
+                                };
+                                for (int s = 0; s < n; ++s) {
+                                    bool same = true;
+                                    ++checked;
+                                    for (int w = 0; w < SW_COUNT; ++w) {
+                                        const BpfPlan &p = scan_bp_plan(zs[s], w);
+                                        if (kind == MBX_GEOM_TRANSLATION && w == SW_INIT) continue;  // (has none)
+                                        if (scan_window_box(zs[s], w, B) != (B.windows[w] ? p.boxq : 0)) return fail("box", w);
+                                        if (p.ts > B.most[w] || p.ts % 4 || p.ts * p.tiles < (zs[s].hbp_slices > 0 && w == SW_HESS ? 1 : R + s % 3))
+                                            return fail("tiles", w);
+                                        if (B.windows[w] && w == SW_HESS && !scans[s].weights) return fail("Hessian without weights", w);
+                                        if (B.windows[w] && kind == MBX_GEOM_PARALLEL && p.boxq * 4 < p.ts) return fail("window rows", w);
+                                        if (B.windows[w] && bpf_window_channels(kind, p.boxq) < BPF_BOX) return fail("window channels", w);
+                                        units[w] += (double)p.gx * p.gy * BPF_WARPS / (8.0 * BPF_LAUNCH_WARPS * num_sms());
+                                        same = same && p.boxq == scan_bp_plan(zs[s], SW_SUBSET).boxq;
+                                    }
+                                    differ += same ? 0 : 1;
                                 }
-                                same = same && scan_window_box(z, w) == scan_window_box(z, 0);
+                                for (int w = 0; w < SW_COUNT; ++w)
+                                    if (B.windows[w] && !(kind == MBX_GEOM_TRANSLATION && w == SW_INIT) && units[w] < BATCH_WINDOW_WAVES)
+                                        return fail("windows on an idle chip", w);
+                                (B.windows[SW_SUBSET] ? with : without) += 1;
                             }
-                            differ += same ? 0 : 1;
-                        }
-    std::printf("ok %ld %ld\n", scans, differ);
-    return scans > 0 ? 0 : 1;
+    std::printf("ok %ld %ld %ld %ld\n", checked, differ, with, without);
+    return checked > 0 ? 0 : 1;
 }

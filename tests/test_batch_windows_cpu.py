@@ -23,10 +23,11 @@ def _run(name, tmp_path):
 
 
 def test_each_back_projection_has_a_tensor_map_of_its_own_rows(tmp_path):
-    """Subset, initial and Hessian back projections of a scan can have slice tiles of different heights (cone scans whose
-    subsets leave the chip idle): each copies through a map whose box has its own rows."""
-    scans, differ = _run('batch_windows_check', tmp_path)
+    """Subset, initial and Hessian back projections of a scan can have slice tiles of different heights (a list that leaves
+    the chip idle takes lower ones): each that reads windows copies through a map whose box has its own rows."""
+    scans, differ, with_windows, without = _run('batch_windows_check', tmp_path)
     assert scans > 5000 and differ > 100  # the sweep holds scans that one map could not serve
+    assert with_windows > 300 and without > 300
 
 
 def test_windows_of_few_slices_keep_their_width(tmp_path):

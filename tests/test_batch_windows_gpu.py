@@ -45,17 +45,25 @@ def _batch_matches_plain(items, weights, seeds, iters=2):
 
 @pytest.mark.parametrize('weighted', [False, True])
 def test_cone_scans_whose_back_projections_differ_in_tile_height(cuda, weighted):
-    """The subsets of these scans take slice tiles of half the height that their set-up's back projections take."""
+    """The subsets of these scans take lower slice tiles than their set-up's back projections."""
     items = [_scan('cone', 60, 32, 64, 3), _scan('cone', 60, 32, 96, 4), _scan('cone', 60, 40, 64, 5)]
     ws = [np.exp(-s / s.max()).astype(np.float32) for _, s in items] if weighted else None
     _batch_matches_plain(items, ws, [3, 4, 5])
 
 
+@pytest.mark.parametrize('weighted', [False, True])
+def test_cone_batch_that_fills_the_chip(cuda, weighted):
+    """Subset, initial and (weighted) Hessian back projections read windows."""
+    items = [_scan('cone', 20 + i, 96 - i, 96 + i, i, 1) for i in range(8)]
+    ws = [np.exp(-s / s.max()).astype(np.float32) for _, s in items] if weighted else None
+    _batch_matches_plain(items, ws, list(range(8)))
+
+
 @pytest.mark.parametrize('channels', [256, 260, 300])
-@pytest.mark.parametrize('subsets', [4, 48])
+@pytest.mark.parametrize('subsets', [1, 4, 48])
 def test_parallel_scans_of_few_slices(cuda, channels, subsets):
     """With at most 4 slices a window holds up to 288 channels, and warps whose pixels lie across the grid (where the
-    Z-order jumps) take windows of that width."""
+    Z-order jumps) take windows of that width (1 subset; the others read their taps from the sinograms)."""
     items = [_scan('parallel', 90, rows, channels, rows, subsets) for rows in (1, 3, 4)]
     _batch_matches_plain(items, None, [1, 3, 4], iters=1 if subsets == 48 else 2)
 
