@@ -388,11 +388,10 @@ __device__ __forceinline__ void bpf_private_wait() {
 
 // The constants of view v of a call, see bpf_footprint.
 template <int KIND, bool TR>
-__device__ __forceinline__ float4 bpf_view(const BpArgs &A, int v, bool flag, int *err) {
+__device__ __forceinline__ float4 bpf_view(const BpArgs &A, int v) {
     const mbx_geom &g = A.g;
     const int vi = A.views ? A.views[v] : v;
     const bool ok = vi >= 0 && vi < g.num_views;
-    if (!ok && flag) flag_error(err, MBX_ERRFLAG_VIEW);
     float4 vw;
     if (KIND == MBX_GEOM_TRANSLATION) {
         vw.x = ok ? g.translations[3 * vi] : 0.0f;
@@ -688,7 +687,7 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
         while (!__any_sync(ALL, todo)) {
             if (v >= v_stop) return false;
             const int t = (v - vb) & 31;
-            if (t == 0 && v != vb) mine = bpf_view<KIND, true>(A, min(v + lane, v_stop - 1), pg == 0 && st == 0, err);
+            if (t == 0 && v != vb) mine = bpf_view<KIND, true>(A, min(v + lane, v_stop - 1));
             const float4 vw = view_constants(t);
             ++v;
             voff = __float_as_int(vw.w);
@@ -803,7 +802,7 @@ __device__ __forceinline__ void bp_fast_unit(const BpArgs &args, const CUtensorM
     for (; vb < v_end && !none && !pipe.failed; vb = v_stop) {
         v = vb;
         v_stop = !FAN ? min(vb + 32, v_end) : v_end;
-        mine = bpf_view<KIND, true>(A, min(vb + lane, v_stop - 1), pg == 0 && st == 0, err);
+        mine = bpf_view<KIND, true>(A, min(vb + lane, v_stop - 1));
         BpfItem cur, nxt;
         cur.in = false;
         cur.tma = false;
@@ -927,7 +926,7 @@ __device__ __forceinline__ void bp_direct_unit(const BpArgs &args, int pg, int s
     bool bad = false;
 
     for (int vb = v_begin; vb < v_end; vb += 32) {
-        const float4 mine = bpf_view<KIND, false>(A, min(vb + lane, v_end - 1), pg == 0 && st == 0, err);
+        const float4 mine = bpf_view<KIND, false>(A, min(vb + lane, v_end - 1));
         const int nv = min(32, v_end - vb);
         for (int t = 0; t < nv; ++t) {
             const float4 vw = make_float4(__shfl_sync(ALL, mine.x, t), __shfl_sync(ALL, mine.y, t),
@@ -1078,6 +1077,11 @@ bp_fast_kernel(const BpArgs args, const __grid_constant__ CUtensorMap map, int *
     float *smw = smf + warp * bpf_warp_floats(KIND, TR);
     BpfPipe pipe = {0, 0, false};
     if (TR) pipe = bpf_pipe_init(smw + bpf_warp_floats(KIND, TR) - 32);
+    if (args.views && unit == 0) {  // bad views of this split, which every unit skips
+        const int v_end = min(args.num_views_sel, ((int)blockIdx.y + 1) * args.views_per_split);
+        for (int v = blockIdx.y * args.views_per_split + (threadIdx.x & 31); v < v_end; v += 32)
+            if (args.views[v] < 0 || args.views[v] >= args.g.num_views) flag_error(err, MBX_ERRFLAG_VIEW);
+    }
     bp_fast_run<KIND, TR>(args, TR ? &map : nullptr, unit >> 3, unit & 7, blockIdx.y, smw, pipe, err);
 }
 

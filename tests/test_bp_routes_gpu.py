@@ -114,3 +114,19 @@ def test_taps_from_the_sinogram(cuda, kind):
         ones = _capi.back_project(g, None, torch.as_tensor(pix, device=cuda), coeff_power=power).cpu().numpy()
         ref = O.sparse_back_project(geom, np.ones(geom.sinogram_shape, np.float32), pix, coeff_power=power)
         assert rel_l2(ones, ref) <= 1e-5
+
+
+def test_bad_views_are_flagged_whatever_the_first_pixels_are(cuda):
+    """Bad indices are skipped and flagged: a bad view too when none of a warp's pixels is in the grid."""
+    model, geom = make_case('parallel', views=260, rows=37, channels=150)
+    g, n = model._geometry(), 150 * 150
+    pix = torch.arange(n, dtype=torch.int32, device=cuda)
+    pix[:64] = -1
+    views = torch.arange(260, dtype=torch.int32, device=cuda)
+    sino = torch.rand(geom.sinogram_shape, device=cuda)
+    _capi.get_device_error()
+    _capi.back_project(g, sino, pix, view_indices=views)
+    assert _capi.get_device_error() == 1
+    views[130] = 260
+    _capi.back_project(g, sino, pix, view_indices=views)
+    assert _capi.get_device_error() == 3
