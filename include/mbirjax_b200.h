@@ -140,6 +140,9 @@ MBX_API int mbx_sparse_forward_project(const mbx_geom *g, const float *voxel_val
 /* Workspace the back projector needs for a call with these sizes (0 when it needs none): partial sums of view splits,
  * and for calls with enough pixels a transposed copy of the projected views. */
 MBX_API size_t mbx_back_project_workspace_bytes(const mbx_geom *g, int64_t num_pixels, int32_t num_views_sel);
+/* The least that mbx_sparse_back_project accepts: with less than the full workspace it makes no transposed copy, which takes
+ * longer (for callers whose memory has no room for one). */
+MBX_API size_t mbx_back_project_least_workspace_bytes(const mbx_geom *g, int64_t num_pixels, int32_t num_views_sel);
 
 /* Sparse back projection of a full sinogram (num_views, R, C) to out (num_pixels, S) (overwritten):
  *   out = scale * sum_views A^coeff_power^T (weights * sinogram)

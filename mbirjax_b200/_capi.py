@@ -66,6 +66,7 @@ _SIGNATURES = {
     'mbx_forward_project_workspace_bytes': (c_size_t, [ctypes.POINTER(MbxGeom), c_int64, c_int32]),
     'mbx_sparse_forward_project': (ctypes.c_int, [ctypes.POINTER(MbxGeom), c_void_p, c_void_p, c_int64, c_void_p,
                                                   c_int32, c_void_p, c_void_p, c_size_t, c_void_p]),
+    'mbx_back_project_least_workspace_bytes': (c_size_t, [ctypes.POINTER(MbxGeom), c_int64, c_int32]),
     'mbx_back_project_workspace_bytes': (c_size_t, [ctypes.POINTER(MbxGeom), c_int64, c_int32]),
     'mbx_sparse_back_project': (ctypes.c_int, [ctypes.POINTER(MbxGeom), c_void_p, c_void_p, c_void_p, c_int64,
                                                c_void_p, c_int32, c_int32, c_float, c_void_p, c_void_p, c_size_t,
@@ -237,8 +238,11 @@ def back_project(geom, sinogram, pixel_indices, view_indices=None, coeff_power=1
     nv = int(view_indices.shape[0]) if view_indices is not None else geom.num_views
     if out is None:
         out = torch.empty((n, geom.num_recon_slices), dtype=torch.float32, device=pixel_indices.device)
-    nbytes = lib.mbx_back_project_workspace_bytes(ctypes.byref(geom), n, nv)
-    ws, nbytes = _workspace(nbytes, pixel_indices.device)
+    try:
+        ws, nbytes = _workspace(lib.mbx_back_project_workspace_bytes(ctypes.byref(geom), n, nv), pixel_indices.device)
+    except torch.OutOfMemoryError:  # no room for a transposed copy of the views: without one
+        nbytes = lib.mbx_back_project_least_workspace_bytes(ctypes.byref(geom), n, nv)
+        ws, nbytes = _workspace(nbytes, pixel_indices.device)
     rc = lib.mbx_sparse_back_project(ctypes.byref(geom), _ptr(sinogram), _ptr(weights), _ptr(pixel_indices), n,
                                      _ptr(view_indices), nv, int(coeff_power), float(scale), _ptr(out), _ptr(ws),
                                      nbytes, _stream())

@@ -135,6 +135,9 @@ int back_project(const mbx_geom &g, const float *sino, const float *w, const int
                  const int32_t *views, int num_views_sel, int coeff_power, float scale, float *out, void *ws,
                  size_t ws_bytes, cudaStream_t st, bool noalloc) {
     if (num_pixels == 0) return MBX_OK;
+    // no room for a transposed copy: without one, if that fits
+    if (!noalloc && ws_bytes < bp_workspace_bytes(g, num_pixels, num_views_sel))
+        noalloc = ws_bytes >= bp_noalloc_bytes(g, num_pixels, num_views_sel);
     BpArgs A = {};
     A.g = g;
     A.sino = sino;
@@ -232,6 +235,12 @@ int back_project(const mbx_geom &g, const float *sino, const float *w, const int
 extern "C" size_t mbx_back_project_workspace_bytes(const mbx_geom *g, int64_t num_pixels, int32_t num_views_sel) {
     if (mbx::validate_geom(g) != MBX_OK || num_pixels < 0 || num_views_sel <= 0) return 0;
     return mbx::bp_workspace_bytes(*g, num_pixels, num_views_sel);
+}
+
+extern "C" size_t mbx_back_project_least_workspace_bytes(const mbx_geom *g, int64_t num_pixels, int32_t num_views_sel) {
+    if (mbx::validate_geom(g) != MBX_OK || num_pixels < 0 || num_views_sel <= 0) return 0;
+    return std::min(mbx::bp_workspace_bytes(*g, num_pixels, num_views_sel),
+                    mbx::bp_noalloc_bytes(*g, num_pixels, num_views_sel));
 }
 
 extern "C" int mbx_sparse_back_project(const mbx_geom *g, const float *sinogram, const float *weights,

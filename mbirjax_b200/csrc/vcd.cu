@@ -14,6 +14,8 @@
 //   5. vcd_alpha_kernel (one block): fixed-order sums, alpha = clip((fl-pl)/(fq+pq+eps), eps, 1.5)
 //   6. vcd_apply_kernel: recon[idx] += alpha*delta, float64 partials of |alpha*delta|
 //   7. vcd_error_kernel: e -= alpha*delta_sino, and the last block folds the l1 partials into stats
+#include <algorithm>
+
 #include "mbx_common.cuh"
 #include "mbx_host.hpp"
 #include "mbx_reduce.cuh"
@@ -214,12 +216,10 @@ static VcdLayout vcd_layout(const mbx_geom &g, long long num_pixels) {
     off += align256(ncyl);
     L.delta = off;
     off += align256(ncyl);
-    L.dsino = off;
-    off += align256(nsino);
-    L.fpws = off;
-    off += align256(L.fp_bytes);
-    L.bpws = off;
-    off += align256(L.bp_bytes);
+    // the back projection's workspace and what the forward projection writes are never needed together
+    L.bpws = L.dsino = off;
+    L.fpws = off + align256(nsino);
+    off += std::max(align256(nsino) + align256(L.fp_bytes), align256(L.bp_bytes));
     L.partials = off;
     off += align256((size_t)3 * L.max_blocks * 2 * sizeof(double));
     L.alpha = off;

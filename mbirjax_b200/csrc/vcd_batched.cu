@@ -540,8 +540,11 @@ static int layout(const mbx_scan *scans, int n, int num_steps, Layout &L, std::v
     for (int s = 0; s < n; ++s) {
         L.buf_off[4 * s] = take(4 * (size_t)zs[s].ncyl);
         L.buf_off[4 * s + 1] = take(4 * (size_t)zs[s].ncyl);
-        L.buf_off[4 * s + 2] = take(4 * (size_t)zs[s].nsino);
-        L.buf_off[4 * s + 3] = take(copies ? bpf_transposed_bytes(scans[s].geom, scans[s].geom.num_views) : 0);
+        // the projection of a step's update and the transposed copy that the next back projection reads are never needed
+        // together
+        const size_t dsino = 4 * (size_t)zs[s].nsino;
+        const size_t copy = copies ? bpf_transposed_bytes(scans[s].geom, scans[s].geom.num_views) : 0;
+        L.buf_off[4 * s + 2] = L.buf_off[4 * s + 3] = take(std::max(dsino, copy));
     }
     L.box_off.resize(n);
     L.fbox_off.assign(n, 0);
@@ -980,7 +983,7 @@ extern "C" int mbx_vcd_batched_prepare2(const mbx_scan *scans, int32_t num_scans
         v.bp = reinterpret_cast<float *>(base + L.buf_off[4 * s]);
         v.delta = reinterpret_cast<float *>(base + L.buf_off[4 * s + 1]);
         v.dsino = reinterpret_cast<float *>(base + L.buf_off[4 * s + 2]);
-        v.tsino = reinterpret_cast<float *>(base + L.buf_off[4 * s + 3]);  // (of no size when nothing reads windows)
+        v.tsino = reinterpret_cast<float *>(base + L.buf_off[4 * s + 3]);  // (the same memory as dsino)
         v.V = g.num_views;
         v.R = g.num_det_rows;
         v.C = g.num_det_channels;

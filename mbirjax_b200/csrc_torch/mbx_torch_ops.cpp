@@ -136,8 +136,14 @@ at::Tensor sparse_back_project(at::IntArrayRef gi, at::ArrayRef<double> gf, cons
     const int64_t n = pixel_indices.numel();
     const int32_t nv = view_indices.has_value() ? (int32_t)view_indices->numel() : g.num_views;
     auto out = at::empty({n, g.num_recon_slices}, pixel_indices.options().dtype(at::kFloat));
-    const size_t wb = mbx_back_project_workspace_bytes(&g, n, nv);
-    auto ws = workspace(wb, out);
+    size_t wb = mbx_back_project_workspace_bytes(&g, n, nv);
+    at::Tensor ws;
+    try {
+        ws = workspace(wb, out);
+    } catch (const c10::OutOfMemoryError &) {  // no room for a transposed copy of the views: without one
+        wb = mbx_back_project_least_workspace_bytes(&g, n, nv);
+        ws = workspace(wb, out);
+    }
     check_rc(mbx_sparse_back_project(&g, opt_ptr<float>(sinogram), opt_ptr<float>(weights),
                                      pixel_indices.data_ptr<int32_t>(), n, opt_ptr<int32_t>(view_indices), nv,
                                      (int32_t)coeff_power, (float)scale, out.data_ptr<float>(),

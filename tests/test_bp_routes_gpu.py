@@ -130,3 +130,40 @@ def test_bad_views_are_flagged_whatever_the_first_pixels_are(cuda):
     views[130] = 260
     _capi.back_project(g, sino, pix, view_indices=views)
     assert _capi.get_device_error() == 3
+
+
+@pytest.mark.parametrize('kind', ['parallel', 'cone'])
+def test_without_room_for_a_copy(cuda, kind, monkeypatch):
+    """A workspace without room for the copy, down to the least: the same sums; below that, an error.  The Python call
+    falls back by itself when the full workspace cannot be allocated."""
+    model, geom = make_case(kind, views=256, rows=66, channels=160)
+    g, lib = model._geometry(), _capi.load_library()
+    n = 160 * 160
+    pix = torch.arange(n, dtype=torch.int32, device=cuda)
+    sino = torch.randn(geom.sinogram_shape, device=cuda, generator=torch.Generator(device=cuda).manual_seed(1))
+    ref = _capi.back_project(g, sino, pix)
+    full = lib.mbx_back_project_workspace_bytes(ctypes.byref(g), n, g.num_views)
+    least = lib.mbx_back_project_least_workspace_bytes(ctypes.byref(g), n, g.num_views)
+    assert full >= 4 * 256 * 68 * 164 and least < full
+    ws = torch.empty(full, dtype=torch.uint8, device=cuda)
+    for nbytes, rc in ((full - 1, 0), (least, 0), (least - 1, _capi.MBX_ERR_WORKSPACE)):
+        if nbytes < 0:
+            continue
+        out = torch.full_like(ref, 7.0)
+        assert lib.mbx_sparse_back_project(ctypes.byref(g), _capi._ptr(sino), None, _capi._ptr(pix), n, None, g.num_views,
+                                           1, 1.0, _capi._ptr(out), _capi._ptr(ws), nbytes, _capi._stream()) == rc
+        torch.cuda.synchronize()
+        assert bool(torch.all(out == 7.0)) if rc else rel_l2(out.cpu().numpy(), ref.cpu().numpy()) <= 1e-5
+
+    asked, real = [], _capi._workspace
+
+    def short_of_memory(nbytes, device):
+        asked.append(nbytes)
+        if nbytes >= full:
+            raise torch.OutOfMemoryError('no room')
+        return real(nbytes, device)
+
+    monkeypatch.setattr(_capi, '_workspace', short_of_memory)
+    got = _capi.back_project(g, sino, pix)
+    assert asked == [full, least]
+    assert rel_l2(got.cpu().numpy(), ref.cpu().numpy()) <= 1e-5
