@@ -15,13 +15,17 @@
 
 namespace mbx {
 
+// FEW: blocks of fewer rows than filter_shape's default, `groups` of them (1.59 ms with a group count that the compiler does
+// not know where 1.50 is taken without, 360 x 256 x 512).
+template <bool WHOLE, bool FEW>
 __global__ void __launch_bounds__(FILT_THREADS, 2)
 direct_filter_kernel(const float *__restrict__ sino, float *__restrict__ out, long long num_rows_total, int R, int C,
                      int rows, double filter_scale, double out_scale, int fdk, double D, double delta_det_channel,
                      double delta_det_row, double det_channel_offset, double det_row_offset, int groups) {
     extern __shared__ __align__(16) double sm[];
-    direct_filter_rows(sino, out, (long long)blockIdx.x * rows, num_rows_total, R, C, filter_scale, out_scale, fdk, D,
-                       delta_det_channel, delta_det_row, det_channel_offset, det_row_offset, sm, groups);
+    direct_filter_rows<WHOLE>(sino, out, (long long)blockIdx.x * rows, num_rows_total, R, C, filter_scale, out_scale, fdk,
+                              D, delta_det_channel, delta_det_row, det_channel_offset, det_row_offset, sm,
+                              FEW ? groups : 0);
 }
 
 }  // namespace mbx
@@ -41,9 +45,11 @@ extern "C" int mbx_direct_filter(const mbx_geom *g, const float *sinogram, float
     int groups = mbx::filter_shape(C).groups;
     while (groups > 1 && mbx::ceil_div(rows_total, 16 * groups) < 2 * mbx::num_sms()) groups /= 2;
     const size_t smem = mbx::filter_smem_bytes(C, groups);
+    const auto kern = groups < mbx::filter_shape(C).groups ? mbx::direct_filter_kernel<false, true>
+                      : mbx::filter_whole(C)               ? mbx::direct_filter_kernel<true, false>
+                                                           : mbx::direct_filter_kernel<false, false>;
     {
-        cudaError_t e = mbx::set_max_dynamic_smem(reinterpret_cast<const void *>(mbx::direct_filter_kernel),
-                                                  200 * 1024);
+        cudaError_t e = mbx::set_max_dynamic_smem(reinterpret_cast<const void *>(kern), 200 * 1024);
         if (e != cudaSuccess) return mbx::set_cuda_error(e);
     }
     double filter_scale, out_scale;
@@ -51,7 +57,7 @@ extern "C" int mbx_direct_filter(const mbx_geom *g, const float *sinogram, float
     mbx::direct_filter_scales(*g, filter_scale, out_scale, fdk);
     const int rows = mbx::filter_shape(C, groups).rows;
     const unsigned blocks = (unsigned)((rows_total + rows - 1) / rows);
-    mbx::direct_filter_kernel<<<blocks, mbx::FILT_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(
+    kern<<<blocks, mbx::FILT_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(
         sinogram, out, rows_total, R, C, rows, filter_scale, out_scale, fdk, g->source_detector_dist, g->delta_det_channel,
         g->delta_det_row, g->det_channel_offset, g->det_row_offset, groups);
     mbx::note_launch();

@@ -60,6 +60,13 @@ __host__ __device__ inline FiltShape filter_shape(int C, int groups = 0) {
     return f;
 }
 
+// Rows whose chunks are nearly all used take them whole: 512 channels (all used) 1.50 ms with unchanging bounds and 1.56
+// without, 1000 (500 of 512 samples) 624 and 644 us, but 437 (219 of 256) 569 and 501.
+inline bool filter_whole(int C) {
+    const FiltShape f = filter_shape(C);
+    return 20 * f.outs >= 19 * f.kp;
+}
+
 inline size_t filter_smem_bytes(int C, int groups = 0) {
     const FiltShape f = filter_shape(C, groups);
     return sizeof(double) * (2 * (size_t)f.kc * f.pitch + 2 * (size_t)f.taps);
@@ -75,7 +82,10 @@ inline size_t filter_smem_bytes(int C, int groups = 0) {
 // one place, so a sample costs one tap load, two 16-byte loads of 4 rows (staged as float64, [sample][row]) and 32 FMAs,
 // and the loop is bound by the float64 pipe (half the float32 rate).  The tap tables (one per parity) are padded to 9
 // doubles per 8 taps, which keeps the lanes' loads, 8 taps apart, in different banks.  Measured on 360 x 256 x 512 (FDK):
-// 5.53 -> 1.59 ms against one output and 8 rows per thread, whose samples were converted to float64 at every use.
+// 5.53 -> 1.50 ms against one output and 8 rows per thread, whose samples were converted to float64 at every use.
+// WHOLE: every chunk of samples is taken whole, zeros past the row, with bounds that do not change from chunk to chunk
+// (filter_whole); else the last one ends with the row.
+template <bool WHOLE = false>
 __device__ __forceinline__ void direct_filter_rows(const float *__restrict__ sino, float *__restrict__ out,
                                                    long long row0, long long num_rows_total, int R, int C,
                                                    double filter_scale, double out_scale, int fdk, double D,
@@ -114,7 +124,7 @@ __device__ __forceinline__ void direct_filter_rows(const float *__restrict__ sin
             for (int r = 0; r < 4; ++r) acc[u][r] = 0.0;
         for (int k0 = 0; k0 < f.kp; k0 += f.kc) {
             __syncthreads();  // the last samples (and, at the start of a pass, its predecessor's outputs) are read
-            const int kn = min(f.kc, (f.outs - k0 + 7) & ~7);  // samples of the chunk, in eights
+            const int kn = WHOLE ? f.kc : min(f.kc, (f.outs - k0 + 7) & ~7);  // samples of the chunk, in eights
             for (int t = tid; t < 2 * kn * f.rows; t += FILT_THREADS) {
                 const int rr = t / (2 * kn), cc = t - rr * 2 * kn, j = 2 * k0 + cc;
                 double v = 0.0;
