@@ -46,3 +46,9 @@ def test_maps_in_global_memory_are_acquired_before_their_first_copy():
         kernel = text[text.rindex('__global__', 0, use):use]
         assert 'bpf_acquire_map(' in kernel
     assert 'bp_fast_run<' in text
+
+
+def test_plans_of_the_second_forward_variant_and_of_the_scratch(tmp_path):
+    """The 4-CTA forward plans hold what each mode reads, and the partial sums of the entry point that allocates nothing
+    fit its scratch."""
+    assert _run('many_plan_check', tmp_path)[0] > 50000
