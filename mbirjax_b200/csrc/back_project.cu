@@ -135,9 +135,6 @@ int back_project(const mbx_geom &g, const float *sino, const float *w, const int
                  const int32_t *views, int num_views_sel, int coeff_power, float scale, float *out, void *ws,
                  size_t ws_bytes, cudaStream_t st, bool noalloc) {
     if (num_pixels == 0) return MBX_OK;
-    // no room for a transposed copy: without one, if that fits
-    if (!noalloc && ws_bytes < bp_workspace_bytes(g, num_pixels, num_views_sel))
-        noalloc = ws_bytes >= bp_noalloc_bytes(g, num_pixels, num_views_sel);
     BpArgs A = {};
     A.g = g;
     A.sino = sino;
@@ -168,7 +165,11 @@ int back_project(const mbx_geom &g, const float *sino, const float *w, const int
     if (A.plan.ok) {
         bool tr = !noalloc && sino && bp_transposes(g, A.plan, num_pixels, num_views_sel);
         const size_t need = A.plan.workspace + (tr ? bpf_transposed_bytes(g, num_views_sel) : 0);
-        if (need > 0 && (ws == nullptr || ws_bytes < need)) return MBX_ERR_WORKSPACE;
+        if (need > 0 && (ws == nullptr || ws_bytes < need)) {
+            if (noalloc || ws_bytes < bp_noalloc_bytes(g, num_pixels, num_views_sel)) return MBX_ERR_WORKSPACE;
+            return back_project(g, sino, w, pix, num_pixels, views, num_views_sel, coeff_power, scale, out, ws, ws_bytes,
+                                st, true);  // no room for a transposed copy: without one
+        }
         float *copy = reinterpret_cast<float *>(static_cast<char *>(ws) + A.plan.workspace);
         tr = tr && bpf_window_map(map, copy, g, num_views_sel, A.plan.boxq);
         // parallel with windows by its size, but no room or no map for them: the gather in the windows' splits, so that the
