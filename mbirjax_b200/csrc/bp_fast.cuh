@@ -2,9 +2,9 @@
 // detector pitch at the magnification).  Same contract and arithmetic as the general bp_kernel (back_project.cuh);
 // organised so that a (pixel, slice, view) costs few instructions and its detector samples come from shared memory:
 //
-//  * CTA = 256 threads = 8 independent warps; a warp owns 32 pixels (one per lane) x a tile of ts <= BPF_ST slices,
-//    with the accumulators of a lane's slices in registers (as pairs, for the two-wide FMA) across all views.
-//    Nothing but the per-view constants is shared between warps, so they run without barriers of their own.
+//  * A warp owns 32 pixels (one per lane) x a tile of ts <= BPF_ST slices, with the accumulators of a lane's slices in
+//    registers (as pairs, for the two-wide FMA) across all views.  Warps share nothing, so they run without barriers; a plan
+//    counts them in tiles of eight, and a launch puts two (four without windows) in a CTA.
 //  * Per view each lane computes the footprint of its pixel in registers: centre channel, three coefficients
 //    (already raised to coeff_power, zero off the detector), and for the fan geometries the affine map slice ->
 //    detector row m_p(k) = A0 + k*A1 and the vertical-angle factor c2 = (mag/D)^2, 1/cos(phi_k) = sqrt(1 + c2 z_k^2).
